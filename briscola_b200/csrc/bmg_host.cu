@@ -1305,7 +1305,7 @@ void smooth(bmg_ctx* c, int l, int sweeps) {
 }
 
 template <typename T>
-void residualRestrict(bmg_ctx* c, int l) {
+void residualRestrict(bmg_ctx* c, int l, bool zeroCoarse = true) {
     exchange<T>(c, l);
     const Bricks<T> F = bricks<T>(c, l);
     const Bricks<T> C = bricks<T>(c, l + 1);
@@ -1314,7 +1314,7 @@ void residualRestrict(bmg_ctx* c, int l) {
         launch_residual_restrict<T, true>(F, C, ttabs(c, l), c->stream);
     else
         launch_residual_restrict<T, false>(F, C, ttabs(c, l), c->stream);
-    BMG_CUDA(cudaMemsetAsync(C.v[0].x, 0, C.v[0].cells * sizeof(T), c->stream));
+    if (zeroCoarse) BMG_CUDA(cudaMemsetAsync(C.v[0].x, 0, C.v[0].cells * sizeof(T), c->stream));
 }
 
 template <typename T>
@@ -1447,52 +1447,166 @@ int levelReps(const bmg_ctx* c, int l) {  // MG.H:106-124
 // MG.C:19-130.  x(l) = 0 for l > 0 is done by the restriction step that
 // produces b(l).  The finest-level residual is always recomputed after
 // pre-smoothing (the reference skips it on the first repetition, MG.C:72).
-// The levels from tailFirst(c) to the coarse solve level run in one CTA
-// (k_tail_cycle) when the cycle is a single-brick V cycle with red-black
-// smoothing and factor-2 quad transfers on every one of them; -1 otherwise.
-int tailFirst(const bmg_ctx* c) {
-    if (!c->opt.fuse_coarse || c->multi || c->opt.cycle_type != BMG_CYCLE_V ||
+// The levels from tailFirst(c) to the coarse solve level run in one
+// thread-block cluster (bmg_tail.cu) when the cycle is a single-brick V or F cycle with red-black
+// smoothing; -1 otherwise.
+//
+// the steps of the sub-cycle from level l, as cycle() takes them
+void tailSteps(bmg_ctx* c, int first, int l, std::vector<unsigned char>& ops) {
+    auto step = [&](int op) { ops.push_back((unsigned char)(op << 3 | (l - first))); };
+    if (c->opt.n_pre > 0 && l < c->lc) step(TAIL_PRE);
+    if (l < c->lc) {
+        const int reps = levelReps(c, l);
+        for (int rep = 0; rep < reps; ++rep) {
+            step(TAIL_RESTRICT);
+            tailSteps(c, first, l + 1, ops);
+            step(TAIL_PROLONG);
+            if (c->opt.n_post > 0) step(TAIL_POST);
+        }
+    } else {
+        step(TAIL_COARSE);
+    }
+    c->visits[l]++;
+}
+
+// the plan of the levels first .. lc in shared memory, without its steps
+template <typename T>
+TailPlan<T> tailPlan(const bmg_ctx* c, int first) {
+    TailPlan<T> P{};
+    P.nlev = c->lc - first + 1;
+    P.ncoarse = c->ncoarse;
+    P.ainv = c->ainv;
+    P.zeroStart = first > 0;
+    int at = 0;
+    auto take = [&](long words) {
+        const int o = at;
+        at += (int)((words + 1) & ~1L);
+        return o;
+    };
+    // planes per CTA: whole pairs where the level halves along axis 0
+    int used = 1;
+    int scratch = 0;
+    auto magic = [](int d) { return d > 1 ? (unsigned)(((1ULL << 32) + d - 1) / d) : 0u; };
+    for (int q = 0; q < P.nlev; ++q) {
+        const int l = first + q;
+        const LevelView<T> V = bricks<T>(c, l).v[0];
+        TailLevel<T>& L = P.v[q];
+        L.n0 = V.n0;
+        L.n1 = V.n1;
+        L.n2 = V.n2;
+        L.ne = (V.n2 + 1) / 2;
+        L.dist = l < c->lc && (long)L.n0 * L.n1 * L.n2 > kTailGather;
+        L.P = L.n0;
+        if (L.dist) {
+            const int g = c->lv[l + 1].br[0].R[0];
+            L.P = g * ((L.n0 + g * kTailRanks - 1) / (g * kTailRanks));
+            used = std::max(used, (L.n0 + L.P - 1) / L.P);
+        }
+        L.sj = V.n2 + 2;
+        L.si = (V.n1 + 2) * L.sj;
+        L.xcells = (L.P + 2) * L.si;
+        L.mne = magic(L.ne);
+        L.mn1 = magic(L.n1);
+        L.mn2 = magic(L.n2);
+        L.mP = magic(L.P);
+        L.per0 = V.per0;
+        L.per1 = V.per1;
+        L.per2 = V.per2;
+        L.cpar = V.cpar;
+        L.gbase = V.base;
+        L.gsi = V.si;
+        L.gsj = V.sj;
+        L.gkh = V.kh;
+        L.x = take(L.xcells);
+        L.b = take((long)L.P * L.n1 * L.n2);
+        if (q > 0 && P.v[q - 1].dist)
+            scratch = std::max(scratch, (P.v[q - 1].P / P.v[q - 1].R0 + 2) * L.si);
+        if (q == 0) {
+            P.g = V;
+            P.gx = V.x;
+            P.gb = V.b;
+        }
+        if (l == c->lc) continue;
+        const int n = L.n0 + L.n1 + L.n2;
+        L.tab = take(2 * n);
+        L.ratio = take(n);
+        L.pw = take(n);
+        L.pidx = take((2 * n * (long)sizeof(int) + sizeof(T) - 1) / sizeof(T));
+        L.gtab = V.tab;
+        const TransferTabs t = ttabs(c, l).t[0];
+        L.gratio = sizeof(T) == 8 ? reinterpret_cast<const T*>(t.ratio64) : reinterpret_cast<const T*>(t.ratio32);
+        L.gpw = sizeof(T) == 8 ? reinterpret_cast<const T*>(t.pw64) : reinterpret_cast<const T*>(t.pw32);
+        L.gpidx = t.pidx;
+        L.R0 = t.R0;
+        L.R1 = t.R1;
+        L.R2 = t.R2;
+        L.quad = t.R0 == 2 && t.R1 == 2 && t.R2 == 2 && V.n2 % 4 == 0;
+        for (int d = 0; d < 3; ++d) {
+            L.wl[d] = V.to.wl[d];
+            L.wh[d] = V.to.wh[d];
+            L.glam[d] = (&V.lam0)[d];
+            if (c->variable)
+                L.lam[d] = take((long)(L.P + (d == 0)) * (L.n1 + (d == 1)) * (L.n2 + (d == 2)));
+        }
+        auto seq = [&](int sweeps, int& len, int& first) {
+            if (sweeps <= 0) return;
+            const std::vector<int> s = colourSequence(c->lv[l], sweeps);  // alternating
+            len = (int)s.size();
+            first = s[0];
+        };
+        seq(c->opt.n_pre, L.npre, L.pre);
+        seq(c->opt.n_post, L.npost, L.post);
+    }
+    P.scratch = take(scratch);
+    // whole power-of-two clusters
+    P.ranks = 1;
+    while (P.ranks < used) P.ranks *= 2;
+    P.spread = P.ranks > 1 && P.ncoarse > kTailSpread;
+    const long words = (long)at * sizeof(T) + (P.ncoarse + 1) * 8L;
+    const long inv = (long)P.ncoarse * P.ncoarse;
+    if (!P.spread && words + inv * 8 + 8 <= kTailSmem) P.ainvWords = (int)(inv + (inv & 1));
+    P.smem = (size_t)(words + P.ainvWords * 8L + 16);
+    return P;
+}
+
+int tailFirst(bmg_ctx* c) {
+    if (!c->opt.fuse_coarse || c->multi ||
+        (c->opt.cycle_type != BMG_CYCLE_V && c->opt.cycle_type != BMG_CYCLE_F) ||
         c->opt.smoother != BMG_SMOOTHER_RBGS || c->opt.coarse_mode != BMG_COARSE_DIRECT)
         return -1;
     const int lc = c->lc;
+    if (c->ncoarse > kTailCoarse) return -1;
+    const bool f32 = c->opt.precision == BMG_PRECISION_MIXED;
     int first = lc;
-    while (first > 0 && c->lv[first - 1].ncell <= kTailCells) --first;
-    if (first == lc || lc - first + 1 > kMaxTail) return -1;
+    for (; first > 0; --first) {
+        const HostLevel& H = c->lv[first - 1];
+        if (lc - first + 2 > kMaxTail) break;
+        const TailPlan<double> S = tailPlan<double>(c, first - 1);
+        if ((long)S.v[0].P * S.v[0].n1 * S.v[0].ne > kTailThreads) break;
+        // (a periodic axis of one cell has two images of it)
+        bool single = false;
+        for (int d = 0; d < 3; ++d) single = single || (c->periodic[d] && H.br[0].n[d] == 1);
+        if (single) break;
+        if ((long)(f32 ? tailPlan<float>(c, first - 1).smem : tailPlan<double>(c, first - 1).smem) > kTailSmem) break;
+        std::vector<unsigned char> ops;
+        std::fill(c->visits.begin(), c->visits.end(), 0);
+        tailSteps(c, first - 1, first - 1, ops);
+        if ((int)ops.size() > kMaxTailOps) break;
+    }
+    std::fill(c->visits.begin(), c->visits.end(), 0);
+    if (first == lc) return -1;
     // a level solver inside the tail's levels would be skipped by it
     if (c->hook && c->hookLevel >= first) return -1;
-    for (int q = first; q < lc; ++q) {
-        const HostBrick& F = c->lv[q].br[0];
-        const HostBrick& C = c->lv[q + 1].br[0];
-        if (F.n[2] % 4 || C.R[0] != 2 || C.R[1] != 2 || C.R[2] != 2) return -1;
-        const int lens[2] = {(int)colourSequence(c->lv[q], c->opt.n_pre).size(),
-                             (int)colourSequence(c->lv[q], c->opt.n_post).size()};
-        if (lens[0] > kMaxSeq || lens[1] > kMaxSeq) return -1;
-    }
     return first;
 }
 
 template <typename T>
 void tailCycle(bmg_ctx* c, int first) {
-    TailPlan<T> P{};
-    P.nlev = c->lc - first + 1;
-    for (int q = 0; q < P.nlev; ++q) {
-        const int l = first + q;
-        P.v[q] = bricks<T>(c, l).v[0];
-        if (l < c->lc) {
-            P.t[q] = ttabs(c, l).t[0];
-            const std::vector<int> pre = c->opt.n_pre > 0 ? colourSequence(c->lv[l], c->opt.n_pre) : std::vector<int>();
-            const std::vector<int> post =
-                c->opt.n_post > 0 ? colourSequence(c->lv[l], c->opt.n_post) : std::vector<int>();
-            P.npre[q] = (int)pre.size();
-            P.npost[q] = (int)post.size();
-            for (size_t e = 0; e < pre.size(); ++e) P.pre[q][e] = pre[e];
-            for (size_t e = 0; e < post.size(); ++e) P.post[q][e] = post[e];
-        }
-        c->visits[l]++;
-    }
-    P.ainv = c->ainv;
-    P.cidx = c->cidx;
-    P.ncoarse = c->ncoarse;
+    TailPlan<T> P = tailPlan<T>(c, first);
+    std::vector<unsigned char> ops;
+    tailSteps(c, first, first, ops);
+    P.nops = (int)ops.size();
+    std::copy(ops.begin(), ops.end(), P.ops);
     c->launches += 1;
     if (c->variable)
         launch_tail_cycle<T, true>(P, c->stream);
@@ -1533,7 +1647,7 @@ void cycle(bmg_ctx* c, int l) {
     if (l < c->lc) {
         const int reps = levelReps(c, l);
         for (int rep = 0; rep < reps; ++rep) {
-            residualRestrict<T>(c, l);
+            residualRestrict<T>(c, l, l + 1 != c->tail);  // the cluster's coarse end starts from zero by itself
             cycle<T>(c, l + 1);
             prolongCorrect<T>(c, l);
             if (c->opt.n_post > 0) smooth<T>(c, l, c->opt.n_post);
@@ -2029,6 +2143,7 @@ int bmg_create(bmg_ctx** out, const bmg_mesh_desc* mesh, const bmg_options* opts
         c->own_stream = true;
         BMG_CUDA(cudaStreamCreateWithFlags(&c->capStream, cudaStreamNonBlocking));
         configure_fused_kernels();
+        BMG_CUDA(configure_tail_kernels());
         build(c, std::move(L0));
         configureCoarse(c);
         c->tail = tailFirst(c);

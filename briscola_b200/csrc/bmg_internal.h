@@ -203,27 +203,64 @@ constexpr int kFusedMaxStages = 3;
 
 constexpr int kReduceThreads = 256;
 
-// The coarse end of a V-cycle in one CTA (k_tail_cycle): levels v[0] (the
-// first fused level) .. v[nlev-1] (the coarse solve level) of one brick,
-// the transfers between them, and each level's colour sequences.
-constexpr int kMaxTail = 6;
-constexpr int kMaxSeq = 16;
-constexpr int kTailThreads = 512;
-constexpr long kTailCells = 4096;  // levels this small run in the fused tail
-constexpr long kSplitMinCells = kTailCells;  // parity-split rows on single-brick levels above this
+// The coarse end of a V or F cycle in one thread-block cluster (bmg_tail.cu):
+// levels v[0] (the first fused level) .. v[nlev-1] (the coarse solve level) of
+// one brick, all of them in shared memory, and the steps of the sub-cycle.
+constexpr int kMaxTail = 8;
+constexpr int kMaxTailOps = 384;
+constexpr int kTailThreads = 1024;
+// A level runs in the cluster where every CTA has at most one pair of cells a
+// thread (32^3 on 16 CTAs), so that a pass is one update's latency.
+constexpr int kTailRanks = 16;         // CTAs of the cluster
+constexpr long kTailGather = 1024;     // levels this small run on CTA 0 alone
+
+constexpr int kTailCoarse = 512;       // largest dense coarse solve there
+constexpr int kTailSpread = 128;       // coarse solves above this are spread over the cluster
+constexpr long kSplitMinCells = 4096;  // parity-split rows on single-brick levels above this
+constexpr long kTailSmem = 232448 - 4096;  // dynamic shared memory of a CTA (227 KB less its descriptors)
+enum { TAIL_PRE = 0, TAIL_POST = 1, TAIL_RESTRICT = 2, TAIL_PROLONG = 3, TAIL_COARSE = 4 };
+
+template <typename T>
+struct TailLevel {
+    int n0, n1, n2;
+    int ne;              // even k of a row: (n2 + 1) / 2
+    int P;               // planes of a CTA: CTA r owns planes r P .. r P + P - 1
+    int dist;            // spread over the cluster; else P = n0 (CTA 0)
+    int si, sj, xcells;  // shared-memory x: (P+2) x (n1+2) rows of n2+2 words
+    int x, b;            // word offsets in shared memory (b: interior cells only)
+    int tab, ratio, pw, pidx, lam[3];
+    unsigned mne, mn1, mn2, mP;  // division by ne, n1, n2 and P: ceil(2^32 / d), 0 for d = 1
+    int per0, per1, per2, cpar;
+    int R0, R1, R2;      // factors to the next level
+    int quad;            // the per-pass restriction is restrict_quad_item's
+    int npre, npost;
+    int pre, post;       // colour of the first pass; the colours alternate
+    const T* gtab;       // the level's tables in global memory
+    int wl[3], wh[3];
+    const T* gratio;     // transfer tables to the next level
+    const T* gpw;
+    const int* gpidx;
+    const T* glam[3];
+    long gbase, gsi, gsj;  // the level's slab
+    int gkh;
+};
 
 template <typename T>
 struct TailPlan {
-    LevelView<T> v[kMaxTail];
-    TransferTabs t[kMaxTail];
-    int pre[kMaxTail][kMaxSeq];
-    int post[kMaxTail][kMaxSeq];
-    int npre[kMaxTail];
-    int npost[kMaxTail];
-    int nlev;
+    TailLevel<T> v[kMaxTail];
+    unsigned char ops[kMaxTailOps];  // step << 3 | level
+    int nlev, nops;
+    int zeroStart;       // x of the first level is zero on entry
+    LevelView<T> g;      // the first level in global memory
+    T* gx;
+    const T* gb;
     const double* ainv;
-    const int* cidx;
     int ncoarse;
+    int ainvWords;       // doubles the inverse takes in shared memory, 0: it stays in global memory
+    int ranks;           // CTAs launched
+    int spread;          // the coarse solve takes every CTA
+    int scratch;         // word offset of the prolongation's coarse planes
+    size_t smem;
 };
 
 // ---- launchers (bmg_kernels.cu) -------------------------------------------
@@ -240,8 +277,10 @@ void launch_prolong_correct(const Bricks<T>& F, const Bricks<T>& C, const Transf
 // dense solve on the coarse level; cidx lists the slab index of each unknown
 template <typename T>
 void launch_coarse_solve(const Bricks<T>& C, const double* ainv, const int* cidx, int n, cudaStream_t s);
+// the coarse end of a cycle in one CTA (bmg_tail.cu)
 template <typename T, bool VAR>
 void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s);
+cudaError_t configure_tail_kernels();
 template <typename T, bool VAR>
 void launch_residual_out(const Bricks<T>& B, double* r_unscaled_compact, cudaStream_t s);
 // x[dst[q]] = x[src[q]]: ghost refresh between bricks

@@ -944,65 +944,6 @@ __global__ void __launch_bounds__(256) k_coarse_solve(Bricks<T> CB, const double
     coarse_solve_block<T>(CB, ainv, cidx, n, sb, blockIdx.x * nw, gridDim.x * nw);
 }
 
-// ---------------------------------------------------------------------------
-// The coarse end of a V-cycle in one CTA: on the small levels every pass is
-// a few thousand cells, so a launch per pass costs more than the pass.  The
-// levels from P.first down to the coarse solve level run here with a barrier
-// between passes: pre-smoothing colour passes, restriction (and the zeroed
-// coarse x), the dense coarse solve, then prolongation and post-smoothing on
-// the way up -- the same per-item functions as the per-pass kernels, so the
-// result is bit-identical to the per-pass path (MG.C:19-130, V cycle).
-// ---------------------------------------------------------------------------
-template <typename T, bool VAR>
-__global__ void __launch_bounds__(kTailThreads) k_tail_cycle(TailPlan<T> P) {
-    grid_dep_sync();
-    extern __shared__ double sb[];
-    const int nt = blockDim.x;
-    const int nl = P.nlev;
-    auto smooth = [&](int q, const int* seq, int nseq) {
-        const LevelView<T>& L = P.v[q];
-        const int nq = L.n2 / 4;
-        const int items = L.n0 * L.n1 * nq;
-        for (int s = 0; s < nseq; ++s) {
-            for (int it = threadIdx.x; it < items; it += nt) {
-                const int p = it % nq, ij = it / nq;
-                colour_quad_item<T, VAR>(L, ij / L.n1, ij % L.n1, p, seq[s]);
-            }
-            __syncthreads();
-        }
-    };
-    for (int q = 0; q < nl - 1; ++q) {
-        smooth(q, P.pre[q], P.npre[q]);
-        const LevelView<T>& F = P.v[q];
-        const LevelView<T>& C = P.v[q + 1];
-        const int np = C.n2 / 2;
-        const int items = C.n0 * C.n1 * np;
-        for (int it = threadIdx.x; it < items; it += nt) {
-            const int pp = it % np, IJ = it / np;
-            restrict_quad_item<T, VAR>(F, C, P.t[q], IJ / C.n1, IJ % C.n1, pp);
-        }
-        // x(q+1) = 0 over the whole slab (the per-pass path's memset)
-        for (long c = threadIdx.x; c < C.cells; c += nt) C.x[c] = T(0);
-        __syncthreads();
-    }
-    Bricks<T> CB{};
-    CB.v[0] = P.v[nl - 1];
-    CB.nb = 1;
-    coarse_solve_block<T>(CB, P.ainv, P.cidx, P.ncoarse, sb);
-    __syncthreads();
-    for (int q = nl - 2; q >= 0; --q) {
-        const LevelView<T>& F = P.v[q];
-        const int nq = F.n2 / 4;
-        const int items = F.n0 * F.n1 * nq;
-        for (int it = threadIdx.x; it < items; it += nt) {
-            const int p = it % nq, ij = it / nq;
-            prolong_quad_item<T>(F, P.v[q + 1], P.t[q], ij / F.n1, ij % F.n1, p);
-        }
-        __syncthreads();
-        smooth(q, P.post[q], P.npost[q]);
-    }
-}
-
 template <typename T>
 __global__ void k_fill_ghosts(T* x, const int* __restrict__ dst, const int* __restrict__ src, long n) {
     grid_dep_sync();
@@ -1396,11 +1337,6 @@ void launch_coarse_solve(const Bricks<T>& C, const double* ainv, const int* cidx
     launch_k(k_coarse_solve<T>, grid, 256, n * sizeof(double), s, C, ainv, cidx, n);
 }
 
-template <typename T, bool VAR>
-void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s) {
-    launch_k(k_tail_cycle<T, VAR>, 1, kTailThreads, P.ncoarse * sizeof(double), s, P);
-}
-
 template <typename T>
 void launch_fill_ghosts(T* x, const int* dst, const int* src, long n, cudaStream_t s) {
     const int blocks = (int)std::min<long>((n + 255) / 256, 148L * 8);
@@ -1507,10 +1443,6 @@ template void launch_prolong_correct<float>(const Bricks<float>&, const Bricks<f
                                             cudaStream_t);
 template void launch_coarse_solve<double>(const Bricks<double>&, const double*, const int*, int, cudaStream_t);
 template void launch_coarse_solve<float>(const Bricks<float>&, const double*, const int*, int, cudaStream_t);
-template void launch_tail_cycle<double, false>(const TailPlan<double>&, cudaStream_t);
-template void launch_tail_cycle<double, true>(const TailPlan<double>&, cudaStream_t);
-template void launch_tail_cycle<float, false>(const TailPlan<float>&, cudaStream_t);
-template void launch_tail_cycle<float, true>(const TailPlan<float>&, cudaStream_t);
 template void launch_fill_ghosts<double>(double*, const int*, const int*, long, cudaStream_t);
 template void launch_fill_ghosts<float>(float*, const int*, const int*, long, cudaStream_t);
 template long launch_residual_norm<false>(const Bricks<double>&, const Walls&, int, double*, float*, cudaStream_t);

@@ -1,0 +1,60 @@
+"""The coarse end of a V or F cycle in one thread-block cluster (bmg_tail.cu)
+against the per-pass launches, over the shapes its planning takes: levels on
+one CTA and spread over several, extents that halve down to 2 and 3, rows of
+odd and even length, levels that stop halving along an axis, periodic,
+Dirichlet and variable-coefficient systems, V and F cycles, both precisions,
+and coarse solves spread over the cluster."""
+import numpy as np
+import pytest
+
+import briscola_b200 as bb
+from briscola_b200 import workloads
+from briscola_b200.mesh import DIRICHLET, NEUMANN, PERIODIC, Brick, Mesh, tanh_points, uniform_points
+
+pytestmark = pytest.mark.gpu
+
+P, N, D = (PERIODIC,) * 2, (NEUMANN,) * 2, (DIRICHLET,) * 2
+
+
+def _mesh(n, bc):
+    pts = [uniform_points(n[0]), tanh_points(n[1], 1.2), uniform_points(n[2])]
+    return Mesh([Brick(pts, sum(bc, ()))])
+
+
+CASES = [
+    ((8, 8, 8), (N, N, N), 1), ((16, 16, 16), (P, N, P), 1), ((32, 32, 32), (N, N, N), 1),
+    ((32, 16, 8), (P, D, P), 0), ((24, 12, 6), (D, N, N), 0), ((12, 24, 48), (N, N, D), 0),
+    ((6, 48, 16), (N, N, P), 1), ((64, 4, 16), (P, N, N), 0),
+    ((3, 24, 24), (N, D, N), 0), ((32, 32, 2), (N, N, P), 1), ((64, 32, 16), (P, N, P), 3),
+]
+
+
+@pytest.mark.parametrize("cycle", ["V", "F"])
+@pytest.mark.parametrize("n,bc,coarse", CASES)
+def test_cluster_tail_matches_per_pass(native, n, bc, coarse, cycle):
+    mesh = _mesh(n, bc)
+    rng = np.random.default_rng(5)
+    V = mesh.bricks[0].cell_volumes()
+    f = rng.standard_normal(n)
+    b = np.ascontiguousarray((-V * workloads.zero_mean(f, V)).ravel())
+    lam = [rng.uniform(0.5, 1.5, s) for s in ((n[0] + 1, n[1], n[2]), (n[0], n[1] + 1, n[2]), (n[0], n[1], n[2] + 1))]
+    for d in range(3):  # one coefficient on both ends of a periodic axis
+        if bc[d] == P:
+            np.moveaxis(lam[d], d, 0)[-1] = np.moveaxis(lam[d], d, 0)[0]
+    for precision in ("fp64", "mixed"):
+        for coef in (None, lam):
+            out = []
+            for fuse in ("on", "off"):
+                c = bb.Context(mesh, bb.make_options({
+                    "relTol": 0.0, "tolerance": 0, "minIter": 3, "maxIter": 3, "nSweepsPre": 2 if cycle == "V" else 0,
+                    "nSweepsPost": 2, "cycleType": cycle, "coarseLevel": coarse, "precision": precision,
+                    "fuseCoarse": fuse, "autotune": "off"}))
+                if coef is not None:
+                    c.set_coefficients(coef)
+                x = np.zeros_like(b)
+                rep = c.solve(b, x, zero_guess=True)
+                out.append((x, rep.kernel_launches))
+                c.close()
+            assert out[0][1] < out[1][1]  # the cluster ran
+            # the same operations cell by cell
+            assert np.array_equal(out[0][0], out[1][0]), (precision, coef is not None)
