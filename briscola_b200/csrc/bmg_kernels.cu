@@ -370,10 +370,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 && !VAR ? 5 : 1) k_colour_
     // the pinned cell (0,0,0), when this pass updates it, keeps its value
     if (L.pin && (i | j | h | m0) == 0) v[0] = ZERO ? T(0) : L.x[own];
     Vec16<T>::st(L.x + own, v);
+    // periodic images: a row inside the plane has two at most, of its first
+    // and last cell, stored as they are (every warp holds a row's end, and the
+    // general form of store_images took half the pass's instructions); the
+    // rows on a periodic i or j edge take the general form
     const bool edge_ij = (L.per0 && (i == 0 || i == L.n0 - 1)) || (L.per1 && (j == 0 || j == L.n1 - 1));
-    if (edge_ij || (L.per2 && (((h | m0) == 0) || (h == 1 && m0 + NC == kh)))) {
+    if (edge_ij) {
 #pragma unroll
         for (int m = 0; m < NC; ++m) store_images(L, own + m, i, j, 2 * (m0 + m) + h, v[m]);
+    } else if (L.per2) {
+        if ((h | m0) == 0) L.x[row + 2 * kh] = v[0];
+        if (h == 1 && m0 + NC == kh) L.x[row - 1] = v[NC - 1];
     }
     if constexpr (ZERO) {
         T zero[NC];
@@ -381,9 +388,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 && !VAR ? 5 : 1) k_colour_
         for (int m = 0; m < NC; ++m) zero[m] = T(0);
         Vec16<T>::st(L.x + oth, zero);
         const int ho = 1 - h;
-        if (edge_ij || (L.per2 && (((ho | m0) == 0) || (ho == 1 && m0 + NC == kh)))) {
+        if (edge_ij) {
 #pragma unroll
             for (int m = 0; m < NC; ++m) store_images(L, oth + m, i, j, 2 * (m0 + m) + ho, T(0));
+        } else if (L.per2) {
+            if ((ho | m0) == 0) L.x[row + 2 * kh] = T(0);
+            if (ho == 1 && m0 + NC == kh) L.x[row - 1] = T(0);
         }
     }
 }
@@ -886,13 +896,16 @@ __global__ void __launch_bounds__(256) k_prolong_split(Bricks<T> FB, Bricks<T> C
     }
     Row4<T>::st(F.x + ce, xe);
     Row4<T>::st(F.x + co, xo);
-    if ((F.per0 && (i == 0 || i == F.n0 - 1)) || (F.per1 && (j == 0 || j == F.n1 - 1)) ||
-        (F.per2 && (m0 == 0 || m0 + 4 == kh))) {
+    // periodic images, as in k_colour_split
+    if ((F.per0 && (i == 0 || i == F.n0 - 1)) || (F.per1 && (j == 0 || j == F.n1 - 1))) {
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             store_images(F, ce + m, i, j, 2 * (m0 + m), xe[m]);
             store_images(F, co + m, i, j, 2 * (m0 + m) + 1, xo[m]);
         }
+    } else if (F.per2) {
+        if (m0 == 0) F.x[row + 2 * kh] = xe[0];
+        if (m0 + 4 == kh) F.x[row - 1] = xo[3];
     }
 }
 
