@@ -1844,6 +1844,7 @@ void segBodyFcg(bmg_ctx* c, bool setCondition) {
 void segPostFcg(bmg_ctx* c, double* xdst) {
     cudaStream_t s = c->stream;
     const Bricks<double> V = fcgView(c);
+    if (launch_fcg_flush(V, c->fp, c->st, s)) c->launches += 1;
     exchangeField<double>(c, 0, c->fx);
     long n;
     if (c->variable)

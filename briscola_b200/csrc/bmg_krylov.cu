@@ -389,8 +389,13 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_step4(Bricks<double> B, 
 
 // The two passes on a parity-split level 0 (one brick): the thread owns four
 // consecutive positions of one half of a row, the cells k = 2 (m0 + e) + h of
-// one parity (as k_fcg_direction_split), so z, its neighbours and the FP64
-// vectors load as whole vectors.
+// one parity, so z, its neighbours and the FP64 vectors load as whole vectors.
+// Pass 2 is bound by memory, and x is the one vector no other step needs: it
+// moves every second step, x += alpha_prev p_prev + alpha p, when both
+// directions are at hand (k_fcg_flush adds a last odd one), 68 B a cell and
+// step on average instead of 76.  Forming q = A'p by the stencil on z +
+// beta p_prev instead of keeping it streams 56 B but was slower (290 us
+// against 257 at 256^3: twice the stencil loads in FP64, half the warps).
 #define BMG_SPLIT_AZ                                                                                   \
     const int h = 4 * qx >= kh ? 1 : 0;                                                                 \
     const int m0 = 4 * qx - h * kh;                                                                     \
@@ -456,6 +461,18 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_step4(Bricks<double> B, 
         }                                                                                               \
     }
 
+// the four x at c and their periodic images (as k_colour_split)
+__device__ __forceinline__ void store_split4(const LevelView<double>& L, int i, int j, int h, int m0, long row, long c,
+                                             const double v[4]) {
+    Quad4<double>::st(L.x + c, 0, v);
+    if ((L.per0 && (i == 0 || i == L.n0 - 1)) || (L.per1 && (j == 0 || j == L.n1 - 1))) {
+        for (int e = 0; e < 4; ++e) store_images(L, c + e, i, j, 2 * (m0 + e) + h, v[e]);
+    } else if (L.per2) {
+        if (h == 0 && m0 == 0) L.x[row + 2 * L.kh] = v[0];
+        if (h == 1 && m0 + 4 == L.kh) L.x[row - 1] = v[3];
+    }
+}
+
 template <typename T, bool VAR>
 __global__ void __launch_bounds__(kReduceThreads, VAR ? 2 : 3) k_fcg_dots3_split(Bricks<double> B, const T* z,
                                                                                   const double* r, const double* q,
@@ -493,31 +510,28 @@ __global__ void __launch_bounds__(kReduceThreads, VAR ? 2 : 3) k_fcg_step_split(
                                                                                  const SolveState* st) {
     grid_dep_sync();
     __shared__ double sh[kReduceThreads / 32];
-    const double beta = st->beta, alpha = st->alpha;
+    const double beta = st->beta, alpha = st->alpha, alpha_prev = st->alpha_prev;
+    const bool odd = st->iter & 1;  // x moves on odd steps
     double a = 0.0;
     BMG_SPLIT_LOOP({
         double pq[4], qq[4], xq[4], rq[4], rn[4];
         Quad4<double>::ld(p + c, 0, pq);
         Quad4<double>::ld(q + c, 0, qq);
-        Quad4<double>::ld(L.x + c, 0, xq);
+        if (odd) Quad4<double>::ld(L.x + c, 0, xq);
         Quad4<double>::ld(r + c, 0, rq);
         for (int e = 0; e < 4; ++e) {
             const double pn = beta != 0.0 ? (double)zc[e] + beta * pq[e] : (double)zc[e];
             const double qn = beta != 0.0 ? Az[e] + beta * qq[e] : Az[e];
+            if (odd) xq[e] = (xq[e] + alpha_prev * pq[e]) + alpha * pn;
             pq[e] = pn;
             qq[e] = qn;
-            xq[e] = xq[e] + alpha * pn;
             rn[e] = rq[e] - alpha * qn;
             const double Vr = (hij * hk[e]) * rn[e];
             a += Vr * Vr;
         }
         Quad4<double>::st(p + c, 0, pq);
         Quad4<double>::st(q + c, 0, qq);
-        Quad4<double>::st(L.x + c, 0, xq);
-        if ((L.per0 && (i == 0 || i == L.n0 - 1)) || (L.per1 && (j == 0 || j == L.n1 - 1)) ||
-            (L.per2 && ((h == 0 && m0 == 0) || (h == 1 && m0 + 4 == kh)))) {
-            for (int e = 0; e < 4; ++e) store_images(L, c + e, i, j, 2 * (m0 + e) + h, xq[e]);
-        }
+        if (odd) store_split4(L, i, j, h, m0, row, c, xq);
         Quad4<double>::st(r + c, 0, rn);
         if (pre32) {
             const float f[4] = {(float)rn[0], (float)rn[1], (float)rn[2], (float)rn[3]};
@@ -531,6 +545,27 @@ __global__ void __launch_bounds__(kReduceThreads, VAR ? 2 : 3) k_fcg_step_split(
 
 #undef BMG_SPLIT_LOOP
 #undef BMG_SPLIT_AZ
+
+// x += alpha p of a last even step, whose x the next step would have updated
+__global__ void __launch_bounds__(kReduceThreads) k_fcg_flush(Bricks<double> B, const double* p,
+                                                              const SolveState* st) {
+    grid_dep_sync();
+    if (!(st->iter & 1)) return;
+    const double alpha = st->alpha;
+    const LevelView<double>& L = B.v[0];
+    const int qx = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int h = 4 * qx >= L.kh ? 1 : 0, m0 = 4 * qx - h * L.kh;
+    if (j >= L.n1 || 4 * qx >= L.n2) return;
+    for (int i = blockIdx.z; i < L.n0; i += gridDim.z) {
+        const long row = row_at(L, i, j), c = row + 4 * qx;
+        double pq[4], xq[4];
+        Quad4<double>::ld(p + c, 0, pq);
+        Quad4<double>::ld(L.x + c, 0, xq);
+        for (int e = 0; e < 4; ++e) xq[e] = xq[e] + alpha * pq[e];
+        store_split4(L, i, j, h, m0, row, c, xq);
+    }
+}
 
 // The level-0 FP64 residual of k_residual_norm / k_fcg_residual on a
 // parity-split level (one brick): the thread owns four consecutive positions
@@ -653,6 +688,7 @@ __global__ void __launch_bounds__(kFinalThreads) k_fcg_coeffs(const double* part
         st->gamma = zr;
         st->beta = beta;
         st->pq = pq;
+        st->alpha_prev = st->alpha;
         st->alpha = zr / pq;
         st->first = 0;
     }
@@ -723,6 +759,12 @@ void launch_fcg_step(const Bricks<double>& B, const T* z, double* p, double* q, 
     launch_k(k_fcg_direction<T, VAR>, g, blk, 0, s, B, z, p, q, partials, st);
     launch_k(k_fcg_alpha, 1, kFinalThreads, 0, s, partials, nb, st);
     launch_k(k_fcg_update, g, blk, 0, s, B, p, r, q, pre32, pre64, partials, st);
+}
+
+bool launch_fcg_flush(const Bricks<double>& B, const double* p, const SolveState* st, cudaStream_t s) {
+    if (!B.v[0].kh) return false;
+    launch_k(k_fcg_flush, quad_grid(B), dim3(16, 16, 1), 0, s, B, p, st);
+    return true;
 }
 
 int fcg_step_launches(const Bricks<double>& B) { return fcg_quads(B) ? 3 : 5; }
