@@ -21,7 +21,8 @@ SOURCES = ["bmg_host.cu", "bmg_kernels.cu", "bmg_smooth_fused.cu", "bmg_krylov.c
 HEADERS = ["bmg_internal.h", "bmg_stencil.cuh", "bmg_grid.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FFT_OUT = os.path.join(HERE, "_lib", "libbfft.so")
-FFT_SOURCES = ["bfft.cu"]
+FFT_SOURCES = ["bfft.cu", "bfft_pair.cu", "bfft_tri.cu"]
+FFT_HEADERS = ["bfft_internal.h"]
 UNET_OUT = os.path.join(HERE, "_lib", "libbunet.so")
 UNET_SOURCES = ["bun_api.cu", "bun_conv.cu", "bun_elem.cu"]
 UNET_HEADERS = ["bun_internal.h", "bun_api_internal.h"]
@@ -58,7 +59,7 @@ def build_native(force: bool = False, verbose: bool = False) -> str:
 
 def build_fft(force: bool = False, verbose: bool = False) -> str:
     """libbfft.so (the FFT Poisson solver, include/bfft.h); returns its path."""
-    return _build(FFT_OUT, FFT_SOURCES, [], "bfft.h", force, verbose)
+    return _build(FFT_OUT, FFT_SOURCES, FFT_HEADERS, "bfft.h", force, verbose)
 
 
 def build_unet(force: bool = False, verbose: bool = False) -> str:

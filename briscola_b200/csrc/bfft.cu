@@ -8,18 +8,15 @@
 //   prep        -b - shift x_old - face terms, times 1/normalisation
 //               (FFTPoissonSolver.C:116-183; the reference divides at the
 //               end, FourierTransforms.C:414-420 -- the steps are linear)
-//   transforms  k_transform along each transform axis: a CTA loads a tile
-//               of lines into shared memory, runs one radix-2 complex FFT of
-//               length M per line and writes the line back.  Every FFTW r2r
-//               kind the reference uses is one zero-padded FFT with a
-//               pre-twiddle of the input and a post-twiddle of the output:
-//               REDFT10/01/11 and RODFT10/01/11 with M = 2N, R2HC/HC2R with
-//               M = N (FourierTransforms.C:228-242).
-//   tridiagonal k_tridiag: one thread per mode marches along the solve
-//               axis (Thomas, or the cyclic two-system form for a periodic
-//               solve axis, tridiagonalSolver.C:330-450); lines of
-//               consecutive k are consecutive threads, so every step is a
-//               coalesced load or store.
+//   transforms  along each transform axis, every FFTW r2r kind the reference
+//               uses (FourierTransforms.C:228-242): the periodic, D-D and N-N
+//               kinds as two lines per N-point complex FFT (bfft_pair.cu;
+//               lines of at most 16 points: k_transform), the quarter-wave
+//               kinds as one zero-padded 2N-point FFT (k_transform)
+//   tridiagonal along the solve axis (tridiagonalSolver.C:330-450): each line
+//               shared by many threads (bfft_tri.cu), or for a periodic solve
+//               axis and very long lines one thread per mode marching along
+//               it (k_tridiag, k_tri_apply)
 // Along the strided axes a transform tile is a run of consecutive k, so its
 // loads and stores are runs of contiguous doubles too.
 
@@ -33,162 +30,11 @@
 #include <vector>
 
 #include "../../include/bfft.h"
+#include "bfft_internal.h"
 
 struct bfft_ctx;
 
 namespace bfft {
-
-// boundary pair of an axis (FourierTransforms.C:130-226)
-enum Pair { P_EMPTY = 0, P_DD = 1, P_NN = 2, P_DN = 3, P_ND = 4, P_CC = 5 };
-// output of a transform: halfcomplex of Z, Re(Z), Re(post Z), -Im(post Z)
-enum Mode { M_R2HC = 0, M_HC2R = 1, M_RE = 2, M_NEG_IM = 3 };
-
-constexpr int kThreads = 256;
-constexpr int kMaxN = 512;
-
-// lines along one axis: line l starts at (l / inner) * outer + (l % inner) * inner_stride
-struct Lines {
-    int n;             // cells along the axis
-    long stride;       // element stride along the axis
-    long inner;        // lines per outer index
-    long inner_stride;
-    long outer_stride;
-    long count;
-    int line_fast;     // consecutive lines are adjacent in memory (strided axes)
-};
-
-struct Transform {
-    int M, logM, mode;
-    int kind;             // Kind
-    int odd;              // K_DCT2 / K_DCT3: the sine kinds RODFT10 / RODFT01
-    int logN;             // log2 of the line length (transformed extents are powers of two)
-    int logLB;            // log2 of the lines per CTA
-    const double2* pre;   // n entries, nullptr: 1
-    const double2* post;  // n entries, nullptr: 1
-    const double2* tw;    // M entries: exp(-2 pi i q / M)
-};
-
-struct Tri {
-    int ns, cyclic;
-    double shift;
-    double s0;            // first diagonal entry of a pinned (singular) mode
-    int pin;              // the solve direction is N-N or periodic: the mode whose two
-                          // eigenvalues are zero is singular and pinned (tridiagonalSolver.C)
-    const double* A;      // D_k = ((e - A_k) - B_k)
-    const double* B;
-    const double* DU;
-    const double* DL;
-    const double* ev1;    // eigenvalue / h^2 of the first transform direction
-    const double* ev2;
-    int dir1_inner;       // the first transform direction is the inner line coordinate
-    // modes with equal eigenvalues share one factorisation: class of each
-    // inner / outer line coordinate, a representative coordinate per class
-    const int* clsI;
-    const int* clsO;
-    const int* repI;
-    const int* repO;
-    int nci, nco;
-    double* mfac;         // [ns][modes]: DL_k / Dh_{k-1}
-    double* rfac;         // [ns][modes]: 1 / Dh_k
-};
-
-constexpr int kTriAhead = 8;  // rows a tridiagonal sweep loads ahead
-constexpr int kSplitBlocks = 592;  // partial maxima of the face coefficients
-
-struct Prep {
-    int n0, n1, n2;
-    double shift, scale;
-    double corr[6];       // face terms subtracted on the boundary cells of each face
-};
-
-__device__ __forceinline__ long line_base(const Lines& L, long l) {
-    // along axes 0 and 2 the outer stride is inner * inner_stride: no division
-    if (L.outer_stride == L.inner * L.inner_stride) return l * L.inner_stride;
-    const unsigned lu = (unsigned)l, in = (unsigned)L.inner;  // line counts fit 32 bits
-    const unsigned o = lu / in;
-    return (long)o * L.outer_stride + (long)(lu - o * in) * L.inner_stride;
-}
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// cos and sin of a pi / 8, a = 0..7: the twiddles of the register DFTs (R <= 16)
-__host__ __device__ constexpr double cos8(int a) {
-    return a == 0   ? 1.0
-           : a == 1 ? 0.92387953251128675613
-           : a == 2 ? 0.70710678118654752440
-           : a == 3 ? 0.38268343236508977173
-           : a == 4 ? 0.0
-           : a == 5 ? -0.38268343236508977173
-           : a == 6 ? -0.70710678118654752440
-                    : -0.92387953251128675613;
-}
-__host__ __device__ constexpr double sin8(int a) { return a <= 4 ? cos8(4 - a) : cos8(a - 4); }
-
-__host__ __device__ constexpr int brev_c(int i, int logR) {
-    int r = 0;
-    for (int b = 0; b < logR; ++b) r |= ((i >> b) & 1) << (logR - 1 - b);
-    return r;
-}
-
-// x * exp(-i pi p / h) for compile-time p < h <= 8
-template <int P, int H>
-__device__ __forceinline__ double2 rot(double2 x) {
-    constexpr int a = P * (8 / H);
-    if constexpr (a == 0) {
-        return x;
-    } else if constexpr (a == 4) {
-        return make_double2(x.y, -x.x);
-    } else {
-        constexpr double c = cos8(a), sn = sin8(a);
-        return make_double2(x.x * c + x.y * sn, x.y * c - x.x * sn);
-    }
-}
-
-template <int H, int I, int P, int R>
-__device__ __forceinline__ void bfly(double2 (&v)[R]) {
-    const double2 u = v[I + P];
-    const double2 t = rot<P, H>(v[I + P + H]);
-    v[I + P] = make_double2(u.x + t.x, u.y + t.y);
-    v[I + P + H] = make_double2(u.x - t.x, u.y - t.y);
-}
-
-template <int H, int I, int P, int R>
-__device__ __forceinline__ void bfly_group(double2 (&v)[R]) {
-    if constexpr (P < H) {
-        bfly<H, I, P, R>(v);
-        bfly_group<H, I, P + 1, R>(v);
-    }
-}
-
-template <int H, int I, int R>
-__device__ __forceinline__ void bfly_stage(double2 (&v)[R]) {
-    if constexpr (I < R) {
-        bfly_group<H, I, 0, R>(v);
-        bfly_stage<H, I + 2 * H, R>(v);
-    }
-}
-
-template <int H, int R>
-__device__ __forceinline__ void bfly_stages(double2 (&v)[R]) {
-    if constexpr (H < R) {
-        bfly_stage<H, 0, R>(v);
-        bfly_stages<2 * H, R>(v);
-    }
-}
-
-// in-register DFT of R points (natural order in and out): bit reversal,
-// then radix-2 stages with the exact twiddles of kCos8 / kSin8
-template <int R, int LOGR>
-__device__ __forceinline__ void dft_regs(double2 (&v)[R]) {
-    double2 t[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) t[i] = v[brev_c(i, LOGR)];
-#pragma unroll
-    for (int i = 0; i < R; ++i) v[i] = t[i];
-    bfly_stages<1, R>(v);
-}
 
 constexpr int kTransformThreads = 128;
 constexpr int kTileComplex = 2048;                              // complex values of a tile (LB lines of M)
@@ -298,49 +144,6 @@ __device__ __forceinline__ void stockham_all(double2* __restrict__ buf, const do
         stockham_pass<2, 1, LOGM, LOGNS, LB>(buf, tw);
     }
 }
-
-// the prep of the first transform's input: -b - shift x_old - face terms,
-// times 1/normalisation (FFTPoissonSolver.C:116-183)
-struct LoadPrep {
-    int on;
-    int axis;             // the transform axis
-    int n1, n2;
-    const double* xo;     // nullptr: no ddt term
-    Prep P;
-};
-
-__device__ __forceinline__ void cp8(void* smem, const void* gmem, bool valid) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(valid ? 8 : 0)
-                 : "memory");
-}
-// 16 bytes, of which `bytes` (0, 8 or 16) are read and the rest zero-filled
-__device__ __forceinline__ void cp16(void* smem, const void* gmem, int bytes) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Transform kinds.  K_TRIG: one zero-padded M = 2N point complex FFT per
-// line with a pre-twiddle of the input and a post-twiddle of the output
-// (the quarter-wave kinds REDFT11 / RODFT11).  The others put two real lines
-// into one N-point complex FFT (line 2u as the real part, line 2u + 1 as the
-// imaginary part) and separate the two spectra afterwards from
-// Z(k) and conj Z(N - k):
-//   K_R2HC  forward real FFT, halfcomplex output
-//   K_HC2R  inverse real FFT of halfcomplex input (unnormalised)
-//   K_DCT2  REDFT10 by Makhoul's reordering (J. Makhoul, "A fast cosine
-//           transform in one and two dimensions", IEEE TASSP 28 (1980)):
-//           v = (x0, x2, x4, ..., x5, x3, x1), X_k = 2 Re(e^{-i pi k/2N} V_k);
-//           with `odd`, RODFT10 as REDFT10 of (-1)^n x_n, read backwards
-//   K_DCT3  REDFT01, the inverse of that reordering: V_k = e^{i pi k/2N}
-//           (X_k - i X_{N-k}) (X_N = 0), v = IDFT(V), x_2n = v_n,
-//           x_2n+1 = v_{N-1-n}; with `odd`, RODFT01 as (-1)^n REDFT01 of
-//           the reversed input
-// so every kind the solver meets on a periodic, Dirichlet-Dirichlet or
-// Neumann-Neumann axis costs half an N-point complex FFT per line.
-enum Kind { K_R2HC = 0, K_HC2R = 1, K_TRIG = 2, K_DCT2 = 3, K_DCT3 = 4 };
 
 // the slot of point p in Makhoul's reordering (even points first, then the
 // odd ones backwards)
@@ -989,14 +792,15 @@ __global__ void k_prep(double* __restrict__ w, const double* __restrict__ b, con
     }
 }
 
-// the line lengths of a kind: M = N = 1 .. kMaxN for the paired kinds,
-// M = 2N = 2 .. 2 kMaxN for K_TRIG
+// the line lengths this kernel takes: M = N = 1 .. 16 for the paired kinds
+// (longer lines: bfft_pair.cu), M = 2N = 2 .. 2 kMaxN for K_TRIG
 constexpr int kMinLogM(int kind) { return kind == K_TRIG ? 1 : 0; }
+constexpr int kMaxLogM(int kind) { return kind == K_TRIG ? 10 : kPairMinLog - 1; }
 
 template <int KIND, bool LF, int LOGM = kMinLogM(KIND)>
 void launch_kind(int logM, unsigned grid, cudaStream_t st, const double* in, double* out, const Lines& L,
                  const Transform& T, const LoadPrep& lp, long tiles, int pair) {
-    if constexpr (LOGM <= kMinLogM(KIND) + 9) {
+    if constexpr (LOGM <= kMaxLogM(KIND)) {
         if (logM == LOGM)
             k_transform<LOGM, KIND, LF><<<grid, kTransformThreads, kTransformSmem, st>>>(in, out, L, T, lp, tiles, pair);
         else
@@ -1026,7 +830,7 @@ void launch_transform(int kind, int logM, unsigned grid, cudaStream_t st, const 
 
 template <int KIND, bool LF, int LOGM = kMinLogM(KIND)>
 void allow_kind() {
-    if constexpr (LOGM <= kMinLogM(KIND) + 9) {
+    if constexpr (LOGM <= kMaxLogM(KIND)) {
         cudaFuncSetAttribute(k_transform<LOGM, KIND, LF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kTransformSmem);
         allow_kind<KIND, LF, LOGM + 1>();
@@ -1093,6 +897,7 @@ struct bfft_ctx {
     bool ownStream = false;
     SplitGeom split{};
     double* part = nullptr;     // reduction partials (split solver)
+    int triLines = 0;           // lines of a tridiagonal CTA, 0: k_tri_apply
     bool factored = false;      // the Thomas factors hold for factorShift
     double factorShift = 0.0;
     std::string err;
@@ -1375,11 +1180,16 @@ void build(bfft_ctx* c, const bfft_desc* d) {
     T.nci = (int)rI.size();
     T.nco = (int)rO.size();
     if (!T.cyclic) {
-        const size_t f = (size_t)T.nci * T.nco * ns;
-        T.mfac = dalloc<double>(f);
-        T.rfac = dalloc<double>(f);
-        c->owned.push_back(T.mfac);
+        // one factor per row where a line's threads fit a CTA (bfft_tri.cu),
+        // two for the march through memory (k_tri_apply)
+        c->triLines = tri_tile_lines(ns, c->solveLines.count, c->sms);
+        const size_t modes = (size_t)T.nci * T.nco;
+        T.rfac = dalloc<double>(modes * ns);
         c->owned.push_back(T.rfac);
+        if (!c->triLines) {
+            T.mfac = dalloc<double>(modes * ns);
+            c->owned.push_back(T.mfac);
+        }
     }
 
     // right-hand side terms of the faces (FFTPoissonSolver.C:140-183)
@@ -1452,6 +1262,10 @@ int guarded(bfft_ctx* c, F&& f) {
 void transform(bfft_ctx* c, int a, bool forward, const double* in, double* out, const LoadPrep& lp) {
     const AxisPlan& A = c->ax[a];
     const Transform& T = forward ? A.fwd : A.bwd;
+    if (T.kind != K_TRIG && T.logN >= kPairMinLog) {
+        check(launch_pair(in, out, A.lines, T, lp, A.adjacent, c->stream), "k_pair");
+        return;
+    }
     const long tiles = (A.lines.count + A.LB - 1) / A.LB;
     // persistent: as many CTAs as fit at once (three per SM)
     const long grid = std::min<long>(tiles, 3L * c->sms);
@@ -1548,8 +1362,12 @@ int bfft_solve(bfft_ctx* c, const double* b, double* x, const double* x_old, dou
         T.shift = shift;
         if (!T.cyclic && (!c->factored || c->factorShift != shift)) {
             const int modes = T.nci * T.nco;
-            k_tri_factor<<<(modes + 127) / 128, 128, 0, c->stream>>>(T);
-            check(cudaGetLastError(), "k_tri_factor");
+            if (c->triLines) {
+                check(launch_tri_factor(T, c->stream), "k_tri_factor");
+            } else {
+                k_tri_factor<<<(modes + 127) / 128, 128, 0, c->stream>>>(T);
+                check(cudaGetLastError(), "k_tri_factor");
+            }
             c->factored = true;
             c->factorShift = shift;
         }
@@ -1557,6 +1375,8 @@ int bfft_solve(bfft_ctx* c, const double* b, double* x, const double* x_old, dou
         if (T.cyclic)
             k_tridiag<<<(unsigned)((lines + kThreads - 1) / kThreads), kThreads, 0, c->stream>>>(c->w, c->dh, c->vv,
                                                                                               c->solveLines, T);
+        else if (c->triLines)
+            check(launch_tri_chunks(c->w, c->solveLines, T, c->triLines, c->stream), "k_tri_chunks");
         else
             k_tri_apply<<<(unsigned)((lines + kThreads - 1) / kThreads), kThreads, 0, c->stream>>>(c->w, c->solveLines,
                                                                                                 T);
