@@ -665,24 +665,40 @@ __global__ void __launch_bounds__(kThreads) k_tri_apply(double* __restrict__ w, 
 
 // ---- split Poisson solver -------------------------------------------------
 
+// The face gradients of an axis as one formula: the outward flux term of
+// cell q's lower (upper) face is lambda' (w (x_nb - x_c) + g), over the cell
+// size, with w = 1 / (distance h_q), the neighbour's x, or at a face with a
+// condition (DirichletBoundaryCondition.C:51-71, NeumannBoundaryCondition.C
+// :59-85) w = 2 / (h h) and the value for x_nb (Dirichlet), or w = 0 and
+// g = gradient / h (Neumann); both 0 on an empty axis.
 struct SplitGeom {
     int n[3];
-    const double* h[3];   // cell sizes per axis
-    int bc[6];            // BFFT_BC_* per face
-    double value[6];      // Dirichlet value or Neumann gradient
+    int per[3];
+    const double* w[3];   // 2 n_d entries: lower, then upper
+    double value[6];      // x_nb at a Dirichlet face
+    double g[6];
 };
 
-// largest of the three face arrays: per-block maxima, then one block
-__global__ void k_max3(const double* __restrict__ a, long na, const double* __restrict__ b, long nb,
-                       const double* __restrict__ c, long nc, double* __restrict__ part) {
-    double m = -1e308;
+// largest of the three face arrays: per-block maxima, then one block; four
+// independent loads a thread
+__global__ void __launch_bounds__(kThreads) k_max3(const double* __restrict__ a, long na, const double* __restrict__ b,
+                                                   long nb, const double* __restrict__ c, long nc,
+                                                   double* __restrict__ part) {
+    double m[4] = {-1e308, -1e308, -1e308, -1e308};
     const long stride = (long)gridDim.x * blockDim.x;
-    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < na + nb + nc; q += stride) {
-        const double v = q < na ? a[q] : q < na + nb ? b[q - na] : c[q - na - nb];
-        m = fmax(m, v);
+    const double* const src[3] = {a, b, c};
+    const long len[3] = {na, nb, nc};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+        for (; q + 3 * stride < len[d]; q += 4 * stride) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) m[e] = fmax(m[e], src[d][q + e * stride]);
+        }
+        for (; q < len[d]; q += stride) m[0] = fmax(m[0], src[d][q]);
     }
     __shared__ double sm[kThreads];
-    sm[threadIdx.x] = m;
+    sm[threadIdx.x] = fmax(fmax(m[0], m[1]), fmax(m[2], m[3]));
     __syncthreads();
     for (int w = kThreads / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + w]);
@@ -704,68 +720,48 @@ __global__ void k_max_final(double* __restrict__ part, int n) {
     if (threadIdx.x == 0) part[0] = sm[0];
 }
 
-// one face's flux term lambda' (x_nb - x_c) delta, with the neighbour or the
-// ghost the face condition sets (DirichletBoundaryCondition.C:51-71,
-// NeumannBoundaryCondition.C:59-85; mirrored ghost cells: delta = 1/h)
-__device__ __forceinline__ double face_term(const SplitGeom& G, int axis, int side, int idx, double lamp, double xc,
-                                            double xnb, bool boundary, double delta) {
-    if (!boundary) return lamp * (xnb - xc) * delta;
-    const int f = 2 * axis + side;
-    const int bc = G.bc[f];
-    if (bc == BFFT_BC_NEUMANN) return lamp * G.value[f];  // (x_g - x_c) delta = g
-    if (bc == BFFT_BC_DIRICHLET) return lamp * (2.0 * G.value[f] - 2.0 * xc) * delta;
-    return 0.0;  // empty
-}
-
-// bhat = b / lambda0 + div((lambda / lambda0 - 1) faceGrad(x) faceArea)
-__global__ void k_split_source(const double* __restrict__ x, const double* __restrict__ b,
-                               const double* __restrict__ lam0, const double* __restrict__ lam1,
-                               const double* __restrict__ lam2, double lambda0, double* __restrict__ bhat,
-                               SplitGeom G) {
+// bhat = b / lambda0 + div((lambda / lambda0 - 1) faceGrad(x) faceArea).
+// Memory bounds it (48 B a cell); the divisions (one a face term and two a
+// face coefficient before) are tables and one reciprocal, since 24 FP64
+// divisions a cell took five times the memory's time.
+__global__ void __launch_bounds__(256) k_split_source(const double* __restrict__ x, const double* __restrict__ b,
+                                                      const double* __restrict__ lam0, const double* __restrict__ lam1,
+                                                      const double* __restrict__ lam2, double lambda0, double inv0,
+                                                      double* __restrict__ bhat, const __grid_constant__ SplitGeom G) {
     const int n1 = G.n[1], n2 = G.n[2];
-    // one CTA row of k per (i, j): grid (k chunks, n1, n0)
-    const int i = blockIdx.z, j = blockIdx.y;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n2; k += gridDim.x * blockDim.x) {
-        const long c = ((long)i * n1 + j) * n2 + k;
-        const int ijk[3] = {i, j, k};
-        const long sx[3] = {(long)n1 * n2, n2, 1};
-        const double xc = x[c];
-        double div = 0.0;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (k >= n2 || j >= n1) return;
+    const long c = ((long)i * n1 + j) * n2 + k;
+    const int at[3] = {i, j, k};
+    const long sx[3] = {(long)n1 * n2, n2, 1};
+    const double* const lam[3] = {lam0, lam1, lam2};
+    // lower faces; the upper one is one face further along the axis
+    const long fl[3] = {c, ((long)i * (n1 + 1) + j) * n2 + k, ((long)i * n1 + j) * (n2 + 1) + k};
+    const double xc = x[c];
+    double div = 0.0;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const int q = ijk[a], n = G.n[a];
-            const double* h = G.h[a];
-            const bool per = G.bc[2 * a] == BFFT_BC_PERIODIC;
-            const double hc = h[q];
-            // lower and upper faces of the cell along axis a
-            const double hlo = q > 0 ? h[q - 1] : (per ? h[n - 1] : hc);
-            const double hhi = q < n - 1 ? h[q + 1] : (per ? h[0] : hc);
-            const double dw = 0.5 * (hc + hlo), de = 0.5 * (hc + hhi);
-            long flo, fhi;  // face indices in the face array of axis a
-            if (a == 0) {
-                flo = ((long)i * n1 + j) * n2 + k;
-                fhi = ((long)(i + 1) * n1 + j) * n2 + k;
-            } else if (a == 1) {
-                flo = ((long)i * (n1 + 1) + j) * n2 + k;
-                fhi = ((long)i * (n1 + 1) + j + 1) * n2 + k;
-            } else {
-                flo = ((long)i * n1 + j) * (n2 + 1) + k;
-                fhi = flo + 1;
-            }
-            const double* lam = a == 0 ? lam0 : a == 1 ? lam1 : lam2;
-            const double llo = lam[flo] / lambda0 - 1.0, lhi = lam[fhi] / lambda0 - 1.0;
-            const bool blo = q == 0 && !per, bhi = q == n - 1 && !per;
-            double xlo = 0.0, xhi = 0.0;
-            if (!blo) xlo = x[q > 0 ? c - sx[a] : c + (long)(n - 1) * sx[a]];
-            if (!bhi) xhi = x[q < n - 1 ? c + sx[a] : c - (long)(n - 1) * sx[a]];
-            // lower face: outward gradient (x_lo - x_c) delta; upper face enters with a minus sign
-            // of its own outward gradient, i.e. (x_hi - x_c) delta
-            const double tlo = face_term(G, a, 0, q, llo, xc, xlo, blo, 1.0 / dw);
-            const double thi = face_term(G, a, 1, q, lhi, xc, xhi, bhi, 1.0 / de);
-            div += (tlo + thi) / hc;
+    for (int a = 0; a < 3; ++a) {
+        const int q = at[a], n = G.n[a];
+        // lambda / lambda0 - 1, exactly zero where lambda is lambda0
+        const double llo = (lam[a][fl[a]] - lambda0) * inv0, lhi = (lam[a][fl[a] + sx[a]] - lambda0) * inv0;
+        double xlo, xhi, glo = 0.0, ghi = 0.0;
+        if (q > 0 || G.per[a]) {
+            xlo = x[q > 0 ? c - sx[a] : c + (n - 1) * sx[a]];
+        } else {
+            xlo = G.value[2 * a];
+            glo = G.g[2 * a];
         }
-        bhat[c] = b[c] / lambda0 + div;
+        if (q < n - 1 || G.per[a]) {
+            xhi = x[q < n - 1 ? c + sx[a] : c - (n - 1) * sx[a]];
+        } else {
+            xhi = G.value[2 * a + 1];
+            ghi = G.g[2 * a + 1];
+        }
+        div += llo * (G.w[a][q] * (xlo - xc) + glo) + lhi * (G.w[a][n + q] * (xhi - xc) + ghi);
     }
+    bhat[c] = b[c] * inv0 + div;
 }
 
 __global__ void k_axpby(double a, const double* x, double c, const double* y, double* out, long n) {
@@ -1216,13 +1212,25 @@ void build(bfft_ctx* c, const bfft_desc* d) {
     }
 
     // geometry of the split solver's source kernel
+    SplitGeom& G = c->split;
     for (int a = 0; a < 3; ++a) {
-        c->split.n[a] = c->n[a];
-        c->split.h[a] = upload(c, h[a]);
-    }
-    for (int f = 0; f < 6; ++f) {
-        c->split.bc[f] = d->bc[f];
-        c->split.value[f] = d->value[f];
+        const int n = c->n[a];
+        G.n[a] = n;
+        G.per[a] = c->ax[a].pair == P_CC;
+        std::vector<double> w(2 * n);
+        for (int q = 0; q < n; ++q)
+            for (int side = 0; side < 2; ++side) {
+                const int f = 2 * a + side;
+                const bool wall = q == (side ? n - 1 : 0) && !G.per[a];
+                // mirrored ghost cells beyond a wall
+                const double hn = wall ? h[a][q] : h[a][(q + (side ? 1 : n - 1)) % n];
+                const double v = 1.0 / (0.5 * (h[a][q] + hn) * h[a][q]);
+                w[side * n + q] = !wall ? v : d->bc[f] == BFFT_BC_DIRICHLET ? 2.0 * v : 0.0;
+                if (!wall) continue;
+                G.value[f] = d->bc[f] == BFFT_BC_DIRICHLET ? d->value[f] : 0.0;
+                G.g[f] = d->bc[f] == BFFT_BC_NEUMANN ? d->value[f] / h[a][q] : 0.0;
+            }
+        G.w[a] = upload(c, w);
     }
     c->part = dalloc<double>(kSplitBlocks);
     c->owned.push_back(c->part);
@@ -1420,8 +1428,9 @@ int bfft_split_source(bfft_ctx* c, const double* x, const double* b, const doubl
     if (!c || !x || !b || !lam0 || !lam1 || !lam2 || !bhat || !(lambda0 > 0.0)) return BMG_BAD_ARG;
     return guarded(c, [&] {
         check(cudaSetDevice(c->dev), "cudaSetDevice");
-        const dim3 grid((unsigned)std::min((c->n[2] + 127) / 128, 8), (unsigned)c->n[1], (unsigned)c->n[0]);
-        k_split_source<<<grid, 128, 0, c->stream>>>(x, b, lam0, lam1, lam2, lambda0, bhat, c->split);
+        const dim3 block = c->n[2] > 32 ? dim3(64, 4) : dim3(32, 8);
+        const dim3 grid((c->n[2] + block.x - 1) / block.x, (c->n[1] + block.y - 1) / block.y, c->n[0]);
+        k_split_source<<<grid, block, 0, c->stream>>>(x, b, lam0, lam1, lam2, lambda0, 1.0 / lambda0, bhat, c->split);
         check(cudaGetLastError(), "k_split_source");
         return (int)BMG_OK;
     });

@@ -25,68 +25,80 @@ namespace bmg {
 
 namespace {
 
-__global__ void k_project_rhs(const double* __restrict__ u0, const double* __restrict__ u1,
-                              const double* __restrict__ u2, double* __restrict__ out, ProjGeom G) {
+// Both kernels stream the face arrays once, one cell (or face index) a
+// thread over blocks of whole runs along k and several rows: memory bounds
+// them, and on small bricks the number of CTAs does (a CTA of one row kept
+// the 128 x 96 x 64 step's four launches at 10-14 us each).
+__global__ void __launch_bounds__(256) k_project_rhs(const double* __restrict__ u0, const double* __restrict__ u1,
+                                                     const double* __restrict__ u2, double* __restrict__ out,
+                                                     ProjGeom G) {
     const int n1 = G.n[1], n2 = G.n[2];
-    const int i = blockIdx.z, j = blockIdx.y;
-    const double h0 = G.h[0][i], h1 = G.h[1][j];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n2; k += gridDim.x * blockDim.x) {
-        const long f0 = ((long)i * n1 + j) * n2 + k;
-        const long f1 = ((long)i * (n1 + 1) + j) * n2 + k;
-        const long f2 = ((long)i * n1 + j) * (n2 + 1) + k;
-        const double h2 = G.h[2][k];
-        // sum of U A over the faces, then divided by V (A / V = 1 / h along each axis)
-        const double div = (u0[f0 + (long)n1 * n2] - u0[f0]) / h0 + (u1[f1 + n2] - u1[f1]) / h1 +
-                           (u2[f2 + 1] - u2[f2]) / h2;
-        const double b = div / (-G.cdt);
-        out[((long)i * n1 + j) * n2 + k] = G.perVolume ? b : -(h0 * h1 * h2) * b;
-    }
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (k >= n2 || j >= n1) return;
+    const double h0 = G.h[0][i], h1 = G.h[1][j], h2 = G.h[2][k];
+    const long f0 = ((long)i * n1 + j) * n2 + k;
+    const long f1 = ((long)i * (n1 + 1) + j) * n2 + k;
+    const long f2 = ((long)i * n1 + j) * (n2 + 1) + k;
+    // sum of U A over the faces, then divided by V (A / V = 1 / h along each axis)
+    const double div = (u0[f0 + (long)n1 * n2] - u0[f0]) / h0 + (u1[f1 + n2] - u1[f1]) / h1 +
+                       (u2[f2 + 1] - u2[f2]) / h2;
+    const double b = div / (-G.cdt);
+    out[f0] = G.perVolume ? b : -(h0 * h1 * h2) * b;
 }
 
-// faces of axis A: grid over (faces along k for A == 2 / cells along k, rows)
-template <int A>
-__global__ void k_project_correct(double* __restrict__ u, const double* __restrict__ p,
-                                  const double* __restrict__ lam, ProjGeom G) {
+// The three faces of index (i, j, k): those below cell (i, j, k) along each
+// axis, and the top faces where i = n0, j = n1 or k = n2.  One pass: p is read
+// once for the three axes.
+__global__ void __launch_bounds__(256) k_project_correct(double* __restrict__ u0, double* __restrict__ u1,
+                                                         double* __restrict__ u2, const double* __restrict__ p,
+                                                         const double* __restrict__ lam0,
+                                                         const double* __restrict__ lam1,
+                                                         const double* __restrict__ lam2, ProjGeom G) {
     const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
-    const int i = blockIdx.z, j = blockIdx.y;  // face coordinates (the face index along A is i, j or k)
-    const int e0 = A == 0 ? n0 + 1 : n0, e1 = A == 1 ? n1 + 1 : n1, e2 = A == 2 ? n2 + 1 : n2;
-    if (i >= e0 || j >= e1) return;
-    const int nA = G.n[A];
-    const double* h = G.h[A];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < e2; k += gridDim.x * blockDim.x) {
-        const int q = A == 0 ? i : A == 1 ? j : k;  // face index along A
-        const long f = ((long)i * e1 + j) * e2 + k;
-        int qc = q, ql = q - 1;  // cells above and below the face
-        if (q == 0 || q == nA) {
-            if (!G.per[A]) continue;  // a wall: zero gradient
+    const int q[3] = {(int)blockIdx.z, (int)(blockIdx.y * blockDim.y + threadIdx.y),
+                      (int)(blockIdx.x * blockDim.x + threadIdx.x)};
+    const int i = q[0], j = q[1], k = q[2];
+    if (j > n1 || k > n2) return;
+    double* const us[3] = {u0, u1, u2};
+    const double* const ls[3] = {lam0, lam1, lam2};
+    const long st[3] = {(long)n1 * n2, n2, 1};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int nA = G.n[a];
+        if ((a != 0 && i == n0) || (a != 1 && j == n1) || (a != 2 && k == n2)) continue;
+        const int e1 = a == 1 ? n1 + 1 : n1, e2 = a == 2 ? n2 + 1 : n2;
+        int qc = q[a], ql = q[a] - 1;  // cells above and below the face
+        if (qc == 0 || qc == nA) {
+            if (!G.per[a]) continue;  // a wall: zero gradient
             qc = 0;  // across the periodic seam: the first and the last cell
             ql = nA - 1;
         }
-        const double delta = 1.0 / (0.5 * (h[qc] + h[ql]));
-        auto cell = [&](int qq) {
-            const int ci = A == 0 ? qq : i, cj = A == 1 ? qq : j, ck = A == 2 ? qq : k;
-            return ((long)ci * n1 + cj) * n2 + ck;
-        };
-        const double g = (p[cell(qc)] - p[cell(ql)]) * delta;
-        const double l = lam ? lam[f] : 1.0;
-        u[f] -= G.cdt * (l * g);
+        const double delta = 1.0 / (0.5 * (G.h[a][qc] + G.h[a][ql]));
+        const long other = (a == 0 ? 0 : i * st[0]) + (a == 1 ? 0 : j * st[1]) + (a == 2 ? 0 : (long)k);
+        const double g = (p[other + qc * st[a]] - p[other + ql * st[a]]) * delta;
+        const long f = ((long)i * e1 + j) * e2 + k;
+        const double l = ls[a] ? ls[a][f] : 1.0;
+        us[a][f] -= G.cdt * (l * g);
     }
 }
+
+dim3 rows_block(int nk) { return nk > 32 ? dim3(64, 4) : dim3(32, 8); }
 
 }  // namespace
 
 void launch_project_rhs(const double* u0, const double* u1, const double* u2, double* out, const ProjGeom& G,
                         cudaStream_t s) {
-    const dim3 grid((unsigned)std::min((G.n[2] + 127) / 128, 8), (unsigned)G.n[1], (unsigned)G.n[0]);
-    k_project_rhs<<<grid, 128, 0, s>>>(u0, u1, u2, out, G);
+    const dim3 b = rows_block(G.n[2]);
+    k_project_rhs<<<dim3((G.n[2] + b.x - 1) / b.x, (G.n[1] + b.y - 1) / b.y, G.n[0]), b, 0, s>>>(u0, u1, u2, out, G);
 }
 
 void launch_project_correct(double* u0, double* u1, double* u2, const double* p, const double* lam0,
                             const double* lam1, const double* lam2, const ProjGeom& G, cudaStream_t s) {
-    const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
-    k_project_correct<0><<<dim3((unsigned)std::min((n2 + 127) / 128, 8), n1, n0 + 1), 128, 0, s>>>(u0, p, lam0, G);
-    k_project_correct<1><<<dim3((unsigned)std::min((n2 + 127) / 128, 8), n1 + 1, n0), 128, 0, s>>>(u1, p, lam1, G);
-    k_project_correct<2><<<dim3((unsigned)std::min((n2 + 128) / 128, 8), n1, n0), 128, 0, s>>>(u2, p, lam2, G);
+    const dim3 b = rows_block(G.n[2] + 1);
+    k_project_correct<<<dim3((G.n[2] + b.x) / b.x, (G.n[1] + b.y) / b.y, G.n[0] + 1), b, 0, s>>>(u0, u1, u2, p, lam0,
+                                                                                            lam1, lam2, G);
 }
 
 }  // namespace bmg
