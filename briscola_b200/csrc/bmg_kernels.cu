@@ -298,7 +298,7 @@ struct Vec16<double> {
 // half's same slots, so the pass leaves the whole level written (the
 // arithmetic of a pass over a zeroed x).
 template <typename T, bool VAR, bool ZERO>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 && !VAR ? 5 : 1) k_colour_split(LevelView<T> L, int colour) {
+__global__ void __launch_bounds__(256, VAR ? 1 : sizeof(T) == 4 ? 5 : 4) k_colour_split(LevelView<T> L, int colour) {
     grid_dep_sync();
     constexpr int NC = Vec16<T>::N;  // cells per thread
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -685,142 +685,163 @@ __global__ void __launch_bounds__(256) k_restrict_quad(Bricks<T> FB, Bricks<T> C
 
 // ---------------------------------------------------------------------------
 // The same two transfers for a parity-split fine level (single brick,
-// factor 2 along every axis): a thread owns the fine slots 4P .. 4P+3 of
-// both halves of a row -- the eight consecutive cells k = 8P .. 8P+7, four
-// even and four odd -- so every fine array moves as whole vectors.  The
-// restriction writes the coarse cells K = 4P .. 4P+3 (the parents of
-// those eight), the prolongation reads them and their two outer
-// neighbours.  Per cell the arithmetic and its order are those of
-// restrict_quad_item and prolong_quad_item, so the results are
-// bit-identical.
+// factor 2 along every axis): a thread owns NS = 16 / sizeof(T) fine slots of
+// both halves of a row -- the 2 NS consecutive cells from k = 2 NS P, half of
+// them even and half odd -- so every fine array moves as one 16-byte vector
+// a thread, whole lines a warp (FP64 threads of four slots moved half lines,
+// and the L1 was their bound: 256^3 restriction 96 us, prolongation 103 us).
+// The restriction writes the coarse cells K = NS P .. (the parents of those
+// cells); on small levels the four fine rows over them go to four lanes, so a
+// thread waits for one row's loads and there are threads enough.  The
+// prolongation reads the parents and their two outer neighbours.  Per cell the arithmetic
+// and its order are those of restrict_quad_item and prolong_quad_item, so the
+// results are bit-identical.
 // ---------------------------------------------------------------------------
+// the share of fine row (i, j) in the NS coarse cells over its slots m0 ..:
+// part[m], to be weighted with the row's own share rab
 template <typename T, bool VAR>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 && !VAR ? 3 : 2) k_restrict_split(Bricks<T> FB, Bricks<T> CB,
-                                                                                   TransferSet ts) {
+__device__ __forceinline__ T restrict_row(const LevelView<T>& F, const T* ratio, int i, int j, int m0,
+                                          T part[Vec16<T>::N]) {
+    constexpr int NS = Vec16<T>::N;
+    const int kh = F.kh;
+    const int si = (int)F.si, sj = (int)F.sj;
+    const int row = (int)row_at(F, i, j);
+    const int ce = row + m0, co = row + kh + m0;            // even and odd slots
+    const int clo = m0 > 0 ? co - 1 : row - 1;             // the k below the first cell
+    const int chi = m0 + NS < kh ? ce + NS : row + 2 * kh;  // the k above the last one
+    T xe[NS], xo[NS], me[NS], mo[NS], pe[NS], po[NS], ne[NS], no[NS], qe[NS], qo[NS], be[NS], bo[NS];
+    Vec16<T>::ld(F.x + ce, xe);
+    Vec16<T>::ld(F.x + co, xo);
+    Vec16<T>::ld(F.x + ce - si, me);
+    Vec16<T>::ld(F.x + co - si, mo);
+    Vec16<T>::ld(F.x + ce + si, pe);
+    Vec16<T>::ld(F.x + co + si, po);
+    Vec16<T>::ld(F.x + ce - sj, ne);
+    Vec16<T>::ld(F.x + co - sj, no);
+    Vec16<T>::ld(F.x + ce + sj, qe);
+    Vec16<T>::ld(F.x + co + sj, qo);
+    Vec16<T>::ld(F.b + ce, be);
+    Vec16<T>::ld(F.b + co, bo);
+    const T left = F.x[clo], right = F.x[chi];
+    // k couplings and k shares of the cells: consecutive k of the natural
+    // tables, as vectors
+    T wl[2 * NS], wh[2 * NS], rk[2 * NS];
+    Vec16<T>::ldg(F.tab + F.to.wl[2] + 2 * m0, wl);
+    Vec16<T>::ldg(F.tab + F.to.wl[2] + 2 * m0 + NS, wl + NS);
+    Vec16<T>::ldg(F.tab + F.to.wh[2] + 2 * m0, wh);
+    Vec16<T>::ldg(F.tab + F.to.wh[2] + 2 * m0 + NS, wh + NS);
+    const T* rp = ratio + F.n0 + F.n1 + 2 * m0;
+    if (((F.n0 + F.n1) & (NS - 1)) == 0) {  // 16-byte aligned: two vectors
+        Vec16<T>::ldg(rp, rk);
+        Vec16<T>::ldg(rp + NS, rk + NS);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 2 * NS; ++q) rk[q] = ldg(rp + q);
+    }
+    const T ra = ldg(ratio + i);
+    const T wil = ldg(F.tab + F.to.wl[0] + i), wih = ldg(F.tab + F.to.wh[0] + i);
+    const T rab = ra * ldg(ratio + F.n0 + j);
+    const T wjl = ldg(F.tab + F.to.wl[1] + j), wjh = ldg(F.tab + F.to.wh[1] + j);
+    T l0e[NS], l0o[NS], l0pe[NS], l0po[NS], l1e[NS], l1o[NS], l1pe[NS], l1po[NS], l2e[NS], l2o[NS], l2r = T(1);
+    if (VAR) {
+        Vec16<T>::ldg(F.lam0 + ce, l0e);
+        Vec16<T>::ldg(F.lam0 + co, l0o);
+        Vec16<T>::ldg(F.lam0 + ce + si, l0pe);
+        Vec16<T>::ldg(F.lam0 + co + si, l0po);
+        Vec16<T>::ldg(F.lam1 + ce, l1e);
+        Vec16<T>::ldg(F.lam1 + co, l1o);
+        Vec16<T>::ldg(F.lam1 + ce + sj, l1pe);
+        Vec16<T>::ldg(F.lam1 + co + sj, l1po);
+        Vec16<T>::ldg(F.lam2 + ce, l2e);
+        Vec16<T>::ldg(F.lam2 + co, l2o);
+        l2r = ldg(F.lam2 + chi);
+    }
+#pragma unroll
+    for (int m = 0; m < NS; ++m) {
+        // the even cell k = 2(m0+m) and the odd cell k + 1, in that order
+        T r2[2];
+#pragma unroll
+        for (int sd = 0; sd < 2; ++sd) {
+            T w[6] = {wil, wih, wjl, wjh, wl[2 * m + sd], wh[2 * m + sd]};
+            if (VAR) {
+                w[0] *= sd ? l0o[m] : l0e[m];
+                w[1] *= sd ? l0po[m] : l0pe[m];
+                w[2] *= sd ? l1o[m] : l1e[m];
+                w[3] *= sd ? l1po[m] : l1pe[m];
+                w[4] *= sd ? l2o[m] : l2e[m];
+                // upper k face: the lower face of the next cell
+                w[5] *= sd ? (m < NS - 1 ? l2e[m + 1] : l2r) : l2o[m];
+            }
+            const T own = sd ? xo[m] : xe[m];
+            const T km = sd ? xe[m] : (m > 0 ? xo[m - 1] : left);
+            const T kp = sd ? (m < NS - 1 ? xe[m + 1] : right) : xo[m];
+            const T xmv = sd ? mo[m] : me[m], xpv = sd ? po[m] : pe[m];
+            const T ymv = sd ? no[m] : ne[m], ypv = sd ? qo[m] : qe[m];
+            const T sv = w[0] * xmv + w[1] * xpv + w[2] * ymv + w[3] * ypv + w[4] * km + w[5] * kp;
+            const T d = w[0] + w[1] + w[2] + w[3] + w[4] + w[5];
+            r2[sd] = (sd ? bo[m] : be[m]) + d * own - sv;
+        }
+        part[m] = rk[2 * m] * r2[0] + rk[2 * m + 1] * r2[1];
+    }
+    return rab;
+}
+
+// SPREAD: four neighbouring lanes share a group, one fine row each
+template <typename T, bool VAR, bool SPREAD>
+__global__ void __launch_bounds__(256, VAR ? 2 : 3) k_restrict_split(Bricks<T> FB, Bricks<T> CB, TransferSet ts) {
     grid_dep_sync();
+    constexpr int NS = Vec16<T>::N;
     const LevelView<T>& F = FB.v[0];
     const LevelView<T>& C = CB.v[0];
     const TransferTabs& t = ts.t[0];
-    const int P = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gx = blockIdx.x * blockDim.x + threadIdx.x;
+    const int m0 = NS * (SPREAD ? gx >> 2 : gx);
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
     const int I = blockIdx.z;
-    const int kh = F.kh;
-    if (J >= C.n1 || 4 * P >= kh) return;
+    const bool ok = J < C.n1 && m0 < F.kh;
     const T* ratio;
     if constexpr (sizeof(T) == 8)
         ratio = reinterpret_cast<const T*>(t.ratio64);
     else
         ratio = reinterpret_cast<const T*>(t.ratio32);
-    const int m0 = 4 * P;
-    // k couplings and k shares of the even (k = 2(m0+m)) and odd cells: the
-    // eight consecutive k = 8P .. 8P+7 of the natural tables, as vectors
-    T wke[4], whe[4], wko[4], who[4], rke[4], rko[4];
-    {
-        T a[8], b[8], r[8];
-        Row4<T>::ldg4(F.tab + F.to.wl[2] + 2 * m0, a);
-        Row4<T>::ldg4(F.tab + F.to.wl[2] + 2 * m0 + 4, a + 4);
-        Row4<T>::ldg4(F.tab + F.to.wh[2] + 2 * m0, b);
-        Row4<T>::ldg4(F.tab + F.to.wh[2] + 2 * m0 + 4, b + 4);
-        const T* rp = ratio + F.n0 + F.n1 + 2 * m0;
-        if (((F.n0 + F.n1) & 3) == 0) {  // 16-byte aligned: two vectors
-            Row4<T>::ldg4(rp, r);
-            Row4<T>::ldg4(rp + 4, r + 4);
-        } else {
+    // the rows' shares in the order (a, e) = (0, 0), (0, 1), (1, 0), (1, 1)
+    T acc[NS];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) r[q] = ldg(rp + q);
+    for (int m = 0; m < NS; ++m) acc[m] = T(0);
+    if constexpr (SPREAD) {
+        const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31, sub = lane & 3;
+        T rab = T(0), part[NS];
+#pragma unroll
+        for (int m = 0; m < NS; ++m) part[m] = T(0);
+        if (ok) rab = restrict_row<T, VAR>(F, ratio, 2 * I + (sub >> 1), 2 * J + (sub & 1), m0, part);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const T rs = __shfl_sync(0xffffffffu, rab, (lane & 28) + s);
+#pragma unroll
+            for (int m = 0; m < NS; ++m) acc[m] += rs * __shfl_sync(0xffffffffu, part[m], (lane & 28) + s);
+        }
+        if (!ok) return;
+#pragma unroll
+        for (int m = 0; m < NS; ++m)
+            if (sub == m) C.b[cell32(C, I, J, m0 + m)] = acc[m];
+    } else {
+        if (!ok) return;
+#pragma unroll(VAR ? 1 : 4)
+        for (int s = 0; s < 4; ++s) {
+            T part[NS];
+            const T rab = restrict_row<T, VAR>(F, ratio, 2 * I + (s >> 1), 2 * J + (s & 1), m0, part);
+#pragma unroll
+            for (int m = 0; m < NS; ++m) acc[m] += rab * part[m];
         }
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            wke[m] = a[2 * m];
-            wko[m] = a[2 * m + 1];
-            whe[m] = b[2 * m];
-            who[m] = b[2 * m + 1];
-            rke[m] = r[2 * m];
-            rko[m] = r[2 * m + 1];
-        }
+        for (int m = 0; m < NS; ++m) C.b[cell32(C, I, J, m0 + m)] = acc[m];
     }
-    T acc[4] = {T(0), T(0), T(0), T(0)};
-    // FP64 and variable-coefficient rows hold twice the registers: one fine
-    // plane at a time there
-#pragma unroll(sizeof(T) == 4 && !VAR ? 2 : 1)
-    for (int a = 0; a < 2; ++a) {
-        const int i = 2 * I + a;
-        const T ra = ldg(ratio + i);
-        const T wil = ldg(F.tab + F.to.wl[0] + i), wih = ldg(F.tab + F.to.wh[0] + i);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int j = 2 * J + e;
-            const T rab = ra * ldg(ratio + F.n0 + j);
-            const T wjl = ldg(F.tab + F.to.wl[1] + j), wjh = ldg(F.tab + F.to.wh[1] + j);
-            const int si = (int)F.si, sj = (int)F.sj;
-            const int row = (int)row_at(F, i, j);
-            const int ce = row + m0, co = row + kh + m0;           // even and odd slots
-            const int clo = m0 > 0 ? co - 1 : row - 1;            // k = 8P - 1
-            const int chi = m0 + 4 < kh ? ce + 4 : row + 2 * kh;  // k = 8P + 8
-            T xe[4], xo[4], me[4], mo[4], pe[4], po[4], ne[4], no[4], qe[4], qo[4], be[4], bo[4];
-            Row4<T>::ld(F.x + ce, xe);
-            Row4<T>::ld(F.x + co, xo);
-            Row4<T>::ld(F.x + ce - si, me);
-            Row4<T>::ld(F.x + co - si, mo);
-            Row4<T>::ld(F.x + ce + si, pe);
-            Row4<T>::ld(F.x + co + si, po);
-            Row4<T>::ld(F.x + ce - sj, ne);
-            Row4<T>::ld(F.x + co - sj, no);
-            Row4<T>::ld(F.x + ce + sj, qe);
-            Row4<T>::ld(F.x + co + sj, qo);
-            Row4<T>::ld(F.b + ce, be);
-            Row4<T>::ld(F.b + co, bo);
-            const T left = F.x[clo], right = F.x[chi];
-            T l0e[4], l0o[4], l0pe[4], l0po[4], l1e[4], l1o[4], l1pe[4], l1po[4], l2e[4], l2o[4], l2r = T(1);
-            if (VAR) {
-                Row4<T>::ldg4(F.lam0 + ce, l0e);
-                Row4<T>::ldg4(F.lam0 + co, l0o);
-                Row4<T>::ldg4(F.lam0 + ce + si, l0pe);
-                Row4<T>::ldg4(F.lam0 + co + si, l0po);
-                Row4<T>::ldg4(F.lam1 + ce, l1e);
-                Row4<T>::ldg4(F.lam1 + co, l1o);
-                Row4<T>::ldg4(F.lam1 + ce + sj, l1pe);
-                Row4<T>::ldg4(F.lam1 + co + sj, l1po);
-                Row4<T>::ldg4(F.lam2 + ce, l2e);
-                Row4<T>::ldg4(F.lam2 + co, l2o);
-                l2r = ldg(F.lam2 + chi);
-            }
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                // the even cell k = 2(m0+m) and the odd cell k + 1, in that order
-                T r2[2];
-#pragma unroll
-                for (int sd = 0; sd < 2; ++sd) {
-                    T w[6] = {wil, wih, wjl, wjh, sd ? wko[m] : wke[m], sd ? who[m] : whe[m]};
-                    if (VAR) {
-                        w[0] *= sd ? l0o[m] : l0e[m];
-                        w[1] *= sd ? l0po[m] : l0pe[m];
-                        w[2] *= sd ? l1o[m] : l1e[m];
-                        w[3] *= sd ? l1po[m] : l1pe[m];
-                        w[4] *= sd ? l2o[m] : l2e[m];
-                        // upper k face: the lower face of the next cell
-                        w[5] *= sd ? (m < 3 ? l2e[m + 1] : l2r) : l2o[m];
-                    }
-                    const T own = sd ? xo[m] : xe[m];
-                    const T km = sd ? xe[m] : (m > 0 ? xo[m - 1] : left);
-                    const T kp = sd ? (m < 3 ? xe[m + 1] : right) : xo[m];
-                    const T xmv = sd ? mo[m] : me[m], xpv = sd ? po[m] : pe[m];
-                    const T ymv = sd ? no[m] : ne[m], ypv = sd ? qo[m] : qe[m];
-                    const T sv = w[0] * xmv + w[1] * xpv + w[2] * ymv + w[3] * ypv + w[4] * km + w[5] * kp;
-                    const T d = w[0] + w[1] + w[2] + w[3] + w[4] + w[5];
-                    r2[sd] = (sd ? bo[m] : be[m]) + d * own - sv;
-                }
-                acc[m] += rab * (rke[m] * r2[0] + rko[m] * r2[1]);
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 4; ++m) C.b[cell32(C, I, J, m0 + m)] = acc[m];
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_prolong_split(Bricks<T> FB, Bricks<T> CB, TransferSet ts) {
     grid_dep_sync();
+    constexpr int NS = Vec16<T>::N;
     const LevelView<T>& F = FB.v[0];
     const LevelView<T>& C = CB.v[0];
     const TransferTabs& t = ts.t[0];
@@ -828,8 +849,8 @@ __global__ void __launch_bounds__(256) k_prolong_split(Bricks<T> FB, Bricks<T> C
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
     const int kh = F.kh;
-    if (j >= F.n1 || 4 * P >= kh) return;
-    const int m0 = 4 * P;
+    if (j >= F.n1 || NS * P >= kh) return;
+    const int m0 = NS * P;
     const int* pidx = t.pidx;
     const T* pw;
     if constexpr (sizeof(T) == 8)
@@ -842,23 +863,23 @@ __global__ void __launch_bounds__(256) k_prolong_split(Bricks<T> FB, Bricks<T> C
     const T ui = T(1) - wi, uj = T(1) - wj;
     const int* pk = pidx + 2 * (F.n0 + F.n1);
     const T* wk = pw + F.n0 + F.n1;
-    // parents of the eight cells: K = m0 .. m0+3; second coarse cells: K - 1
-    // for the even cells and K + 1 for the odd ones, the outer two from the
+    // parents of the cells: K = m0 .. m0+NS-1; second coarse cells: K - 1 for
+    // the even cells and K + 1 for the odd ones, the outer two from the
     // tables (they may be a wrapped, a ghost or the parent's own index)
     const int Klo = kpos(C, ldg(pk + 2 * (2 * m0) + 1));
-    const int Khi = kpos(C, ldg(pk + 2 * (2 * m0 + 7) + 1));
-    T we[4], ue[4], wo[4], uo[4];
+    const int Khi = kpos(C, ldg(pk + 2 * (2 * m0 + 2 * NS - 1) + 1));
+    T we[NS], ue[NS], wo[NS], uo[NS];
     {
-        T a[8];  // the weights of k = 8P .. 8P+7 (natural order, contiguous)
-        if (((F.n0 + F.n1) & 3) == 0) {  // 16-byte aligned: two vectors
-            Row4<T>::ldg4(wk + 2 * m0, a);
-            Row4<T>::ldg4(wk + 2 * m0 + 4, a + 4);
+        T a[2 * NS];  // the weights of the cells (natural order, contiguous)
+        if (((F.n0 + F.n1) & (NS - 1)) == 0) {  // 16-byte aligned: two vectors
+            Vec16<T>::ldg(wk + 2 * m0, a);
+            Vec16<T>::ldg(wk + 2 * m0 + NS, a + NS);
         } else {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) a[q] = ldg(wk + 2 * m0 + q);
+            for (int q = 0; q < 2 * NS; ++q) a[q] = ldg(wk + 2 * m0 + q);
         }
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
+        for (int m = 0; m < NS; ++m) {
             we[m] = a[2 * m];
             wo[m] = a[2 * m + 1];
             ue[m] = T(1) - we[m];
@@ -866,46 +887,51 @@ __global__ void __launch_bounds__(256) k_prolong_split(Bricks<T> FB, Bricks<T> C
         }
     }
     const int rows[4] = {cell32(C, I0, J0, 0), cell32(C, I0, J1, 0), cell32(C, I1, J0, 0), cell32(C, I1, J1, 0)};
-    T ve[4][4], vo[4][4];
+    T ve[4][NS], vo[4][NS];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const T* X = C.x + rows[r];
-        T xc[4];  // the parents K = m0 .. m0+3
+        T xc[NS];  // the parents K = m0 .. m0+NS-1
         if (C.kh) {
-            Row4<T>::ld2(X + m0 / 2, xc[0], xc[2]);
-            Row4<T>::ld2(X + C.kh + m0 / 2, xc[1], xc[3]);
+            if constexpr (NS == 4) {
+                Row4<T>::ld2(X + m0 / 2, xc[0], xc[2]);
+                Row4<T>::ld2(X + C.kh + m0 / 2, xc[1], xc[3]);
+            } else {
+                xc[0] = X[m0 / 2];
+                xc[1] = X[C.kh + m0 / 2];
+            }
         } else {
-            Row4<T>::ld(X + m0, xc);
+            Vec16<T>::ld(X + m0, xc);
         }
         const T xlo = X[Klo], xhi = X[Khi];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
+        for (int m = 0; m < NS; ++m) {
             ve[r][m] = ue[m] * xc[m] + we[m] * (m > 0 ? xc[m - 1] : xlo);
-            vo[r][m] = uo[m] * xc[m] + wo[m] * (m < 3 ? xc[m + 1] : xhi);
+            vo[r][m] = uo[m] * xc[m] + wo[m] * (m < NS - 1 ? xc[m + 1] : xhi);
         }
     }
     const int row = (int)row_at(F, i, j);
     const int ce = row + m0, co = row + kh + m0;
-    T xe[4], xo[4];
-    Row4<T>::ld(F.x + ce, xe);
-    Row4<T>::ld(F.x + co, xo);
+    T xe[NS], xo[NS];
+    Vec16<T>::ld(F.x + ce, xe);
+    Vec16<T>::ld(F.x + co, xo);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < NS; ++m) {
         xe[m] += ui * (uj * ve[0][m] + wj * ve[1][m]) + wi * (uj * ve[2][m] + wj * ve[3][m]);
         xo[m] += ui * (uj * vo[0][m] + wj * vo[1][m]) + wi * (uj * vo[2][m] + wj * vo[3][m]);
     }
-    Row4<T>::st(F.x + ce, xe);
-    Row4<T>::st(F.x + co, xo);
+    Vec16<T>::st(F.x + ce, xe);
+    Vec16<T>::st(F.x + co, xo);
     // periodic images, as in k_colour_split
     if ((F.per0 && (i == 0 || i == F.n0 - 1)) || (F.per1 && (j == 0 || j == F.n1 - 1))) {
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
+        for (int m = 0; m < NS; ++m) {
             store_images(F, ce + m, i, j, 2 * (m0 + m), xe[m]);
             store_images(F, co + m, i, j, 2 * (m0 + m) + 1, xo[m]);
         }
     } else if (F.per2) {
         if (m0 == 0) F.x[row + 2 * kh] = xe[0];
-        if (m0 + 4 == kh) F.x[row - 1] = xo[3];
+        if (m0 + NS == kh) F.x[row - 1] = xo[NS - 1];
     }
 }
 
@@ -1309,10 +1335,17 @@ inline dim3 split_block(int groups) {
 template <typename T, bool VAR>
 void launch_residual_restrict(const Bricks<T>& F, const Bricks<T>& C, const TransferSet& t, cudaStream_t s) {
     if (F.v[0].kh && quad_transfers(F, t)) {
-        const int groups = F.v[0].kh / 4;
-        const dim3 blk = split_block(groups);
-        const dim3 grid((groups + blk.x - 1) / blk.x, (C.v[0].n1 + blk.y - 1) / blk.y, C.v[0].n0);
-        launch_k(k_restrict_split<T, VAR>, grid, blk, 0, s, F, C, t);
+        // four lanes a group where the groups alone are at most 256 CTAs (64^3
+        // fine: 11 -> 6 us); above that one thread reads its rows' shared
+        // planes and rows once (256^3 FP64: 124 us with four lanes)
+        const int groups = F.v[0].kh / Vec16<T>::N;
+        const bool spread = (long)groups * C.v[0].n1 * C.v[0].n0 <= 256 * 256;
+        const dim3 blk = split_block(spread ? 4 * groups : groups);
+        const dim3 grid(((spread ? 4 * groups : groups) + blk.x - 1) / blk.x, (C.v[0].n1 + blk.y - 1) / blk.y, C.v[0].n0);
+        if (spread)
+            launch_k(k_restrict_split<T, VAR, true>, grid, blk, 0, s, F, C, t);
+        else
+            launch_k(k_restrict_split<T, VAR, false>, grid, blk, 0, s, F, C, t);
         return;
     }
     if (quad_transfers(F, t)) {
@@ -1328,7 +1361,7 @@ void launch_residual_restrict(const Bricks<T>& F, const Bricks<T>& C, const Tran
 template <typename T>
 void launch_prolong_correct(const Bricks<T>& F, const Bricks<T>& C, const TransferSet& t, cudaStream_t s) {
     if (F.v[0].kh && quad_transfers(F, t)) {
-        const int groups = F.v[0].kh / 4;
+        const int groups = F.v[0].kh / Vec16<T>::N;
         const dim3 blk = split_block(groups);
         const dim3 grid((groups + blk.x - 1) / blk.x, (F.v[0].n1 + blk.y - 1) / blk.y, F.v[0].n0);
         launch_k(k_prolong_split<T>, grid, blk, 0, s, F, C, t);
