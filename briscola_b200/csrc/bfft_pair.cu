@@ -19,8 +19,8 @@
 // Measured, 256^3, us a pass (268 MB, 41 us at the copy rate), against the
 // persistent kernel with a cp.async staging buffer that it replaces
 // (k_transform, 12 warps an SM; it keeps the short lines and the quarter-wave
-// kinds): real forward along k 123 -> 47, strided 128 -> 57, inverse along k
-// 112 -> 48, strided 130 -> 70.
+// kinds): real forward along k 123 -> 47, strided 128 -> 55, inverse along k
+// 112 -> 48, strided 130 -> 51.
 
 #include "bfft_internal.h"
 
@@ -124,6 +124,7 @@ struct StorePoints {
     double* out;
     const Lines* L;
     long tile;
+    PairLine own;  // strided axes: a thread's line pair is the same in every pass
     int odd, adjacent;
     __device__ __forceinline__ void begin() const {}
     __device__ __forceinline__ void operator()(int u, int k, double2 z) const;
@@ -166,8 +167,7 @@ __device__ __forceinline__ void StorePoints<LOGN, KIND, LF>::operator()(int u, i
         a = -a;
         b = -b;
     }
-    const PairLine P = pair_line<LOGN, LF>(*L, tile, u);
-    put2<LF>(out, P, LF ? (long)q * L->stride : q, adjacent, a, b);
+    put2<LF>(out, LF ? own : pair_line<LOGN, LF>(*L, tile, u), LF ? (long)q * L->stride : q, adjacent, a, b);
 }
 
 template <int LOGN, int KIND, bool LF>
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kPairThreads, 4) k_pair(const double* in, doub
     for (int r = 0; r < 16; ++r) buf[slot<LOGN>((u << LOGN) + 16 * j + r)] = v[r];
     __syncthreads();
     if constexpr (SPEC) {
-        pair_passes<LOGN, 4, LOGLB, LF>(buf, T.tw, StorePoints<LOGN, KIND, LF>{out, &L, tile, T.odd, adjacent});
+        pair_passes<LOGN, 4, LOGLB, LF>(buf, T.tw, StorePoints<LOGN, KIND, LF>{out, &L, tile, P, T.odd, adjacent});
     } else {
         pair_passes<LOGN, 4, LOGLB, LF>(buf, T.tw, KeepSpectrum<LOGN>{buf});
         __syncthreads();
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kPairThreads, 4) k_pair(const double* in, doub
             group_of<LOGH, LOGLB, LF>((int)threadIdx.x + s * kPairThreads, uu, k);
             const int k2 = k ? N - k : N / 2;
             const double2 z = buf[slot<LOGN>((uu << LOGN) + k)], y = buf[slot<LOGN>((uu << LOGN) + k2)];
-            const PairLine Q = pair_line<LOGN, LF>(L, tile, uu);
+            const PairLine Q = LF ? P : pair_line<LOGN, LF>(L, tile, uu);
             double a1, b1, a2, b2;
             int q1 = k, q2 = k2;
             if constexpr (KIND == K_R2HC) {

@@ -8,11 +8,11 @@
 // of shared memory, from both ends, 219 us.  With the factors 1 / D_k known,
 // both sweeps are first-order recurrences, y_k = a_k - m_k y_{k-1}, so a line
 // is cut into chunks of C rows, one thread each, held in registers: the chunk
-// from a zero start together with its running product, a scan over the line's
-// chunks for the value entering each (in shared memory, log2 steps), and one
-// independent multiply-add per row.  The serial chain is C rows and the scan
-// instead of n, the field is read and written once, and a thread has all its
-// 2 C loads in flight: 139 us there, 93 -> 14 us for 128 x 96 x 64 cells.
+// from a zero start and its product, a scan over the line's chunks for the
+// value entering each (in shared memory, log2 steps), and the chunk again from
+// that value.  The serial chain is 2 C rows and the scan instead of n, the field is read and written once, and a thread has all its
+// 2 C loads in flight: 115 us there (139 with chunks of 16 rows, which also
+// kept every row's product), 93 -> 12 us for 128 x 96 x 64 cells.
 //
 // Bound: memory (16 B a cell of the field and 8 B of each factor).
 
@@ -77,53 +77,73 @@ __device__ __forceinline__ double chunk_carry(double2* buf, int TL, int Q, int q
 
 // TL lines a CTA, Q chunks of C rows a line; thread (q, t), t fastest
 template <int C>
-__global__ void __launch_bounds__(kTriMaxThreads, 1) k_tri_chunks(double* __restrict__ w, const __grid_constant__ Lines L,
-                                                                  const __grid_constant__ Tri T, int logTL, int Q) {
+__global__ void __launch_bounds__(kTriMaxThreads, C <= 8 ? 2 : 1)
+    k_tri_chunks(double* __restrict__ w, const __grid_constant__ Lines L, const __grid_constant__ Tri T, int logTL,
+                 int Q) {
     extern __shared__ __align__(16) double2 scan[];
     const int TL = 1 << logTL, t = threadIdx.x & (TL - 1), q = threadIdx.x >> logTL;
     const long l = (long)blockIdx.x * TL + t;
     const bool ok = l < L.count;
-    const int ns = T.ns, k0 = q * C, modes = T.nci * T.nco;
+    const int k0 = q * C, modes = T.nci * T.nco;
     const unsigned inner = (unsigned)L.inner, lu = ok ? (unsigned)l : 0u;
     const int co = (int)(lu / inner), ci = (int)(lu - (unsigned)co * inner);
-    double* wl = w + line_base(L, lu) + k0 * L.stride;
+    const int rows = ok ? min(C, T.ns - k0) : 0;  // rows of this chunk
+    const long st = L.stride;
+    double* wl = w + line_base(L, lu) + k0 * st;
     const double* rl = T.rfac + T.clsO[co] * T.nci + T.clsI[ci] + (long)k0 * modes;
-    double f[C], r[C], p[C];
-    double rp = q ? __ldg(rl - modes) : 0.0;  // 1 / D of the row before the chunk
+    double f[C], r[C];
+    double rp = q && rows > 0 ? __ldg(rl - modes) : 0.0;  // 1 / D of the row before the chunk
+    {
+        const double* src = wl;
+        const double* fac = rl;
 #pragma unroll
-    for (int e = 0; e < C; ++e) {
-        const bool in = ok && k0 + e < ns;
-        f[e] = in ? wl[e * L.stride] : 0.0;
-        r[e] = in ? __ldg(rl + (long)e * modes) : 0.0;
+        for (int e = 0; e < C; ++e) {
+            f[e] = e < rows ? *src : 0.0;
+            r[e] = e < rows ? __ldg(fac) : 0.0;
+            src += st;
+            fac += modes;
+        }
     }
     // forward: y_k = f_k - (DL_k / D_{k-1}) y_{k-1}
+    double m[C];
+#pragma unroll
+    for (int e = 0; e < C; ++e) {
+        m[e] = e < rows && k0 + e > 0 ? -__ldg(T.DL + k0 + e) * rp : 0.0;
+        rp = r[e];
+    }
     double y = 0.0, b = 1.0;
 #pragma unroll
     for (int e = 0; e < C; ++e) {
-        const double m = k0 + e < ns && k0 + e > 0 ? -__ldg(T.DL + k0 + e) * rp : 0.0;
-        rp = r[e];
-        y = f[e] + m * y;
-        b = m * b;
-        f[e] = y;
-        p[e] = b;
+        y = f[e] + m[e] * y;
+        b = m[e] * b;
     }
-    double c = chunk_carry(scan, TL, Q, q, t, y, b);
+    y = chunk_carry(scan, TL, Q, q, t, y, b);
+#pragma unroll
+    for (int e = 0; e < C; ++e) {
+        y = f[e] + m[e] * y;
+        f[e] = y * r[e];
+    }
     // backward: x_k = y_k / D_k - (DU_k / D_k) x_{k+1}
+#pragma unroll
+    for (int e = 0; e < C; ++e) m[e] = e < rows && k0 + e < T.ns - 1 ? -__ldg(T.DU + k0 + e) * r[e] : 0.0;
     double x = 0.0;
     b = 1.0;
 #pragma unroll
     for (int e = C - 1; e >= 0; --e) {
-        const double g = (f[e] + p[e] * c) * r[e];
-        const double m = k0 + e < ns - 1 ? -__ldg(T.DU + k0 + e) * r[e] : 0.0;
-        x = g + m * x;
-        b = m * b;
-        f[e] = x;
-        p[e] = b;
+        x = f[e] + m[e] * x;
+        b = m[e] * b;
     }
-    c = chunk_carry(scan, TL, Q, Q - 1 - q, t, x, b);
+    x = chunk_carry(scan, TL, Q, Q - 1 - q, t, x, b);
 #pragma unroll
-    for (int e = 0; e < C; ++e)
-        if (ok && k0 + e < ns) wl[e * L.stride] = f[e] + p[e] * c;
+    for (int e = C - 1; e >= 0; --e) {
+        x = f[e] + m[e] * x;
+        f[e] = x;
+    }
+#pragma unroll
+    for (int e = 0; e < C; ++e) {
+        if (e < rows) *wl = f[e];
+        wl += st;
+    }
 }
 
 template <int C>
@@ -134,10 +154,9 @@ cudaError_t launch_c(double* w, const Lines& L, const Tri& T, int logTL, int Q, 
     return cudaGetLastError();
 }
 
-// rows of a chunk: the fewest that leave a line at most 16 threads of 4 or
-// 20 of 8, so that a CTA has 16 lines (a whole 128-byte run of every row) and
-// several fit an SM; 16 above that
-int chunk_rows(int ns) { return ns <= 64 ? 4 : ns <= 160 ? 8 : 16; }
+// rows of a chunk: as few as leave a CTA 16 lines (a whole 128-byte run of
+// every row) within 512 threads
+int chunk_rows(int ns) { return ns <= 64 ? 4 : ns <= 256 ? 8 : 16; }
 
 }  // namespace
 

@@ -45,7 +45,7 @@ def test_paired_transforms(m, kind):
     _check((32, m, 7), (P, kind, N), 2)  # odd rows: no adjacent pairs, solve along z
 
 
-@pytest.mark.parametrize("ns", [2, 3, 4, 5, 63, 64, 65, 160, 161, 511, 512, 513, 1030])
+@pytest.mark.parametrize("ns", [2, 3, 4, 5, 63, 64, 65, 255, 256, 257, 512, 513, 1030])
 def test_tridiagonal_chunks(ns):
     _check((8, ns, 4), (P, N, P), 1)
     _check((ns, 4, 8), (D, P, N), 0)
