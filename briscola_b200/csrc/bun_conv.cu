@@ -21,6 +21,10 @@
 // gradient.  K is split over grid.y; each split writes FP32 partial sums
 // that a CUDA-core kernel adds in a fixed order.
 //
+// Weight gradients of 16 and 32 output channels on rows of whole 16-voxel
+// groups march along j instead (k_wgrad_rows, below): each row is loaded once
+// for the taps that need it.
+//
 // Shared-memory operand layouts are the canonical no-swizzle (interleaved)
 // ones of the tcgen05 matrix descriptors: a core matrix is 8 rows of 16
 // bytes (128 contiguous bytes).  K-major tiles: a row is one M/N index with
@@ -439,6 +443,203 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(WgradArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// weight gradient marching along j (16 or 32 output channels, n2 % 16 == 0)
+// ---------------------------------------------------------------------------
+// k_wgrad gathers the 128 voxels of a K block once for every (tap, channel)
+// row tile, 27 times over, and its loads bound it (48 -> 16 channels at 128^3:
+// 1.94 ms, tensor pipe idle).  Here a CTA owns one plane offset di and a group
+// of NG input channels and walks row segments (plane i, 128 voxels along k, up
+// to 32 rows j).  One step takes the input row jj of plane i + di and the
+// three rows j = jj-1, jj, jj+1 of the output gradient that meet it:
+//   M = (output-gradient row, output channel), N = input channel, K = voxels,
+// one MMA chain per tap offset dk -- a shift of the input row's start address,
+// as in k_conv_rows -- so a row is loaded once and 24 MMAs of K = 16 use it.
+// The three rows are neighbours in a ring of R rows whose first two are kept
+// twice, behind its end, so that any three in turn are one matrix; M is padded
+// to 128 by whatever follows them, whose products nobody reads.  Rows outside
+// the segment or the grid are zero.  Both operands are MN-major: chunks of 8
+// channels x voxels of 16 bytes.
+// D: lane = (row, output channel), column = (dk, input channel); it is added
+// up over every segment of the split and written once, as k_wgrad's partials.
+// Measured at 128^3, us: 48 -> 16 channels 1936 -> 663, 16 -> 16 735 -> 250;
+// at 64^3: 96 -> 32 802 -> 210, 32 -> 32 286 -> 78, 16 -> 32 160 -> 72.
+constexpr int kWgVox = 128;                      // voxels of a segment row
+constexpr int kWgInChunk = (kWgVox + 2) * 16;    // bytes of 8 input channels of a row (k0-1 .. k0+128)
+constexpr int kWgDzChunk = kWgVox * 16;          // bytes of 8 output channels of a row
+constexpr int kWgSeg = 32;                       // rows of a segment
+
+template <int NG, int COUT>
+struct WgRowShape {
+    static constexpr int R = NG * COUT > 1024 ? 4 : 5;  // rows of the rings (two CTAs an SM)
+    static constexpr int DZROW = (COUT / 8) * kWgDzChunk;
+    static constexpr int INROW = (NG / 8) * kWgInChunk;
+    // the last window starts at row R - 1 and reads 128 / COUT rows: past the
+    // ring's R + 2 rows it reads the input rows behind them
+    static constexpr int DZ = (R + 2) * DZROW;
+    static constexpr int OVER = (R - 1 + 128 / COUT) * DZROW - DZ;
+    static constexpr int IN = R * INROW > OVER ? R * INROW : OVER;
+    static constexpr uint32_t NCOLS = 3 * NG <= 64 ? 64 : 3 * NG <= 128 ? 128 : 256;
+    static constexpr int smem = DZ + IN + (2 * R + 1) * 8 + 16;
+};
+
+template <int NG, int COUT>
+__global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
+    using F = WgRowShape<NG, COUT>;
+    constexpr int R = F::R;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + F::DZ + F::IN);
+    uint64_t* empty = full + R;
+    uint64_t* accb = empty + R;
+    uint32_t* slot = reinterpret_cast<uint32_t*>(accb + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int n0 = a.n0, n1 = a.n1, n2 = a.n2;
+    const int split = blockIdx.x, di = blockIdx.y, cb = blockIdx.z * NG;
+    const int nks = (n2 + kWgVox - 1) / kWgVox, njs = (n1 + kWgSeg - 1) / kWgSeg;
+    const int units = n0 * nks * njs;
+
+    if (tid == 0) {
+        for (int r = 0; r < R; ++r) {
+            mbar_init(&full[r], kProducers);
+            mbar_init(&empty[r], 1);
+        }
+        mbar_init(accb, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 4) tmem_alloc(slot, F::NCOLS);
+    tc_before();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = *slot;
+    const uint32_t base = smem_u32(smem);
+    bool ok = true, any = false;
+
+    // a unit's plane, first voxel and row, rows and voxels; false where the
+    // input plane lies outside the grid
+    auto unit = [&](int un, int& i, int& k0, int& js, int& nr, int& kv) {
+        const int ks = un % nks, q = un / nks;
+        k0 = ks * kWgVox;
+        kv = min(kWgVox, n2 - k0);
+        js = (q % njs) * kWgSeg;
+        nr = min(kWgSeg, n1 - js);
+        i = q / njs;
+        const int ii = i + di - 1;
+        return ii >= 0 && ii < n0;
+    };
+
+    if (warp < 4) {
+        // ---- loader: entry v = 0 .. nr+3 of a unit is output-gradient row
+        // q = v - 2 (zero outside 0 .. nr-1) and, from v = 2 on, the input row
+        // of step u = v - 2, row js - 1 + u
+        int e = 0;
+        for (int un = split; ok && un < units; un += a.nsplit) {
+            int i, k0, js, nr, kv;
+            if (!unit(un, i, k0, js, nr, kv)) continue;
+            const int ii = i + di - 1;
+            for (int v = 0; v < nr + 4; ++v, ++e) {
+                const int r = e % R;
+                if (!mbar_wait(&empty[r], ((uint32_t)(e / R) & 1) ^ 1)) {
+                    ok = false;
+                    break;
+                }
+                const int q = v - 2;
+                {
+                    const bool valid = q >= 0 && q < nr && tid < kv;
+                    const bf16* src = valid ? a.dz + (((long)i * n1 + js + q) * n2 + k0 + tid) * COUT : a.dz;
+                    const uint32_t d = base + r * F::DZROW + tid * 16;
+#pragma unroll
+                    for (int h = 0; h < COUT / 8; ++h) {
+                        cp16(d + h * kWgDzChunk, src + (valid ? h * 8 : 0), valid);
+                        if (r < 2) cp16(d + R * F::DZROW + h * kWgDzChunk, src + (valid ? h * 8 : 0), valid);
+                    }
+                }
+                if (v >= 2) {
+                    const int jj = js - 1 + q;
+                    for (int kk = tid; kk < kv + 2; kk += kProducers) {
+                        const int k = k0 - 1 + kk;
+                        const bool valid = jj >= 0 && jj < n1 && k >= 0 && k < n2;
+                        const uint32_t d = base + F::DZ + r * F::INROW + kk * 16;
+#pragma unroll
+                        for (int h = 0; h < NG / 8; ++h)
+                            cp16(d + h * kWgInChunk, valid ? in_ptr(a.in, n1, n2, ii, jj, k, cb + h * 8) : a.dz, valid);
+                    }
+                }
+                cp_arrive(&full[r]);
+            }
+        }
+    } else if (tid == kProducers) {
+        // ---- MMA issue: per step and dk, kv / 16 MMAs of 128 x NG x 16
+        constexpr uint32_t idesc = idesc_bf16(128, NG, true, true);
+        int e = 0;
+        for (int un = split; ok && un < units; un += a.nsplit) {
+            int i, k0, js, nr, kv;
+            if (!unit(un, i, k0, js, nr, kv)) continue;
+            for (int u = 0; ok && u < nr + 2; ++u) {
+                for (int v = u == 0 ? 0 : u + 2; v <= u + 2; ++v)
+                    if (!mbar_wait(&full[(e + v) % R], (uint32_t)((e + v) / R) & 1)) ok = false;
+                if (!ok) break;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                tc_after();
+                const uint32_t as = base + (uint32_t)((e + u) % R) * F::DZROW;
+                const uint32_t bs = base + F::DZ + (uint32_t)((e + u + 2) % R) * F::INROW;
+#pragma unroll 1
+                for (int dk = 0; dk < 3; ++dk)
+#pragma unroll 1
+                    for (int q = 0; q < kv / 16; ++q)
+                        umma(tmem + dk * NG, sdesc(as + q * 256, 128, kWgDzChunk),
+                             sdesc(bs + dk * 16 + q * 256, 128, kWgInChunk), idesc, any || q != 0);
+                any = true;
+                umma_commit(&empty[(e + u) % R]);  // entry u of the unit is not needed again
+            }
+            // nor are the last two
+            if (ok) {
+                umma_commit(&empty[(e + nr + 2) % R]);
+                umma_commit(&empty[(e + nr + 3) % R]);
+            }
+            e += nr + 4;
+        }
+        umma_commit(accb);
+    }
+
+    if (warp < 4) {
+        for (int un = split; !any && un < units; un += a.nsplit) {
+            int i, k0, js, nr, kv;
+            any = unit(un, i, k0, js, nr, kv);
+        }
+        bool done = mbar_wait(accb, 0);
+        done = __all_sync(0xffffffffu, done);
+        tc_after();
+        if (!done) ok = false;
+        if (done) {
+            // lane = (ring row r, output channel n): row r met input row jj
+            // with dj = 2 - r
+            const int r = tid / COUT, n = tid % COUT;
+            const int C = a.in.c0 + a.in.c1;
+#pragma unroll 1
+            for (int c0 = 0; c0 < 3 * NG; c0 += 16) {
+                float acc[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
+                if (r >= 3) continue;
+                const int dk = c0 / NG, c = cb + c0 % NG;
+                const int row = (di * 9 + (2 - r) * 3 + dk) * C + c;
+                float* dst = a.part + ((long)split * a.rows_pad + row) * COUT + n;
+#pragma unroll
+                for (int q = 0; q < 16; ++q) dst[q * COUT] = any ? acc[q] : 0.f;
+            }
+        }
+    }
+
+    if (!ok && a.err) atomicExch(a.err, kErrTimeout);
+    tc_before();
+    __syncthreads();
+    if (warp == 4) {
+        tc_after();
+        mbar_wait(accb, 0);  // no MMA may still write the accumulator
+        tmem_free(tmem, F::NCOLS);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // forward / data-gradient convolution marching along j (n2 % 128 == 0)
 // ---------------------------------------------------------------------------
 // A CTA owns plane i and the 128-voxel k-segment k0 .. k0+127 and walks the
@@ -469,6 +670,68 @@ struct RowShape {
     static constexpr int NCOLS = NOUT <= 32 ? 32 : NOUT <= 64 ? 64 : 128;
     static constexpr int smem = NR * SET + WBYTES + (2 * NR + 6) * 8 + 16;
 };
+
+// One row-set: the rows (i-1 .. i+1, jj) over voxels k0-1 .. k0+128, NH chunks
+// of 8 channels from channel cb on, zero outside the grid.  A thread of the
+// 128 takes a voxel and its chunks of all three rows, so the addresses are
+// formed once per row (per copy, with divisions by the set's shape, they took
+// more issue slots than a set's MMAs: 48 -> 16 channels at 256^3, 3.36 ms).
+template <int NH>
+__device__ __forceinline__ void load_rows(const ConvArgs& a, uint32_t sb, uint32_t row_bytes, int i, int jj, int k0,
+                                          int cb, int lt) {
+    const int n0 = a.n0, n1 = a.n1, n2 = a.n2, up = a.in.up0, c0 = a.in.c0, c1 = a.in.c1;
+    const bool jok = jj >= 0 && jj < n1;
+#pragma unroll
+    for (int di = 0; di < 3; ++di) {
+        const int ii = i + di - 1;
+        const bool rok = jok && ii >= 0 && ii < n0;
+        const bf16* r0 = rok ? a.in.src0 + ((long)(ii >> up) * (n1 >> up) + (jj >> up)) * (n2 >> up) * c0 + cb : a.wpack;
+        const bf16* r1 = rok ? a.in.src1 + ((long)ii * n1 + jj) * n2 * c1 + (cb - c0) : a.wpack;
+        for (int kk = lt; kk < kRowVox; kk += kProducers) {
+            const int k = k0 - 1 + kk;
+            const bool valid = rok && k >= 0 && k < n2;
+            const bf16* p0 = valid ? r0 + (long)(k >> up) * c0 : a.wpack;
+            const bf16* p1 = valid ? r1 + (long)k * c1 : a.wpack;
+            const uint32_t d = sb + di * row_bytes + kk * 16;
+#pragma unroll
+            for (int h = 0; h < NH; ++h)
+                cp16(d + h * kRowChunk, valid ? (cb + h * 8 < c0 ? p0 : p1) + h * 8 : a.wpack, valid);
+        }
+    }
+}
+
+// a row's accumulator (NOUT columns from col, this warp's lanes) to voxel v
+template <int NOUT>
+__device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int warp, long v) {
+#pragma unroll 1
+    for (int c0 = 0; c0 < NOUT; c0 += 16) {
+        float accv[16];
+        tmem_ld16(col + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, accv);
+        if (a.bias) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) accv[q] += a.bias[c0 + q];
+        }
+        if (a.relu) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) accv[q] = fmaxf(accv[q], 0.f);
+        }
+        if (a.mask) {
+            const uint4* mp = reinterpret_cast<const uint4*>(a.mask + v * NOUT + c0);
+            uint4 mv[2] = {mp[0], mp[1]};
+            const bf16* m = reinterpret_cast<const bf16*>(mv);
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                if (!(__bfloat162float(m[q]) > 0.f)) accv[q] = 0.f;
+        }
+        uint4 ov[2];
+        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(ov);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) o[q] = __floats2bfloat162_rn(accv[2 * q], accv[2 * q + 1]);
+        uint4* op = reinterpret_cast<uint4*>(a.out + v * NOUT + c0);
+        op[0] = ov[0];
+        op[1] = ov[1];
+    }
+}
 
 template <int CIN, int NOUT, int NR>
 __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a) {
@@ -529,17 +792,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a) {
                 break;
             }
             const uint32_t sb = base + r * F::SET;
-            const bool jok = jj >= 0 && jj < n1;
-            // 3 rows x 130 voxels x CIN/8 chunks
-            for (int e = lt; e < 3 * kRowVox * (CIN / 8); e += kProducers) {
-                const int di = e / (kRowVox * (CIN / 8));
-                const int rem = e - di * (kRowVox * (CIN / 8));
-                const int h = rem / kRowVox, kk = rem - h * kRowVox;
-                const int ii = i + di - 1, k = k0 - 1 + kk;
-                const bool valid = jok && ii >= 0 && ii < n0 && k >= 0 && k < n2;
-                const bf16* src = valid ? in_ptr(a.in, n1, n2, ii, jj, k, h * 8) : a.wpack;
-                cp16(sb + di * F::ROW + h * kRowChunk + kk * 16, src, valid);
-            }
+            load_rows<CIN / 8>(a, sb, F::ROW, i, jj, k0, 0, lt);
             cp_arrive(&full[r]);
         }
     } else if (tid == 256) {
@@ -600,34 +853,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a) {
             tc_after();
             const int j = js + st;
             const long v = ((long)i * n1 + j) * n2 + k0 + tid;
-#pragma unroll 1
-            for (int c0 = 0; c0 < NOUT; c0 += 16) {
-                float accv[16];
-                tmem_ld16(tmem + (uint32_t)(acc * F::NCOLS) + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, accv);
-                if (a.bias) {
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) accv[q] += a.bias[c0 + q];
-                }
-                if (a.relu) {
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) accv[q] = fmaxf(accv[q], 0.f);
-                }
-                if (a.mask) {
-                    const uint4* mp = reinterpret_cast<const uint4*>(a.mask + v * NOUT + c0);
-                    uint4 mv[2] = {mp[0], mp[1]};
-                    const bf16* m = reinterpret_cast<const bf16*>(mv);
-#pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        if (!(__bfloat162float(m[q]) > 0.f)) accv[q] = 0.f;
-                }
-                uint4 ov[2];
-                __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(ov);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) o[q] = __floats2bfloat162_rn(accv[2 * q], accv[2 * q + 1]);
-                uint4* op = reinterpret_cast<uint4*>(a.out + v * NOUT + c0);
-                op[0] = ov[0];
-                op[1] = ov[1];
-            }
+            store_row<NOUT>(a, tmem + (uint32_t)(acc * F::NCOLS), warp, v);
             tc_before();
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[acc])) : "memory");
         }
@@ -640,6 +866,164 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a) {
         tc_after();
         mbar_wait(fin, 0);  // no MMA may still write the accumulators
         tmem_free(tmem, 2 * F::NCOLS);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// the same for more input channels than one ring and one set of weights hold
+// ---------------------------------------------------------------------------
+// The channels go in groups of CG: a CTA marches its kGrpSeg rows once per
+// group, with that group's weights (two buffers, the next group's load under
+// this one's MMAs), and keeps every row's accumulator in tensor memory from
+// the first group to the last, so partial sums stay in FP32 and never leave
+// the SM.  96 -> 32 channels on 128^3: see conv_launch.
+constexpr int kGrpSeg = 16;
+
+template <int CG, int NOUT, int NR>
+struct GroupShape {
+    static constexpr int ROW = (CG / 8) * kRowChunk;
+    static constexpr int SET = 3 * ROW;
+    static constexpr int WBYTES = 27 * CG * NOUT * 2;
+    static constexpr int NCOLS = kGrpSeg * NOUT;
+    static_assert(NCOLS == 512, "tensor memory");
+    static constexpr int smem = NR * SET + 2 * WBYTES + (2 * NR + 4 + kGrpSeg + 1) * 8 + 16;
+};
+
+template <int CG, int NOUT, int NR>
+__global__ void __launch_bounds__(kRowThreads, 1) k_conv_groups(ConvArgs a) {
+    using F = GroupShape<CG, NOUT, NR>;
+    constexpr int NQ = CG / 16;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + NR * F::SET + 2 * F::WBYTES);
+    uint64_t* empty = full + NR;
+    uint64_t* wfull = empty + NR;     // [2]
+    uint64_t* wempty = wfull + 2;     // [2]
+    uint64_t* tfull = wempty + 2;     // [kGrpSeg]
+    uint64_t* fin = tfull + kGrpSeg;  // every MMA of the CTA has completed
+    uint32_t* slot = reinterpret_cast<uint32_t*>(fin + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int n1 = a.n1, n2 = a.n2;
+    const int k0 = blockIdx.x * kTile;
+    const int i = blockIdx.y;
+    const int js = blockIdx.z * kGrpSeg;
+    const int nsteps = min(kGrpSeg, n1 - js);
+    const int nqt = (a.in.c0 + a.in.c1) / 16, groups = nqt / NQ;
+
+    if (tid == 0) {
+        for (int r = 0; r < NR; ++r) {
+            mbar_init(&full[r], kProducers);
+            mbar_init(&empty[r], 1);
+        }
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(&wfull[q], kProducers);
+            mbar_init(&wempty[q], 1);
+        }
+        for (int q = 0; q < kGrpSeg; ++q) mbar_init(&tfull[q], 1);
+        mbar_init(fin, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 8) tmem_alloc(slot, F::NCOLS);
+    tc_before();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = *slot;
+    bool ok = true;
+    const uint32_t base = smem_u32(smem), wb = base + NR * F::SET;
+
+    if (warp >= 4 && warp < 8) {
+        // ---- loader: per group its weights, then the row-sets js-1 .. je
+        const int lt = tid - 128;
+        int e = 0;  // row-sets so far
+        for (int g = 0; ok && g < groups; ++g) {
+            if (!mbar_wait(&wempty[g & 1], ((uint32_t)(g >> 1) & 1) ^ 1)) {
+                ok = false;
+                break;
+            }
+            // blocks of 16 channels: (tap, block) of the packed weights
+            constexpr int WCH = NOUT * 32 / 16;  // 16-byte pieces of a block
+            for (int c = lt; c < 27 * NQ * WCH; c += kProducers) {
+                const int blk = c / WCH, t = blk / NQ, u = blk - t * NQ;
+                cp16(wb + (g & 1) * F::WBYTES + c * 16,
+                     a.wpack + ((long)(t * nqt + g * NQ + u) * WCH + (c - blk * WCH)) * 8, true);
+            }
+            cp_arrive(&wfull[g & 1]);
+            for (int jj = js - 1; jj <= js + nsteps; ++jj, ++e) {
+                const int r = e % NR;
+                if (!mbar_wait(&empty[r], ((uint32_t)(e / NR) & 1) ^ 1)) {
+                    ok = false;
+                    break;
+                }
+                load_rows<CG / 8>(a, base + r * F::SET, F::ROW, i, jj, k0, g * CG, lt);
+                cp_arrive(&full[r]);
+            }
+        }
+    } else if (tid == 256) {
+        // ---- MMA issue
+        constexpr uint32_t idesc = idesc_bf16(kTile, NOUT, false, false);
+        int e = 0;
+        for (int g = 0; ok && g < groups; ++g) {
+            if (!mbar_wait(&wfull[g & 1], (uint32_t)(g >> 1) & 1)) ok = false;
+            const uint32_t wg = wb + (g & 1) * F::WBYTES;
+            for (int st = 0; ok && st < nsteps; ++st) {
+                for (int q = st == 0 ? 0 : st + 2; q <= st + 2; ++q)
+                    if (!mbar_wait(&full[(e + q) % NR], (uint32_t)((e + q) / NR) & 1)) ok = false;
+                if (!ok) break;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                tc_after();
+                bool first = g == 0;
+#pragma unroll 1
+                for (int dj = 0; dj < 3; ++dj) {
+                    const uint32_t set = base + ((e + st + dj) % NR) * F::SET;
+#pragma unroll 1
+                    for (int di = 0; di < 3; ++di) {
+#pragma unroll
+                        for (int dk = 0; dk < 3; ++dk) {
+#pragma unroll
+                            for (int u = 0; u < NQ; ++u) {
+                                umma(tmem + (uint32_t)(st * NOUT),
+                                     sdesc(set + di * F::ROW + 2 * u * kRowChunk + dk * 16, kRowChunk, 128),
+                                     sdesc(wg + (uint32_t)(((di * 9 + dj * 3 + dk) * NQ + u) * NOUT * 32), 128, 256),
+                                     idesc, first ? 0u : 1u);
+                                first = false;
+                            }
+                        }
+                    }
+                }
+                if (g == groups - 1) umma_commit(&tfull[st]);
+                umma_commit(&empty[(e + st) % NR]);  // the row-set is not needed again in this group
+            }
+            if (ok) {  // nor are the last two, nor the weights
+                umma_commit(&empty[(e + nsteps) % NR]);
+                umma_commit(&empty[(e + nsteps + 1) % NR]);
+                umma_commit(&wempty[g & 1]);
+            }
+            e += nsteps + 2;
+        }
+        umma_commit(fin);
+    }
+
+    if (warp < 4) {
+        // ---- epilogue, row by row as the last group completes them
+        for (int st = 0; st < nsteps; ++st) {
+            bool done = mbar_wait(&tfull[st], 0);
+            done = __all_sync(0xffffffffu, done);
+            if (!done) {
+                ok = false;
+                break;
+            }
+            tc_after();
+            store_row<NOUT>(a, tmem + (uint32_t)(st * NOUT), warp, ((long)i * n1 + js + st) * n2 + k0 + tid);
+        }
+    }
+
+    if (!ok && a.err) atomicExch(a.err, kErrTimeout);
+    tc_before();
+    __syncthreads();
+    if (warp == 8) {
+        tc_after();
+        mbar_wait(fin, 0);  // no MMA may still write the accumulators
+        tmem_free(tmem, F::NCOLS);
     }
 }
 
@@ -670,6 +1054,34 @@ cudaError_t wgrad_inst(const WgradArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <int NG, int COUT>
+cudaError_t wgrad_rows_inst(const WgradArgs& a, cudaStream_t s) {
+    constexpr int smem = WgRowShape<NG, COUT>::smem;
+    static_assert(smem <= 113 * 1024, "two CTAs an SM");
+    cudaError_t e = cudaFuncSetAttribute(k_wgrad_rows<NG, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_wgrad_rows<NG, COUT><<<dim3((unsigned)a.nsplit, 3, (unsigned)((a.in.c0 + a.in.c1) / NG)), kThreads, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
+// input channels of a group: all of them up to 48 (three taps' columns then
+// leave room for two CTAs' accumulators an SM), else halves; 0: not covered
+int wgrad_group(int cin) {
+    switch (cin) {
+        case 16: case 32: case 48: return cin;
+        case 64: return 32;
+        case 96: return 48;
+        default: return 0;
+    }
+}
+
+template <int COUT>
+cudaError_t wgrad_rows(const WgradArgs& a, int ng, cudaStream_t s) {
+    return ng == 16 ? wgrad_rows_inst<16, COUT>(a, s)
+           : ng == 32 ? wgrad_rows_inst<32, COUT>(a, s)
+                      : wgrad_rows_inst<48, COUT>(a, s);
+}
+
 template <int CIN, int NOUT>
 cudaError_t rows_inst(const ConvArgs& a, cudaStream_t s) {
     constexpr int NR = RowShape<CIN, NOUT, 4>::smem <= 200 * 1024 ? 4 : 3;
@@ -683,6 +1095,17 @@ cudaError_t rows_inst(const ConvArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <int CG, int NOUT>
+cudaError_t groups_inst(const ConvArgs& a, cudaStream_t s) {
+    constexpr int NR = 4, smem = GroupShape<CG, NOUT, NR>::smem;
+    static_assert(smem <= 227 * 1024, "group kernel does not fit shared memory");
+    cudaError_t e = cudaFuncSetAttribute(k_conv_groups<CG, NOUT, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((unsigned)(a.n2 / kTile), (unsigned)a.n0, (unsigned)((a.n1 + kGrpSeg - 1) / kGrpSeg));
+    k_conv_groups<CG, NOUT, NR><<<grid, kRowThreads, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 // the row-marching kernel covers these (input channels, output channels)
@@ -690,7 +1113,7 @@ cudaError_t rows_inst(const ConvArgs& a, cudaStream_t s) {
 bool rows_supported(int cin, int nout, int n2) {
     if (n2 % 128) return false;
     return (cin == 16 && (nout == 16 || nout == 32 || nout == 48)) || (cin == 32 && (nout == 16 || nout == 32)) ||
-           (cin == 48 && nout == 16);
+           (cin == 48 && nout == 16) || (cin == 96 && nout == 32);
 }
 
 cudaError_t rows_launch(const ConvArgs& a, int nout, cudaStream_t s) {
@@ -701,6 +1124,7 @@ cudaError_t rows_launch(const ConvArgs& a, int nout, cudaStream_t s) {
     if (cin == 32 && nout == 16) return rows_inst<32, 16>(a, s);
     if (cin == 32 && nout == 32) return rows_inst<32, 32>(a, s);
     if (cin == 48 && nout == 16) return rows_inst<48, 16>(a, s);
+    if (cin == 96 && nout == 32) return groups_inst<32, 32>(a, s);
     return cudaErrorInvalidValue;
 }
 
@@ -737,6 +1161,10 @@ cudaError_t conv_launch(const ConvArgs& a, int kc, int nout, cudaStream_t s) {
 #undef BUN_CONV_CASE
 
 cudaError_t wgrad_launch(const WgradArgs& a, int cout, cudaStream_t s) {
+    // rows of whole 16-voxel groups and channels in whole chunks of 16
+    const int ng = wgrad_group(a.in.c0 + a.in.c1);
+    if (ng && a.n2 % 16 == 0 && a.in.c0 % 8 == 0 && (cout == 16 || cout == 32))
+        return cout == 16 ? wgrad_rows<16>(a, ng, s) : wgrad_rows<32>(a, ng, s);
     if (cout == 16) return wgrad_inst<16>(a, s);
     if (cout == 32) return wgrad_inst<32>(a, s);
     if (cout == 64) return wgrad_inst<64>(a, s);
