@@ -100,6 +100,7 @@ struct HostLevel {
     // ghost refresh between bricks: slab[gdst[q]] = slab[gsrc[q]]
     int* gdst = nullptr;
     int* gsrc = nullptr;
+    int* gmap = nullptr;  // gmap[gdst[q]] = gsrc[q], every other cell itself
     long nghost = 0;
 };
 
@@ -355,6 +356,8 @@ Bricks<T> bricks(const bmg_ctx* c, int l) {
         v.per2 = c->periodic[2];
         v.cpar = K.cpar;
         v.kh = H.ks ? K.n[2] / 2 : 0;
+        v.mask = c->multi && !c->userLambda;
+        v.gmap = H.gmap;
         // a smoothed coarse level of a singular system keeps global cell 0
         // (brick 0's first cell) at zero
         v.pin = l == c->lc && b == 0 && c->singular && c->opt.coarse_mode == BMG_COARSE_SMOOTH;
@@ -579,7 +582,7 @@ void freeAll(bmg_ctx* c) {
     for (auto& L : c->lv) {
         for (void* p : {(void*)L.x64, (void*)L.b64, (void*)L.x32, (void*)L.b32, (void*)L.tab64, (void*)L.tab32,
                         (void*)L.jtmp64, (void*)L.jtmp32, (void*)L.x64b, (void*)L.x32b, (void*)L.gdst,
-                        (void*)L.gsrc})
+                        (void*)L.gsrc, (void*)L.gmap})
             if (p) cudaFree(p);
         for (int d = 0; d < 3; ++d) {
             if (L.lam64[d]) cudaFree(L.lam64[d]);
@@ -1129,6 +1132,11 @@ void build(bmg_ctx* c, HostLevel&& L0) {
             L.gsrc = dalloc<int>(src.size());
             upload(L.gdst, dst);
             upload(L.gsrc, src);
+            std::vector<int> map(L.cells);
+            for (long q = 0; q < L.cells; ++q) map[q] = (int)q;
+            for (size_t q = 0; q < dst.size(); ++q) map[dst[q]] = src[q];
+            L.gmap = dalloc<int>(map.size());
+            upload(L.gmap, map);
         }
     }
     // multi-brick meshes whose faces are partly in contact carry face
@@ -1293,8 +1301,8 @@ void smooth(bmg_ctx* c, int l, int sweeps) {
         }
         return;
     }
+    // (several bricks: the passes read their neighbours through gmap)
     for (int col : seq) {
-        exchange<T>(c, l);
         c->launches += 1;
         if (c->variable)
             launch_colour_pass<T, true>(B, col, s, zeroFirst);

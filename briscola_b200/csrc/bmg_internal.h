@@ -102,6 +102,12 @@ struct LevelView {
     int cpar;          // parity of the brick origin: colour = (i+j+k+cpar) & 1
     int pin;           // smoothers keep cell (0,0,0) at zero: the singularity pin
                        // of an iteratively smoothed coarse level (solver.C:201-231)
+    int mask;          // the face arrays are 1 but on the brick's outer faces (the
+                       // contact mask of a constant coefficient): only cells there
+                       // read them
+    const int* gmap;   // multi-brick levels: for a ghost cell's slab index, the cell
+                       // that it copies (itself beyond a Dirichlet face); the colour
+                       // passes read through it, so they need no ghost refresh
     int kh;            // parity-split rows: offset n2/2 of the odd-k half (see
                        // above); 0: natural k order
 };

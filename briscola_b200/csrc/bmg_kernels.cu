@@ -62,8 +62,16 @@ __global__ void __launch_bounds__(256) k_colour_pass(Bricks<T> B, int colour) {
     if (L.pin && (i | j | k) == 0) return;  // the pinned cell stays zero
     T w[6];
     couplings<T, VAR>(L, i, j, k, c, c + 1, w);  // natural rows only (n2 % 4 != 0)
-    const T xn[6] = {e ? xm.y : xm.x, e ? xp.y : xp.x, e ? ym.y : ym.x, e ? yp.y : yp.x,
-                     e ? own.x : x[c0 - 1], e ? x[c0 + 2] : own.y};
+    T xn[6] = {e ? xm.y : xm.x, e ? xp.y : xp.x, e ? ym.y : ym.x, e ? yp.y : yp.x,
+               e ? own.x : x[c0 - 1], e ? x[c0 + 2] : own.y};
+    if (L.gmap) {  // neighbours in other bricks
+        if (i == 0) xn[0] = x[ldg(L.gmap + c - L.si)];
+        if (i == L.n0 - 1) xn[1] = x[ldg(L.gmap + c + L.si)];
+        if (j == 0) xn[2] = x[ldg(L.gmap + c - L.sj)];
+        if (j == L.n1 - 1) xn[3] = x[ldg(L.gmap + c + L.sj)];
+        if (k == 0) xn[4] = x[ldg(L.gmap + c - 1)];
+        if (k == L.n2 - 1) xn[5] = x[ldg(L.gmap + c + 1)];
+    }
     store_x(L, c, i, j, k, gs_value(w, xn, L.b[c]));
 }
 
@@ -198,15 +206,49 @@ __device__ __forceinline__ void colour_quad_item(const LevelView<T>& L, int i, i
     Row4<T>::ldg4(L.tab + L.to.wl[2] + k0, wkl);
     Row4<T>::ldg4(L.tab + L.to.wh[2] + k0, wkh);
     const T wil = ldg(L.tab + L.to.wl[0] + i), wih = ldg(L.tab + L.to.wh[0] + i);
-    const T left = x[c - 1], right = x[c + 4];
+    T left = x[c - 1], right = x[c + 4];
     const T wjl = ldg(L.tab + L.to.wl[1] + j), wjh = ldg(L.tab + L.to.wh[1] + j);
     // the two cells of the colour: (0, 2) or (1, 3); every array index
     // below is a compile-time constant picked by a select
     const bool odd = ((colour ^ (i + j + k0 + L.cpar)) & 1) != 0;
 #define BMG_SEL(a, e) (odd ? a[(e) + 1] : a[e])
+    if (L.gmap) {  // neighbours in other bricks, of the two cells of the colour
+        auto across = [&](T v[4], int at) {
+            const T a = x[ldg(L.gmap + at + (odd ? 1 : 0))], b = x[ldg(L.gmap + at + (odd ? 3 : 2))];
+            v[0] = v[1] = a;
+            v[2] = v[3] = b;
+        };
+        if (i == 0) across(xm, c - si);
+        if (i == L.n0 - 1) across(xp, c + si);
+        if (j == 0) across(ym, c - sj);
+        if (j == L.n1 - 1) across(yp, c + sj);
+        if (k0 == 0) left = x[ldg(L.gmap + c - 1)];
+        if (k0 + 4 == L.n2) right = x[ldg(L.gmap + c + 4)];
+    }
     T w0[6] = {wil, wih, wjl, wjh, BMG_SEL(wkl, 0), BMG_SEL(wkh, 0)};
     T w2[6] = {wil, wih, wjl, wjh, BMG_SEL(wkl, 2), BMG_SEL(wkh, 2)};
-    if (VAR) {
+    if (VAR && L.mask) {
+        // 1 but on the brick's outer faces
+        const int o = odd ? 1 : 0;
+        if (i == 0) {
+            w0[0] *= ldg(L.lam0 + c + o);
+            w2[0] *= ldg(L.lam0 + c + o + 2);
+        }
+        if (i == L.n0 - 1) {
+            w0[1] *= ldg(L.lam0 + c + si + o);
+            w2[1] *= ldg(L.lam0 + c + si + o + 2);
+        }
+        if (j == 0) {
+            w0[2] *= ldg(L.lam1 + c + o);
+            w2[2] *= ldg(L.lam1 + c + o + 2);
+        }
+        if (j == L.n1 - 1) {
+            w0[3] *= ldg(L.lam1 + c + sj + o);
+            w2[3] *= ldg(L.lam1 + c + sj + o + 2);
+        }
+        if (k0 == 0 && !odd) w0[4] *= ldg(L.lam2 + c);
+        if (k0 + 4 == L.n2 && odd) w2[5] *= ldg(L.lam2 + c + 4);
+    } else if (VAR) {
         T l0[4], l0p[4], l1[4], l1p[4], l2[4];
         Row4<T>::ldg4(L.lam0 + c, l0);
         Row4<T>::ldg4(L.lam0 + c + si, l0p);
@@ -640,12 +682,15 @@ __device__ __forceinline__ void restrict_quad_item(const LevelView<T>& F, const 
             const T left = F.x[cl], right = F.x[cr];
             T l0[4], l0p[4], l1[4], l1p[4], l2[4], l2r = T(1);
             if (VAR) {
-                ldgq(F.lam0 + c, kh, l0);
-                ldgq(F.lam0 + c + si, kh, l0p);
-                ldgq(F.lam1 + c, kh, l1);
-                ldgq(F.lam1 + c + sj, kh, l1p);
-                ldgq(F.lam2 + c, kh, l2);
-                l2r = ldg(F.lam2 + cr);
+                const bool all = !F.mask;  // else 1 but on the brick's outer faces
+#pragma unroll
+                for (int q = 0; q < 4; ++q) l0[q] = l0p[q] = l1[q] = l1p[q] = l2[q] = T(1);
+                if (all || i == 0) ldgq(F.lam0 + c, kh, l0);
+                if (all || i == F.n0 - 1) ldgq(F.lam0 + c + si, kh, l0p);
+                if (all || j == 0) ldgq(F.lam1 + c, kh, l1);
+                if (all || j == F.n1 - 1) ldgq(F.lam1 + c + sj, kh, l1p);
+                if (all || k0 == 0) ldgq(F.lam2 + c, kh, l2);
+                if (all || k0 + 4 == F.n2) l2r = ldg(F.lam2 + cr);
             }
             T r[4];
 #pragma unroll
@@ -1300,8 +1345,10 @@ void launch_colour_pass(const Bricks<T>& B, int colour, cudaStream_t s, bool zer
     if (quads) {
         // one row per thread: two rows per thread (R = 2) measured no faster
         // on the 256^3 level and costs registers in FP64
+        // several bricks: runs of 8 quads (128 bytes of FP32), which bricks of
+        // different row lengths all fill
         const int nq = B.max2 / 4;
-        const dim3 blk = nq >= 32 ? dim3(32, 8, 1) : nq >= 8 ? dim3(8, 32, 1) : dim3(2, 128, 1);
+        const dim3 blk = nq >= 32 && B.nb == 1 ? dim3(32, 8, 1) : nq >= 8 ? dim3(8, 32, 1) : dim3(2, 128, 1);
         launch_k(k_colour_quad<T, VAR>, grid_for(B, nq, blk), blk, 0, s, B, colour);
         return;
     }

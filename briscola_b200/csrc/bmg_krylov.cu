@@ -702,9 +702,11 @@ bool fcg_quads(const Bricks<double>& B) {
     return true;
 }
 
+// several bricks: more plane groups, since many blocks of a plane lie outside
+// their brick
 dim3 quad_grid(const Bricks<double>& B) {
     return dim3((unsigned)((B.max2 / 4 + 15) / 16), (unsigned)((B.max1 + 15) / 16),
-                (unsigned)std::min(B.z0[B.nb], kQuadPlanes));
+                (unsigned)std::min(B.z0[B.nb], B.nb > 1 ? 4 * kQuadPlanes : kQuadPlanes));
 }
 
 }  // namespace

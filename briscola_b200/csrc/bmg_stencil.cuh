@@ -39,12 +39,13 @@ __device__ __forceinline__ void couplings(const LevelView<T>& L, int i, int j, i
     w[4] = ldg(L.tab + L.to.wl[2] + k);
     w[5] = ldg(L.tab + L.to.wh[2] + k);
     if (VAR) {
-        w[0] *= ldg(L.lam0 + c);
-        w[1] *= ldg(L.lam0 + c + L.si);
-        w[2] *= ldg(L.lam1 + c);
-        w[3] *= ldg(L.lam1 + c + L.sj);
-        w[4] *= ldg(L.lam2 + c);
-        w[5] *= ldg(L.lam2 + ckp);
+        const bool all = !L.mask;  // else only the brick's outer faces differ from 1
+        if (all || i == 0) w[0] *= ldg(L.lam0 + c);
+        if (all || i == L.n0 - 1) w[1] *= ldg(L.lam0 + c + L.si);
+        if (all || j == 0) w[2] *= ldg(L.lam1 + c);
+        if (all || j == L.n1 - 1) w[3] *= ldg(L.lam1 + c + L.sj);
+        if (all || k == 0) w[4] *= ldg(L.lam2 + c);
+        if (all || k == L.n2 - 1) w[5] *= ldg(L.lam2 + ckp);
     }
 }
 
