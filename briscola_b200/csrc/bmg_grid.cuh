@@ -56,6 +56,30 @@ __device__ __forceinline__ long block_id() {
     return ((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
 }
 
+// The convergence decision of solver.C:64-95 for a residual norm l2 (one
+// thread): mode 0 the initial one (nf and bnorm are set), 1 after a cycle
+__device__ __forceinline__ void solve_decision(SolveState* st, double l2, int mode) {
+    if (mode == 0) {
+        st->init = l2 / st->nf;
+        st->cur = st->init;
+        st->l2_0 = l2;
+        st->iter = 0;
+    } else {
+        st->cur = l2 / st->nf;
+        st->iter += 1;
+    }
+    st->l2 = l2;
+    st->nan = !isfinite(st->cur);
+    // criterion 1 measures the residual against ||b|| instead of the initial
+    // residual
+    if (st->criterion == 1)
+        st->converged = !((st->bnorm > 0.0) && (st->cur > st->abs_tol) && (l2 > st->rel_tol * st->bnorm));
+    else
+        st->converged = !((st->init > 0.0) && (st->cur > st->abs_tol) &&
+                          (st->cur / (st->init + 1e-20) > st->rel_tol));
+    st->keep_going = !st->nan && ((st->iter < st->max_iter && !st->converged) || st->iter < st->min_iter);
+}
+
 inline dim3 block_for(int n2) {
     // k extent on lanes; small rows give the spare lanes to j
     if (n2 >= 64) return dim3(64, 4, 1);

@@ -1622,6 +1622,27 @@ void tailCycle(bmg_ctx* c, int first) {
         launch_tail_cycle<T, false>(P, c->stream);
 }
 
+// A graphed solve runs its whole loop in the cluster where all its levels
+// fit there and the loop is the reference's FP64 one.
+bool tailSolves(const bmg_ctx* c) {
+    return c->tail == 0 && c->opt.krylov == BMG_KRYLOV_NONE && c->opt.precision == BMG_PRECISION_FP64;
+}
+
+void tailSolve(bmg_ctx* c) {
+    TailPlan<double> P = tailPlan<double>(c, 0);
+    std::vector<unsigned char> ops;
+    std::fill(c->visits.begin(), c->visits.end(), 0);
+    tailSteps(c, 0, 0, ops);
+    P.nops = (int)ops.size();
+    std::copy(ops.begin(), ops.end(), P.ops);
+    P.st = c->st;
+    c->launches += 1;
+    if (c->variable)
+        launch_tail_solve<true>(P, c->stream);
+    else
+        launch_tail_solve<false>(P, c->stream);
+}
+
 // The level solver's turn (bmg_set_level_solver): the level's right-hand
 // side out to the solver, its result back as the level's x.
 void hookSolve(bmg_ctx* c, int l) {
@@ -1870,7 +1891,7 @@ void segPostFcg(bmg_ctx* c, double* xdst) {
 }
 
 // Whole solve as one graph: init -> WHILE(keep_going){ cycle, residual,
-// decision } -> mean removal and store.  Reads b from stage_b (and x from
+// decision } (or one kernel, tailSolve) -> mean removal and store.  Reads b from stage_b (and x from
 // stage_x), writes x to stage_x.
 void captureGraph(bmg_ctx* c, bool zero) {
     destroyGraph(c);
@@ -1894,9 +1915,21 @@ void captureGraph(bmg_ctx* c, bool zero) {
     } restore{c, user};
     cudaStream_t s = c->stream;
     BMG_CUDA(cudaGraphCreate(&c->graph, 0));
-    BMG_CUDA(cudaGraphConditionalHandleCreate(&c->cond, c->graph, 0, 0));
+    if (!tailSolves(c)) BMG_CUDA(cudaGraphConditionalHandleCreate(&c->cond, c->graph, 0, 0));
     const long l0 = c->launches;
     BMG_CUDA(cudaStreamBeginCaptureToGraph(s, c->graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    if (tailSolves(c)) {
+        segInit(c, c->stage_b, c->stage_x, zero, false);
+        tailSolve(c);
+        segPost(c, c->stage_x);
+        cudaGraph_t g = nullptr;
+        BMG_CUDA(cudaStreamEndCapture(s, &g));
+        c->launchesInitPost = c->launches - l0;
+        c->launchesBody = 0;
+        BMG_CUDA(cudaGraphInstantiate(&c->gexec, c->graph, 0));
+        c->graphZero = zero;
+        return;
+    }
     segInit(c, c->stage_b, c->stage_x, zero, true);
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t* deps = nullptr;

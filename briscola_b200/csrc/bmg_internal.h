@@ -259,6 +259,7 @@ struct TailPlan {
     int nlev, nops;
     int zeroStart;       // x of the first level is zero on entry
     LevelView<T> g;      // the first level in global memory
+    struct SolveState* st;  // launch_tail_solve
     T* gx;
     const T* gb;
     const double* ainv;
@@ -287,6 +288,9 @@ void launch_coarse_solve(const Bricks<T>& C, const double* ainv, const int* cidx
 // the coarse end of a cycle in one CTA (bmg_tail.cu)
 template <typename T, bool VAR>
 void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s);
+// the whole FP64 loop of a solve whose level 0 is the first level there
+template <bool VAR>
+void launch_tail_solve(const TailPlan<double>& P, cudaStream_t s);
 cudaError_t configure_tail_kernels();
 template <typename T, bool VAR>
 void launch_residual_out(const Bricks<T>& B, double* r_unscaled_compact, cudaStream_t s);

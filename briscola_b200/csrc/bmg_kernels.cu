@@ -1126,30 +1126,12 @@ __global__ void __launch_bounds__(kFinalThreads) k_finalize(const double* partia
         a3 = sum_partials<kFinalThreads>(partials + 2 * nblocks, nblocks, sh);
     }
     if (threadIdx.x == 0) {
-        const double l2 = sqrt(a1);
         if (mode == 0) {
             // normFactor floor: 1e-12 per cell (solver.C:53-58)
             st->nf = fmax(sqrt(a2), st->ncells * 1e-12);
-            st->init = l2 / st->nf;
-            st->cur = st->init;
-            st->l2_0 = l2;
             st->bnorm = sqrt(a3);
-            st->iter = 0;
-        } else {
-            st->cur = l2 / st->nf;
-            st->iter += 1;
         }
-        st->l2 = l2;
-        st->nan = !isfinite(st->cur);
-        // solver.C:64-95; criterion 1 measures the residual against ||b||
-        // instead of the initial residual
-        if (st->criterion == 1)
-            st->converged = !((st->bnorm > 0.0) && (st->cur > st->abs_tol) && (l2 > st->rel_tol * st->bnorm));
-        else
-            st->converged = !((st->init > 0.0) && (st->cur > st->abs_tol) &&
-                              (st->cur / (st->init + 1e-20) > st->rel_tol));
-        st->keep_going = !st->nan && ((st->iter < st->max_iter && !st->converged) ||
-                                      st->iter < st->min_iter);
+        solve_decision(st, sqrt(a1), mode);
         if (setCondition) cudaGraphSetConditional(cond, st->keep_going ? 1u : 0u);
     }
 }

@@ -32,6 +32,7 @@
 
 #include <cooperative_groups.h>
 
+#include "bmg_grid.cuh"
 #include "bmg_stencil.cuh"
 
 namespace bmg {
@@ -391,7 +392,46 @@ __device__ __forceinline__ void tail_coarse(const TailLevel<T>& C, T* sm, double
     }
 }
 
-template <typename T, bool VAR>
+// ||b - A x||^2 of this CTA's planes of level 0 (unscaled: times the volumes),
+// per cell as k_residual_norm; valid in thread 0
+template <bool VAR>
+__device__ __forceinline__ double tail_residual(const TailPlan<double>& P, const TailLevel<double>& L,
+                                                const double* sm, int rank) {
+    __shared__ double part[kTailThreads / 32];
+    const double* x = sm + L.x;
+    const Own o = own_planes(L, rank);
+    const int cells = o.cnt * L.n1 * L.n2;
+    double a = 0.0;
+    for (int it = threadIdx.x; it < cells; it += kTailThreads) {
+        const int ij = div_by(it, L.mn2), pos = it - ij * L.n2;
+        const int li = div_by(ij, L.mn1), j = ij - li * L.n1, i = o.p0 + li;
+        const int k = pos < L.ne ? 2 * pos : 2 * (pos - L.ne) + 1;
+        const int row = (li + 1) * L.si + (j + 1) * L.sj + 1, c = row + pos;
+        double w[6];
+        tail_couplings<double, VAR>(L, sm, li, i, j, k, w);
+        const double xn[6] = {x[c - L.si], x[c + L.si], x[c - L.sj], x[c + L.sj], x[row + spos(L, k - 1)],
+                              x[row + spos(L, k + 1)]};
+        const double r = res_value(w, xn, x[c], sm[L.b + ij * L.n2 + pos]);
+        const double V = __ldg(P.g.tab64 + P.g.to.h[0] + i) * __ldg(P.g.tab64 + P.g.to.h[1] + j) *
+                         __ldg(P.g.tab64 + P.g.to.h[2] + k);
+        a += (V * r) * (V * r);
+    }
+    for (int s = 16; s > 0; s >>= 1) a += __shfl_xor_sync(0xffffffffu, a, s);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = a;
+    __syncthreads();
+    a = 0.0;
+    if (threadIdx.x < 32) {
+        a = part[threadIdx.x];
+        for (int s = 16; s > 0; s >>= 1) a += __shfl_xor_sync(0xffffffffu, a, s);
+    }
+    return a;
+}
+
+// SOLVE (FP64, the first level is level 0): not one cycle but the solve's
+// whole loop (MG.C:191-242), cycles until the residual decides, bounded by
+// maxIter; a launch and its reload per cycle, the residual's and the
+// decision's launches were half of a 16^3 solve's time.
+template <typename T, bool VAR, bool SOLVE>
 __global__ void __launch_bounds__(kTailThreads, 1) k_tail_cycle(const __grid_constant__ TailPlan<T> P) {
     extern __shared__ __align__(16) double smd[];
     double* sb = smd;  // ncoarse doubles, then the inverse where it fits
@@ -464,30 +504,55 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail_cycle(const __grid_con
     }
     // every CTA has started (its shared memory may be written) and is loaded
     step_end(nranks > 1);
-    for (int s = 0; s < P.nops; ++s) {
-        const int op = ops[s] >> 3, q = ops[s] & 7;
-        const TailLevel<T>& L = lv[q];
-        const bool all = L.dist;  // every CTA takes part, and the cluster's barrier ends each pass
-        if (op == TAIL_PRE || op == TAIL_POST) {
-            if (all || !rank)
-                tail_smooth<T, VAR>(L, sm, rank, op == TAIL_PRE ? L.pre : L.post, op == TAIL_PRE ? L.npre : L.npost);
-        } else if (op == TAIL_RESTRICT) {
-            if (!all && rank) continue;
-            tail_restrict<T, VAR>(L, lv[q + 1], sm, rank);
-            step_end(all);
-        } else if (op == TAIL_PROLONG) {
-            if (!all && rank) continue;
-            // the coarse level is complete (CTA 0 may have worked alone on it)
-            if (all && !lv[q + 1].dist) step_end(true);
-            tail_prolong<T>(L, lv[q + 1], sm, rank, P.scratch);
-            step_end(all);
-        } else if (P.spread) {
-            step_end(true);
-            tail_coarse<T>(L, sm, sb, ainv, P.ncoarse, rank, nranks);
-            step_end(true);
-        } else if (!rank) {
-            tail_coarse<T>(L, sm, sb, ainv, P.ncoarse, 0, 1);
-            __syncthreads();
+    // the CTAs' shares of the norm and the decision, in CTA 0's and every
+    // CTA's shared memory
+    __shared__ double norms[kTailRanks];
+    __shared__ int go;
+    if (SOLVE && threadIdx.x == 0) go = P.st->keep_going;
+    if (SOLVE) __syncthreads();
+    while (!SOLVE || go) {
+        for (int s = 0; s < P.nops; ++s) {
+            const int op = ops[s] >> 3, q = ops[s] & 7;
+            const TailLevel<T>& L = lv[q];
+            const bool all = L.dist;  // every CTA takes part, and the cluster's barrier ends each pass
+            if (op == TAIL_PRE || op == TAIL_POST) {
+                if (all || !rank)
+                    tail_smooth<T, VAR>(L, sm, rank, op == TAIL_PRE ? L.pre : L.post, op == TAIL_PRE ? L.npre : L.npost);
+            } else if (op == TAIL_RESTRICT) {
+                if (!all && rank) continue;
+                tail_restrict<T, VAR>(L, lv[q + 1], sm, rank);
+                step_end(all);
+            } else if (op == TAIL_PROLONG) {
+                if (!all && rank) continue;
+                // the coarse level is complete (CTA 0 may have worked alone on it)
+                if (all && !lv[q + 1].dist) step_end(true);
+                tail_prolong<T>(L, lv[q + 1], sm, rank, P.scratch);
+                step_end(all);
+            } else if (P.spread) {
+                step_end(true);
+                tail_coarse<T>(L, sm, sb, ainv, P.ncoarse, rank, nranks);
+                step_end(true);
+            } else if (!rank) {
+                tail_coarse<T>(L, sm, sb, ainv, P.ncoarse, 0, 1);
+                __syncthreads();
+            }
+        }
+        if constexpr (SOLVE) {
+            const double a = tail_residual<VAR>(P, lv[0], sm, rank);
+            if (threadIdx.x == 0) st_cluster(word_at(norms + rank, 0), a);
+            step_end(nranks > 1);
+            if (!rank && threadIdx.x == 0) {
+                double l2 = 0.0;
+                for (int r = 0; r < nranks; ++r) l2 += norms[r];
+                solve_decision(P.st, sqrt(l2), 1);
+                for (int r = 0; r < nranks; ++r) {
+                    const unsigned d = word_at(&go, r);
+                    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(d), "r"(P.st->keep_going) : "memory");
+                }
+            }
+            step_end(nranks > 1);
+        } else {
+            break;
         }
     }
     // x of the first level with its periodic images.  In a cluster of several
@@ -505,8 +570,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail_cycle(const __grid_con
 
 }  // namespace
 
-template <typename T, bool VAR>
-void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s) {
+template <typename T, bool VAR, bool SOLVE>
+static void launch_tail(const TailPlan<T>& P, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P.ranks);
     cfg.blockDim = dim3(kTailThreads);
@@ -521,20 +586,30 @@ void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s) {
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = kProgrammaticLaunch ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, k_tail_cycle<T, VAR>, P);
+    cudaLaunchKernelEx(&cfg, k_tail_cycle<T, VAR, SOLVE>, P);
 }
 
 template <typename T, bool VAR>
+void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s) {
+    launch_tail<T, VAR, false>(P, s);
+}
+
+template <bool VAR>
+void launch_tail_solve(const TailPlan<double>& P, cudaStream_t s) {
+    launch_tail<double, VAR, true>(P, s);
+}
+
+template <typename T, bool VAR, bool SOLVE = false>
 static cudaError_t allow_tail() {
     const cudaError_t e =
-        cudaFuncSetAttribute(k_tail_cycle<T, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem);
+        cudaFuncSetAttribute(k_tail_cycle<T, VAR, SOLVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_tail_cycle<T, VAR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return cudaFuncSetAttribute(k_tail_cycle<T, VAR, SOLVE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
 cudaError_t configure_tail_kernels() {
     for (cudaError_t e : {allow_tail<float, false>(), allow_tail<float, true>(), allow_tail<double, false>(),
-                          allow_tail<double, true>()})
+                          allow_tail<double, true>(), allow_tail<double, false, true>(), allow_tail<double, true, true>()})
         if (e != cudaSuccess) return e;
     return cudaSuccess;
 }
@@ -543,5 +618,7 @@ template void launch_tail_cycle<double, false>(const TailPlan<double>&, cudaStre
 template void launch_tail_cycle<double, true>(const TailPlan<double>&, cudaStream_t);
 template void launch_tail_cycle<float, false>(const TailPlan<float>&, cudaStream_t);
 template void launch_tail_cycle<float, true>(const TailPlan<float>&, cudaStream_t);
+template void launch_tail_solve<false>(const TailPlan<double>&, cudaStream_t);
+template void launch_tail_solve<true>(const TailPlan<double>&, cudaStream_t);
 
 }  // namespace bmg
