@@ -40,6 +40,8 @@
 
 #include "bun_internal.h"
 
+#include <algorithm>
+
 namespace bun {
 
 namespace {
@@ -640,73 +642,88 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// forward / data-gradient convolution marching along j (n2 % 128 == 0)
+// forward / data-gradient convolution marching along j
 // ---------------------------------------------------------------------------
-// A CTA owns plane i and the 128-voxel k-segment k0 .. k0+127 and walks the
-// rows j of a segment of kJSeg rows.  For output row j it needs the input
-// rows (i+di, j+dj), di, dj in {-1, 0, 1}, over k0-1 .. k0+128; they live in
-// a ring of NR row-sets (a row-set = the three rows di = -1, 0, 1 of one j')
-// filled once per j' by cp.async, laid out per row as [8-channel chunk h]
-// [voxel 0 .. 129] x 16 bytes.  The operand of tap (di, dj, dk) and channels
-// 16u .. 16u+15 is then a K-major no-swizzle matrix starting at
-//   row(j+dj, di) + 2u * 2080 + (dk + 1) * 16
-// with 2080 bytes between channel chunks (leading byte offset) and 128 bytes
-// between groups of 8 voxels (stride byte offset): shifting along k is a
-// change of start address, so every input row is loaded once, not 27 times.
-// All weights stay in shared memory; the TMEM accumulator is double-
-// buffered so the epilogue of row j overlaps the MMAs of row j+1.
-// Warps 0-3: epilogue (thread = voxel = TMEM lane); warps 4-7: row loader;
-// warp 8: TMEM allocation, one thread issues the MMAs.
-constexpr int kRowVox = 130;                 // k0-1 .. k0+128
-constexpr int kRowChunk = kRowVox * 16;      // bytes of one 8-channel chunk of a row
-constexpr int kJSeg = 32;                    // rows per CTA
+// A CTA owns 128 positions of a plane (fixed j) of the grid and JS rows j, and
+// walks the input rows jj = js-1 .. je, each loaded once by cp.async into a
+// ring.  A position of row jj and its neighbours (di, dk) lie P di + dk apart in
+// the loaded run, one of two ways:
+//   n2 % 128 == 0  128 voxels k0 .. k0+127 of plane i, the run being the three
+//                  rows i-1 .. i+1 over k0-1 .. k0+128 (P = 130);
+//   else           a stretch of the planes' rows one behind another with one
+//                  zero voxel between them, the halo of both (P = n2 + 1), so
+//                  short rows fill the 128 positions too.
+// The run is laid out as [8-channel chunk h][position] x 16 bytes.  The A operand
+// of (di, dk) and channels 16u .. 16u+15 is then a K-major no-swizzle matrix
+// starting at chunk 2u, position P di + dk, with the chunks' distance as
+// leading and 128 bytes (8 positions) as stride byte offset: a tap is a change
+// of start address.
+// With 16 to 48 output channels an MMA costs what its A operand's 4 KB cost
+// (54 cycles for N up to 48), whatever N is, so the three dj of (di, dk) are one
+// MMA: the input row's products for output rows jj-1, jj and jj+1, whose
+// accumulators are neighbours in tensor memory (all JS rows' are there, zeroed
+// at the start), with the weights of dj = 2, 1, 0 side by side as B.
+// Input channels go in groups of CG: the CTA walks its rows once per group
+// with that group's weights (two buffers, the next group's load under this
+// one's MMAs); the sums stay in FP32 in tensor memory from the first group to
+// the last.
+// Warps 0-3: epilogue (thread = position = TMEM lane), a row as soon as the
+// last group completes it; warps 4-7: loader; warp 8: TMEM allocation, one
+// thread issues the MMAs.
+// Measured against a tap an MMA on the n2 % 128 == 0 rows, the only ones that
+// marched, and against k_conv elsewhere (256^3 network, cin -> nout at the
+// level's size, us before / now; two thirds of the time is the rows' supply and
+// the hand-over between the warps, not the MMAs):
+//   256^3  16 -> 16   663 /  592     48 -> 16   3359 / 1336
+//   128^3  96 -> 32  2869 /  442     (16 -> 32: 145, 32 -> 32: 196)
+//    64^3  32 -> 64   119 /   47     64 -> 64    319 /   78   128 -> 64  589 / 139
+//    32^3  64 -> 64    50 /   21;  16^3 64 -> 64   30 /   17
 constexpr int kRowThreads = 288;
+constexpr int kRowRing = 8;  // most rows of the ring
+constexpr int kSms = 148;
 
-template <int CIN, int NOUT, int NR>
-struct RowShape {
-    static constexpr int ROW = (CIN / 8) * kRowChunk;  // one input row
-    static constexpr int SET = 3 * ROW;                // rows di = -1, 0, 1
-    static constexpr int WBYTES = 27 * CIN * NOUT * 2;
-    static constexpr int NCOLS = NOUT <= 32 ? 32 : NOUT <= 64 ? 64 : 128;
-    static constexpr int smem = NR * SET + WBYTES + (2 * NR + 6) * 8 + 16;
+struct RowPlan {
+    int P;       // distance of the planes' rows in the run
+    int nvox;    // positions of the run: 2 P + 130
+    int nr;      // rows of the ring
+    int rows;    // rows j a CTA, at most JS
+    int stream;  // rows one behind another
 };
 
-// One row-set: the rows (i-1 .. i+1, jj) over voxels k0-1 .. k0+128, NH chunks
-// of 8 channels from channel cb on, zero outside the grid.  A thread of the
-// 128 takes a voxel and its chunks of all three rows, so the addresses are
-// formed once per row (per copy, with divisions by the set's shape, they took
-// more issue slots than a set's MMAs: 48 -> 16 channels at 256^3, 3.36 ms).
-template <int NH>
-__device__ __forceinline__ void load_rows(const ConvArgs& a, uint32_t sb, uint32_t row_bytes, int i, int jj, int k0,
-                                          int cb, int lt) {
-    const int n0 = a.n0, n1 = a.n1, n2 = a.n2, up = a.in.up0, c0 = a.in.c0, c1 = a.in.c1;
-    const bool jok = jj >= 0 && jj < n1;
-#pragma unroll
-    for (int di = 0; di < 3; ++di) {
-        const int ii = i + di - 1;
-        const bool rok = jok && ii >= 0 && ii < n0;
-        const bf16* r0 = rok ? a.in.src0 + ((long)(ii >> up) * (n1 >> up) + (jj >> up)) * (n2 >> up) * c0 + cb : a.wpack;
-        const bf16* r1 = rok ? a.in.src1 + ((long)ii * n1 + jj) * n2 * c1 + (cb - c0) : a.wpack;
-        for (int kk = lt; kk < kRowVox; kk += kProducers) {
-            const int k = k0 - 1 + kk;
-            const bool valid = rok && k >= 0 && k < n2;
-            const bf16* p0 = valid ? r0 + (long)(k >> up) * c0 : a.wpack;
-            const bf16* p1 = valid ? r1 + (long)k * c1 : a.wpack;
-            const uint32_t d = sb + di * row_bytes + kk * 16;
-#pragma unroll
-            for (int h = 0; h < NH; ++h)
-                cp16(d + h * kRowChunk, valid ? (cb + h * 8 < c0 ? p0 : p1) + h * 8 : a.wpack, valid);
-        }
+template <int CG, int NOUT, int JS>
+struct RowShape {
+    static constexpr int WBYTES = 27 * CG * NOUT * 2;
+    static constexpr uint32_t NCOLS = JS * NOUT <= 256 ? 256 : 512;
+    static constexpr int BARS = (2 * kRowRing + 4 + JS + 1) * 8 + 16;
+    // longest run: P of 256 (or 130; groups of 32 have rows below 128 only)
+    static constexpr int MAXVOX = CG == 16 ? 2 * 256 + kTile + 2 : 2 * 130 + kTile + 2;
+    static_assert(JS * NOUT <= 512 && 3 * NOUT <= 256, "tensor memory");
+};
+
+// the plane and voxel of a position of the run (q = 0: one row and one voxel
+// before the CTA's first position); false outside the grid
+__device__ __forceinline__ bool row_voxel(const ConvArgs& a, const RowPlan& R, int q, int& i, int& k) {
+    if (R.stream) {
+        const int g = (int)blockIdx.x * kTile - 1 + q;  // counted from the plane before the first
+        i = g < 0 ? -1 : g / R.P - 1;
+        k = g - (i + 1) * R.P;
+    } else {
+        const int nk = a.n2 / kTile, di = q / R.P;
+        i = (int)blockIdx.x / nk + di - 1;
+        k = ((int)blockIdx.x % nk) * kTile - 1 + (q - di * R.P);
     }
+    return i >= 0 && i < a.n0 && k >= 0 && k < a.n2;
 }
 
-// a row's accumulator (NOUT columns from col, this warp's lanes) to voxel v
+// a row's accumulator (NOUT columns from col, this warp's lanes) to voxel v, if
+// the position is one
 template <int NOUT>
-__device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int warp, long v) {
+__device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int warp, long v, bool live) {
 #pragma unroll 1
     for (int c0 = 0; c0 < NOUT; c0 += 16) {
         float accv[16];
         tmem_ld16(col + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, accv);
+        if (!live) continue;
         if (a.bias) {
 #pragma unroll
             for (int q = 0; q < 16; ++q) accv[q] += a.bias[c0 + q];
@@ -733,181 +750,34 @@ __device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int w
     }
 }
 
-template <int CIN, int NOUT, int NR>
-__global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a) {
-    using F = RowShape<CIN, NOUT, NR>;
-    constexpr int NQ = CIN / 16;
-    extern __shared__ __align__(1024) uint8_t smem[];
-    // the NR row slots start at smem (addressed through `base` below)
-    uint8_t* wts = smem + NR * F::SET;
-    uint64_t* full = reinterpret_cast<uint64_t*>(wts + F::WBYTES);
-    uint64_t* empty = full + NR;
-    uint64_t* wbar = empty + NR;
-    uint64_t* tfull = wbar + 1;   // [2]
-    uint64_t* tempty = tfull + 2; // [2]
-    uint64_t* fin = tempty + 2;   // every MMA of the CTA has completed
-    uint32_t* slot = reinterpret_cast<uint32_t*>(fin + 1);
-
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int n0 = a.n0, n1 = a.n1, n2 = a.n2;
-    const int k0 = blockIdx.x * kTile;
-    const int i = blockIdx.y;
-    const int js = blockIdx.z * kJSeg;
-    const int je = min(js + kJSeg, n1);
-    const int nsteps = je - js;
-
-    if (tid == 0) {
-        for (int r = 0; r < NR; ++r) {
-            mbar_init(&full[r], kProducers);
-            mbar_init(&empty[r], 1);
-        }
-        mbar_init(wbar, kProducers);
-        for (int q = 0; q < 2; ++q) {
-            mbar_init(&tfull[q], 1);
-            mbar_init(&tempty[q], kProducers);
-        }
-        mbar_init(fin, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 8) tmem_alloc(slot, 2 * F::NCOLS);
-    tc_before();
-    __syncthreads();
-    tc_after();
-    const uint32_t tmem = *slot;
-    bool ok = true;
-    const uint32_t base = smem_u32(smem);
-
-    if (warp >= 4 && warp < 8) {
-        // ---- loader: weights once, then the row-sets js-1 .. je
-        const int lt = tid - 128;
-        const uint32_t wb = base + NR * F::SET;
-        for (int c = lt; c < F::WBYTES / 16; c += kProducers) cp16(wb + c * 16, a.wpack + c * 8, true);
-        cp_arrive(wbar);
-        for (int jj = js - 1; jj <= je; ++jj) {
-            const int q = jj - (js - 1);
-            const int r = q % NR;
-            const uint32_t use = (uint32_t)(q / NR);
-            if (!mbar_wait(&empty[r], (use & 1) ^ 1)) {
-                ok = false;
-                break;
-            }
-            const uint32_t sb = base + r * F::SET;
-            load_rows<CIN / 8>(a, sb, F::ROW, i, jj, k0, 0, lt);
-            cp_arrive(&full[r]);
-        }
-    } else if (tid == 256) {
-        // ---- MMA issue
-        constexpr uint32_t idesc = idesc_bf16(kTile, NOUT, false, false);
-        const uint32_t wb = base + NR * F::SET;
-        if (!mbar_wait(wbar, 0)) ok = false;
-        for (int st = 0; ok && st < nsteps; ++st) {
-            const int acc = st & 1;
-            const uint32_t ause = (uint32_t)(st >> 1);
-            if (!mbar_wait(&tempty[acc], (ause & 1) ^ 1)) {
-                ok = false;
-                break;
-            }
-            // row-sets st-1+1 .. st+1+1 in ring order (q = jj - (js-1))
-            for (int q = (st == 0 ? 0 : st + 2); q <= st + 2; ++q) {
-                if (!mbar_wait(&full[q % NR], (uint32_t)(q / NR) & 1)) ok = false;
-            }
-            if (!ok) break;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            tc_after();
-            const uint32_t d = tmem + (uint32_t)(acc * F::NCOLS);
-            bool first = true;
-#pragma unroll 1
-            for (int dj = 0; dj < 3; ++dj) {
-                const uint32_t set = base + ((st + dj) % NR) * F::SET;
-#pragma unroll 1
-                for (int di = 0; di < 3; ++di) {
-#pragma unroll
-                    for (int dk = 0; dk < 3; ++dk) {
-                        const int t = di * 9 + dj * 3 + dk;
-#pragma unroll
-                        for (int u = 0; u < NQ; ++u) {
-                            const uint32_t as = set + di * F::ROW + 2 * u * kRowChunk + dk * 16;
-                            const uint32_t bs = wb + (uint32_t)((t * NQ + u) * NOUT * 32);
-                            umma(d, sdesc(as, kRowChunk, 128), sdesc(bs, 128, 256), idesc, first ? 0u : 1u);
-                            first = false;
-                        }
-                    }
-                }
-            }
-            umma_commit(&tfull[acc]);
-            umma_commit(&empty[st % NR]);  // row-set js-1+st is not needed again
-        }
-        umma_commit(fin);  // one phase, after every MMA issued above
-    }
-
-    if (warp < 4) {
-        // ---- epilogue
-        for (int st = 0; st < nsteps; ++st) {
-            const int acc = st & 1;
-            bool done = mbar_wait(&tfull[acc], (uint32_t)(st >> 1) & 1);
-            done = __all_sync(0xffffffffu, done);
-            if (!done) {
-                ok = false;
-                break;
-            }
-            tc_after();
-            const int j = js + st;
-            const long v = ((long)i * n1 + j) * n2 + k0 + tid;
-            store_row<NOUT>(a, tmem + (uint32_t)(acc * F::NCOLS), warp, v);
-            tc_before();
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[acc])) : "memory");
-        }
-    }
-
-    if (!ok && a.err) atomicExch(a.err, kErrTimeout);
-    tc_before();
-    __syncthreads();
-    if (warp == 8) {
-        tc_after();
-        mbar_wait(fin, 0);  // no MMA may still write the accumulators
-        tmem_free(tmem, 2 * F::NCOLS);
-    }
+// this warp's 32 lanes of 16 consecutive columns to zero
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
+        ::"r"(taddr), "r"(0)
+        : "memory");
 }
 
-// ---------------------------------------------------------------------------
-// the same for more input channels than one ring and one set of weights hold
-// ---------------------------------------------------------------------------
-// The channels go in groups of CG: a CTA marches its kGrpSeg rows once per
-// group, with that group's weights (two buffers, the next group's load under
-// this one's MMAs), and keeps every row's accumulator in tensor memory from
-// the first group to the last, so partial sums stay in FP32 and never leave
-// the SM.  96 -> 32 channels on 128^3: see conv_launch.
-constexpr int kGrpSeg = 16;
-
-template <int CG, int NOUT, int NR>
-struct GroupShape {
-    static constexpr int ROW = (CG / 8) * kRowChunk;
-    static constexpr int SET = 3 * ROW;
-    static constexpr int WBYTES = 27 * CG * NOUT * 2;
-    static constexpr int NCOLS = kGrpSeg * NOUT;
-    static_assert(NCOLS == 512, "tensor memory");
-    static constexpr int smem = NR * SET + 2 * WBYTES + (2 * NR + 4 + kGrpSeg + 1) * 8 + 16;
-};
-
-template <int CG, int NOUT, int NR>
-__global__ void __launch_bounds__(kRowThreads, 1) k_conv_groups(ConvArgs a) {
-    using F = GroupShape<CG, NOUT, NR>;
+template <int CG, int NOUT, int JS>
+__global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a, RowPlan R) {
+    using F = RowShape<CG, NOUT, JS>;
     constexpr int NQ = CG / 16;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + NR * F::SET + 2 * F::WBYTES);
-    uint64_t* empty = full + NR;
-    uint64_t* wfull = empty + NR;     // [2]
-    uint64_t* wempty = wfull + 2;     // [2]
-    uint64_t* tfull = wempty + 2;     // [kGrpSeg]
-    uint64_t* fin = tfull + kGrpSeg;  // every MMA of the CTA has completed
+    const int NR = R.nr;
+    const uint32_t chunk = (uint32_t)R.nvox * 16, set_bytes = (CG / 8) * chunk;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + NR * set_bytes + 2 * F::WBYTES);
+    uint64_t* empty = full + kRowRing;
+    uint64_t* wfull = empty + kRowRing;   // [2]
+    uint64_t* wempty = wfull + 2;   // [2]
+    uint64_t* tfull = wempty + 2;   // [JS]
+    uint64_t* fin = tfull + JS;     // every MMA of the CTA has completed
     uint32_t* slot = reinterpret_cast<uint32_t*>(fin + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5;
     const int n1 = a.n1, n2 = a.n2;
-    const int k0 = blockIdx.x * kTile;
-    const int i = blockIdx.y;
-    const int js = blockIdx.z * kGrpSeg;
-    const int nsteps = min(kGrpSeg, n1 - js);
+    const int js = blockIdx.y * R.rows, je = min(js + R.rows, n1);
+    // input rows inside the grid (those outside are zero)
+    const int jlo = max(js - 1, 0), jhi = min(je, n1 - 1);
     const int nqt = (a.in.c0 + a.in.c1) / 16, groups = nqt / NQ;
 
     if (tid == 0) {
@@ -919,7 +789,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_groups(ConvArgs a) {
             mbar_init(&wfull[q], kProducers);
             mbar_init(&wempty[q], 1);
         }
-        for (int q = 0; q < kGrpSeg; ++q) mbar_init(&tfull[q], 1);
+        for (int q = 0; q < JS; ++q) mbar_init(&tfull[q], 1);
         mbar_init(fin, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -928,92 +798,121 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_groups(ConvArgs a) {
     __syncthreads();
     tc_after();
     const uint32_t tmem = *slot;
+    if (warp < 4) {
+#pragma unroll 1
+        for (int c = 0; c < JS * NOUT; c += 16) tmem_zero16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    tc_before();
+    __syncthreads();
+    tc_after();
     bool ok = true;
-    const uint32_t base = smem_u32(smem), wb = base + NR * F::SET;
+    const uint32_t base = smem_u32(smem), wb = base + NR * set_bytes;
 
     if (warp >= 4 && warp < 8) {
-        // ---- loader: per group its weights, then the row-sets js-1 .. je
-        const int lt = tid - 128;
+        // ---- loader: per group its weights, then its row-sets; the thread
+        // fetches chunk h of positions q0, q0 + QS, ..., whose voxels (of row 0,
+        // in either source; -1 outside the grid) it keeps
+        constexpr int QS = kProducers * 8 / CG, M = (F::MAXVOX + QS - 1) / QS;
+        const int lt = tid - 128, h = lt % (CG / 8), q0 = lt / (CG / 8);
+        const int up = a.in.up0, c0 = a.in.c0;
+        int v0[M], v1[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            int i, k;
+            const bool valid = row_voxel(a, R, q0 + m * QS, i, k);
+            v0[m] = valid ? (i >> up) * (n1 >> up) * (n2 >> up) + (k >> up) : -1;
+            v1[m] = valid ? i * n1 * n2 + k : -1;
+        }
         int e = 0;  // row-sets so far
         for (int g = 0; ok && g < groups; ++g) {
             if (!mbar_wait(&wempty[g & 1], ((uint32_t)(g >> 1) & 1) ^ 1)) {
                 ok = false;
                 break;
             }
-            // blocks of 16 channels: (tap, block) of the packed weights
+            // packed blocks (tap, 16 channels) to ((di, dk), u, dj = 2, 1, 0)
             constexpr int WCH = NOUT * 32 / 16;  // 16-byte pieces of a block
             for (int c = lt; c < 27 * NQ * WCH; c += kProducers) {
                 const int blk = c / WCH, t = blk / NQ, u = blk - t * NQ;
-                cp16(wb + (g & 1) * F::WBYTES + c * 16,
+                const int di = t / 9, dj = (t / 3) % 3, dk = t % 3;
+                cp16(wb + (g & 1) * F::WBYTES + ((((di * 3 + dk) * NQ + u) * 3 + 2 - dj) * WCH + (c - blk * WCH)) * 16,
                      a.wpack + ((long)(t * nqt + g * NQ + u) * WCH + (c - blk * WCH)) * 8, true);
             }
             cp_arrive(&wfull[g & 1]);
-            for (int jj = js - 1; jj <= js + nsteps; ++jj, ++e) {
+            const int ch = g * CG + h * 8;
+            const bool first = ch < c0;
+            for (int jj = jlo; jj <= jhi; ++jj, ++e) {
                 const int r = e % NR;
                 if (!mbar_wait(&empty[r], ((uint32_t)(e / NR) & 1) ^ 1)) {
                     ok = false;
                     break;
                 }
-                load_rows<CG / 8>(a, base + r * F::SET, F::ROW, i, jj, k0, g * CG, lt);
+                const bf16* p = first ? a.in.src0 + (long)(jj >> up) * (n2 >> up) * c0 + ch
+                                      : a.in.src1 + (long)jj * n2 * a.in.c1 + (ch - c0);
+                const int cs = first ? c0 : a.in.c1;
+                const uint32_t d = base + r * set_bytes + h * chunk + q0 * 16;
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int v = first ? v0[m] : v1[m];
+                    if (q0 + m * QS < R.nvox) cp16(d + m * QS * 16, v >= 0 ? p + (long)v * cs : a.wpack, v >= 0);
+                }
                 cp_arrive(&full[r]);
             }
         }
     } else if (tid == 256) {
         // ---- MMA issue
-        constexpr uint32_t idesc = idesc_bf16(kTile, NOUT, false, false);
         int e = 0;
         for (int g = 0; ok && g < groups; ++g) {
             if (!mbar_wait(&wfull[g & 1], (uint32_t)(g >> 1) & 1)) ok = false;
             const uint32_t wg = wb + (g & 1) * F::WBYTES;
-            for (int st = 0; ok && st < nsteps; ++st) {
-                for (int q = st == 0 ? 0 : st + 2; q <= st + 2; ++q)
-                    if (!mbar_wait(&full[(e + q) % NR], (uint32_t)((e + q) / NR) & 1)) ok = false;
-                if (!ok) break;
+            for (int jj = jlo; ok && jj <= jhi; ++jj, ++e) {
+                if (!mbar_wait(&full[e % NR], (uint32_t)(e / NR) & 1)) {
+                    ok = false;
+                    break;
+                }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 tc_after();
-                bool first = g == 0;
-#pragma unroll 1
-                for (int dj = 0; dj < 3; ++dj) {
-                    const uint32_t set = base + ((e + st + dj) % NR) * F::SET;
-#pragma unroll 1
-                    for (int di = 0; di < 3; ++di) {
+                // output rows lo .. hi of jj-1 .. jj+1 lie in the segment
+                const int lo = max(js, jj - 1), hi = min(je - 1, jj + 1);
+                const uint32_t idesc = idesc_bf16(kTile, (hi - lo + 1) * NOUT, false, false);
+                const uint32_t d = tmem + (uint32_t)((lo - js) * NOUT);
+                const uint32_t set = base + (e % NR) * set_bytes, wj = wg + (uint32_t)((lo - (jj - 1)) * NOUT * 32);
 #pragma unroll
-                        for (int dk = 0; dk < 3; ++dk) {
+                for (int di = 0; di < 3; ++di) {
 #pragma unroll
-                            for (int u = 0; u < NQ; ++u) {
-                                umma(tmem + (uint32_t)(st * NOUT),
-                                     sdesc(set + di * F::ROW + 2 * u * kRowChunk + dk * 16, kRowChunk, 128),
-                                     sdesc(wg + (uint32_t)(((di * 9 + dj * 3 + dk) * NQ + u) * NOUT * 32), 128, 256),
-                                     idesc, first ? 0u : 1u);
-                                first = false;
-                            }
-                        }
+                    for (int dk = 0; dk < 3; ++dk) {
+#pragma unroll
+                        for (int u = 0; u < NQ; ++u)
+                            umma(d, sdesc(set + 2 * u * chunk + (di * R.P + dk) * 16, chunk, 128),
+                                 sdesc(wj + (uint32_t)(((di * 3 + dk) * NQ + u) * 3 * NOUT * 32), 128, 256), idesc, 1u);
                     }
                 }
-                if (g == groups - 1) umma_commit(&tfull[st]);
-                umma_commit(&empty[(e + st) % NR]);  // the row-set is not needed again in this group
+                umma_commit(&empty[e % NR]);
+                if (g == groups - 1) {
+                    // complete: the row before, and at the end the last one
+                    if (jj - 1 >= js) umma_commit(&tfull[jj - 1 - js]);
+                    if (jj == jhi && jj < je) umma_commit(&tfull[jj - js]);
+                }
             }
-            if (ok) {  // nor are the last two, nor the weights
-                umma_commit(&empty[(e + nsteps) % NR]);
-                umma_commit(&empty[(e + nsteps + 1) % NR]);
-                umma_commit(&wempty[g & 1]);
-            }
-            e += nsteps + 2;
+            if (ok) umma_commit(&wempty[g & 1]);
         }
         umma_commit(fin);
     }
 
     if (warp < 4) {
-        // ---- epilogue, row by row as the last group completes them
-        for (int st = 0; st < nsteps; ++st) {
-            bool done = mbar_wait(&tfull[st], 0);
+        // ---- epilogue: position tid of the tile, one row and one voxel into
+        // the run
+        int i, k;
+        const bool live = row_voxel(a, R, R.P + 1 + tid, i, k);
+        for (int j = js; j < je; ++j) {
+            bool done = mbar_wait(&tfull[j - js], 0);
             done = __all_sync(0xffffffffu, done);
             if (!done) {
                 ok = false;
                 break;
             }
             tc_after();
-            store_row<NOUT>(a, tmem + (uint32_t)(st * NOUT), warp, ((long)i * n1 + js + st) * n2 + k0 + tid);
+            store_row<NOUT>(a, tmem + (uint32_t)((j - js) * NOUT), warp, ((long)i * n1 + j) * n2 + k, live);
         }
     }
 
@@ -1082,49 +981,60 @@ cudaError_t wgrad_rows(const WgradArgs& a, int ng, cudaStream_t s) {
                       : wgrad_rows_inst<48, COUT>(a, s);
 }
 
-template <int CIN, int NOUT>
+template <int CG, int NOUT, int JS>
 cudaError_t rows_inst(const ConvArgs& a, cudaStream_t s) {
-    constexpr int NR = RowShape<CIN, NOUT, 4>::smem <= 200 * 1024 ? 4 : 3;
-    constexpr int smem = RowShape<CIN, NOUT, NR>::smem;
-    static_assert(smem <= 227 * 1024, "row kernel does not fit shared memory");
-    cudaError_t e = cudaFuncSetAttribute(k_conv_rows<CIN, NOUT, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem);
+    using F = RowShape<CG, NOUT, JS>;
+    RowPlan R;
+    R.stream = a.n2 % kTile != 0;
+    R.P = R.stream ? a.n2 + 1 : kTile + 2;
+    R.nvox = 2 * R.P + kTile + 2;
+    const int set = (CG / 8) * R.nvox * 16, fixed = 2 * F::WBYTES + F::BARS;
+    // as deep a ring as fits: two CTAs an SM where their accumulators do
+    const int room = (F::NCOLS == 256 ? 113 : 227) * 1024 - fixed;
+    R.nr = std::min(kRowRing, room / set);
+    if (R.nr < 2) R.nr = std::min(kRowRing, (227 * 1024 - fixed) / set);
+    if (R.nr < 1) return cudaErrorInvalidValue;
+    const int smem = R.nr * set + fixed;
+    cudaError_t e = cudaFuncSetAttribute(k_conv_rows<CG, NOUT, JS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)(a.n2 / kTile), (unsigned)a.n0, (unsigned)((a.n1 + kJSeg - 1) / kJSeg));
-    k_conv_rows<CIN, NOUT, NR><<<grid, kRowThreads, smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <int CG, int NOUT>
-cudaError_t groups_inst(const ConvArgs& a, cudaStream_t s) {
-    constexpr int NR = 4, smem = GroupShape<CG, NOUT, NR>::smem;
-    static_assert(smem <= 227 * 1024, "group kernel does not fit shared memory");
-    cudaError_t e = cudaFuncSetAttribute(k_conv_groups<CG, NOUT, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)(a.n2 / kTile), (unsigned)a.n0, (unsigned)((a.n1 + kGrpSeg - 1) / kGrpSeg));
-    k_conv_groups<CG, NOUT, NR><<<grid, kRowThreads, smem, s>>>(a);
+    const long tiles = R.stream ? ((long)a.n0 * R.P + kTile - 1) / kTile : (long)a.n0 * (a.n2 / kTile);
+    // rows a CTA: input rows walked (two more than it owns) times the CTAs an
+    // SM gets, at its least; the most rows where that is equal
+    long best = 0;
+    for (int t = std::min(JS, a.n1); t >= 1; --t) {
+        const long ctas = tiles * ((a.n1 + t - 1) / t), cost = (ctas + kSms - 1) / kSms * (t + 2);
+        if (!best || cost < best) {
+            best = cost;
+            R.rows = t;
+        }
+    }
+    k_conv_rows<CG, NOUT, JS>
+        <<<dim3((unsigned)tiles, (unsigned)((a.n1 + R.rows - 1) / R.rows)), kRowThreads, smem, s>>>(a, R);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-// the row-marching kernel covers these (input channels, output channels)
-// on grids with n2 % 128 == 0; other shapes use k_conv
+// The row-marching kernel covers 16 to 64 output channels from inputs in whole
+// blocks of 16: it was the faster one at every level of the network (figures at
+// the kernel).  Rows are whole 128-voxel segments or have at most 256 voxels:
+// a longer run would not leave room for the weights, nor the loader's registers;
+// those, and more than 256 input channels, use k_conv.
 bool rows_supported(int cin, int nout, int n2) {
-    if (n2 % 128) return false;
-    return (cin == 16 && (nout == 16 || nout == 32 || nout == 48)) || (cin == 32 && (nout == 16 || nout == 32)) ||
-           (cin == 48 && nout == 16) || (cin == 96 && nout == 32);
+    return cin % 16 == 0 && cin <= 256 && (nout == 16 || nout == 32 || nout == 48 || nout == 64) &&
+           (n2 % kTile == 0 || n2 <= 256);
 }
 
+// Rows a CTA: 16 of 16 output channels (256 columns of tensor memory, two CTAs
+// an SM), 16 of 32, 10 of 48 and 8 of 64 (all of it).  Groups of 32 input
+// channels where both weight buffers leave room for a ring.
 cudaError_t rows_launch(const ConvArgs& a, int nout, cudaStream_t s) {
     const int cin = a.in.c0 + a.in.c1;
-    if (cin == 16 && nout == 16) return rows_inst<16, 16>(a, s);
-    if (cin == 16 && nout == 32) return rows_inst<16, 32>(a, s);
-    if (cin == 16 && nout == 48) return rows_inst<16, 48>(a, s);
-    if (cin == 32 && nout == 16) return rows_inst<32, 16>(a, s);
-    if (cin == 32 && nout == 32) return rows_inst<32, 32>(a, s);
-    if (cin == 48 && nout == 16) return rows_inst<48, 16>(a, s);
-    if (cin == 96 && nout == 32) return groups_inst<32, 32>(a, s);
+    if (nout == 16) return rows_inst<16, 16, 16>(a, s);
+    if (nout == 32) return cin % 32 || (a.n2 % kTile && a.n2 > kTile) ? rows_inst<16, 32, 16>(a, s)
+                                                                     : rows_inst<32, 32, 16>(a, s);
+    if (nout == 48) return rows_inst<16, 48, 10>(a, s);
+    if (nout == 64) return rows_inst<16, 64, 8>(a, s);
     return cudaErrorInvalidValue;
 }
 
@@ -1143,8 +1053,11 @@ bool wgrad_supported(int cout) { return cout == 16 || cout == 32 || cout == 64; 
     if (kc == KC && nout == N) return conv_inst<KC, N>(a, s);
 
 cudaError_t conv_launch(const ConvArgs& a, int kc, int nout, cudaStream_t s) {
-    // rows of 128 voxels with 16-channel weight blocks: the row-marching kernel
-    if (kc == 16 && rows_supported(a.in.c0 + a.in.c1, nout, a.n2)) return rows_launch(a, nout, s);
+    // 16-channel weight blocks: the row-marching kernel
+    // (it counts voxels in 32 bits and column segments in 16)
+    if (kc == 16 && a.in.c0 % 16 == 0 && a.in.c1 % 16 == 0 && rows_supported(a.in.c0 + a.in.c1, nout, a.n2) &&
+        (a.n0 + 1L) * a.n1 * (a.n2 + 1L) < 1L << 31 && a.n1 <= 65535)
+        return rows_launch(a, nout, s);
     BUN_CONV_CASE(16, 16)
     BUN_CONV_CASE(16, 32)
     BUN_CONV_CASE(16, 48)
