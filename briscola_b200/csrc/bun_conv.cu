@@ -21,9 +21,9 @@
 // gradient.  K is split over grid.y; each split writes FP32 partial sums
 // that a CUDA-core kernel adds in a fixed order.
 //
-// Weight gradients of 16 and 32 output channels on rows of whole 16-voxel
-// groups march along j instead (k_wgrad_rows, below): each row is loaded once
-// for the taps that need it.
+// Convolutions of 16 to 64 output channels march along j instead (k_conv_rows,
+// below), and weight gradients on rows of whole 16-voxel groups take blocks of
+// rows (k_wgrad_rows): a row is loaded once for the taps that need it.
 //
 // Shared-memory operand layouts are the canonical no-swizzle (interleaved)
 // ones of the tcgen05 matrix descriptors: a core matrix is 8 rows of 16
@@ -445,63 +445,67 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(WgradArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// weight gradient marching along j (16 or 32 output channels, n2 % 16 == 0)
+// weight gradient by blocks of rows (n2 % 16 == 0, channels in blocks of 16)
 // ---------------------------------------------------------------------------
 // k_wgrad gathers the 128 voxels of a K block once for every (tap, channel)
 // row tile, 27 times over, and its loads bound it (48 -> 16 channels at 128^3:
-// 1.94 ms, tensor pipe idle).  Here a CTA owns one plane offset di and a group
-// of NG input channels and walks row segments (plane i, 128 voxels along k, up
-// to 32 rows j).  One step takes the input row jj of plane i + di and the
-// three rows j = jj-1, jj, jj+1 of the output gradient that meet it:
-//   M = (output-gradient row, output channel), N = input channel, K = voxels,
-// one MMA chain per tap offset dk -- a shift of the input row's start address,
-// as in k_conv_rows -- so a row is loaded once and 24 MMAs of K = 16 use it.
-// The three rows are neighbours in a ring of R rows whose first two are kept
-// twice, behind its end, so that any three in turn are one matrix; M is padded
-// to 128 by whatever follows them, whose products nobody reads.  Rows outside
-// the segment or the grid are zero.  Both operands are MN-major: chunks of 8
+// 1.94 ms, tensor pipe idle).  Here a CTA owns one plane offset di and 16 input
+// channels and takes blocks of W = 128 / COUT rows j of the output gradient
+// (plane i, 128 voxels along k) with the W + 2 input rows of plane i + di that
+// meet them:
+//   M = (output-gradient row, output channel), N = (input row, input channel),
+//   K = voxels,
+// one MMA chain per tap offset dk -- a shift of the input rows' start address,
+// as in k_conv_rows.  M is full (an MMA costs its 128 rows' operand, whatever
+// they hold); of the products those of rows j and j-1 .. j+1 are wanted, the
+// diagonal blocks, which is 3 W of W (W + 2).  One input row against the three
+// rows that meet it filled 48 of the 128 rows of M for 16 channels and was bound
+// by the tensor pipe (68 - 90 %): five times as many MMA cycles a row.
+// Rows outside the grid are zero.  Both operands are MN-major: chunks of 8
 // channels x voxels of 16 bytes.
-// D: lane = (row, output channel), column = (dk, input channel); it is added
-// up over every segment of the split and written once, as k_wgrad's partials.
-// Measured at 128^3, us: 48 -> 16 channels 1936 -> 663, 16 -> 16 735 -> 250;
-// at 64^3: 96 -> 32 802 -> 210, 32 -> 32 286 -> 78, 16 -> 32 160 -> 72.
-constexpr int kWgVox = 128;                      // voxels of a segment row
+// D: lane = (row, output channel), column = (dk, input row, input channel),
+// added up over all blocks of the split.  At the end the W diagonals are added
+// in order by way of shared memory and written once, as k_wgrad's partials.
+// Measured, us, k_wgrad / one input row at a time / now: at 128^3 48 -> 16
+// channels 1936 / 663 / 292, 16 -> 16 735 / 250 / 119; at 64^3 96 -> 32
+// 802 / 210 / 162, 32 -> 32 286 / 78 / 61, 16 -> 32 160 / 72 / 40; k_wgrad / now:
+// at 32^3 128 -> 64 150 / 74, 64 -> 64 90 / 42; at 16^3 64 -> 64 27 / 17.  Bound
+// by the blocks' supply from L2 at the larger sizes (74 KB against 24 MMAs).
+constexpr int kWgVox = 128;                      // voxels of a block's rows
 constexpr int kWgInChunk = (kWgVox + 2) * 16;    // bytes of 8 input channels of a row (k0-1 .. k0+128)
 constexpr int kWgDzChunk = kWgVox * 16;          // bytes of 8 output channels of a row
-constexpr int kWgSeg = 32;                       // rows of a segment
 
-template <int NG, int COUT>
+template <int COUT>
 struct WgRowShape {
-    static constexpr int R = NG * COUT > 1024 ? 4 : 5;  // rows of the rings (two CTAs an SM)
-    static constexpr int DZROW = (COUT / 8) * kWgDzChunk;
-    static constexpr int INROW = (NG / 8) * kWgInChunk;
-    // the last window starts at row R - 1 and reads 128 / COUT rows: past the
-    // ring's R + 2 rows it reads the input rows behind them
-    static constexpr int DZ = (R + 2) * DZROW;
-    static constexpr int OVER = (R - 1 + 128 / COUT) * DZROW - DZ;
-    static constexpr int IN = R * INROW > OVER ? R * INROW : OVER;
-    static constexpr uint32_t NCOLS = 3 * NG <= 64 ? 64 : 3 * NG <= 128 ? 128 : 256;
-    static constexpr int smem = DZ + IN + (2 * R + 1) * 8 + 16;
+    static constexpr int W = 128 / COUT;                    // rows of a block
+    static constexpr int N = (W + 2) * 16;
+    static constexpr int DZ = W * (COUT / 8) * kWgDzChunk;
+    static constexpr int STAGE = DZ + (W + 2) * 2 * kWgInChunk;
+    // three stages and one CTA an SM; 64 channels: two and two
+    static constexpr int S = COUT == 64 ? 2 : 3;
+    static constexpr uint32_t NCOLS = 3 * N <= 256 ? 256 : 512;
+    static constexpr int smem = S * STAGE + (2 * S + 1) * 8 + 16;
+    static_assert(W * 9 * 16 * COUT * 4 <= S * STAGE, "the diagonals take the stages' place");
 };
 
-template <int NG, int COUT>
+template <int COUT>
 __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
-    using F = WgRowShape<NG, COUT>;
-    constexpr int R = F::R;
+    using F = WgRowShape<COUT>;
+    constexpr int S = F::S, W = F::W, N = F::N;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + F::DZ + F::IN);
-    uint64_t* empty = full + R;
-    uint64_t* accb = empty + R;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * F::STAGE);
+    uint64_t* empty = full + S;
+    uint64_t* accb = empty + S;
     uint32_t* slot = reinterpret_cast<uint32_t*>(accb + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5;
     const int n0 = a.n0, n1 = a.n1, n2 = a.n2;
-    const int split = blockIdx.x, di = blockIdx.y, cb = blockIdx.z * NG;
-    const int nks = (n2 + kWgVox - 1) / kWgVox, njs = (n1 + kWgSeg - 1) / kWgSeg;
+    const int split = blockIdx.x, di = blockIdx.y, cb = blockIdx.z * 16;
+    const int nks = (n2 + kWgVox - 1) / kWgVox, njs = (n1 + W - 1) / W;
     const int units = n0 * nks * njs;
 
     if (tid == 0) {
-        for (int r = 0; r < R; ++r) {
+        for (int r = 0; r < S; ++r) {
             mbar_init(&full[r], kProducers);
             mbar_init(&empty[r], 1);
         }
@@ -516,117 +520,146 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
     const uint32_t base = smem_u32(smem);
     bool ok = true, any = false;
 
-    // a unit's plane, first voxel and row, rows and voxels; false where the
-    // input plane lies outside the grid
-    auto unit = [&](int un, int& i, int& k0, int& js, int& nr, int& kv) {
+    // a block's plane, first voxel and row, and voxels; false where the input
+    // plane lies outside the grid
+    auto unit = [&](int un, int& i, int& k0, int& js, int& kv) {
         const int ks = un % nks, q = un / nks;
         k0 = ks * kWgVox;
         kv = min(kWgVox, n2 - k0);
-        js = (q % njs) * kWgSeg;
-        nr = min(kWgSeg, n1 - js);
+        js = (q % njs) * W;
         i = q / njs;
         const int ii = i + di - 1;
         return ii >= 0 && ii < n0;
     };
 
     if (warp < 4) {
-        // ---- loader: entry v = 0 .. nr+3 of a unit is output-gradient row
-        // q = v - 2 (zero outside 0 .. nr-1) and, from v = 2 on, the input row
-        // of step u = v - 2, row js - 1 + u
+        // ---- loader; the sources of the two chunks of channels
+        const bf16* src[2];
+        int cs[2], up[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int ch = cb + h * 8;
+            const bool first = ch < a.in.c0;
+            src[h] = first ? a.in.src0 + ch : a.in.src1 + (ch - a.in.c0);
+            cs[h] = first ? a.in.c0 : a.in.c1;
+            up[h] = first ? a.in.up0 : 0;
+        }
         int e = 0;
         for (int un = split; ok && un < units; un += a.nsplit) {
-            int i, k0, js, nr, kv;
-            if (!unit(un, i, k0, js, nr, kv)) continue;
-            const int ii = i + di - 1;
-            for (int v = 0; v < nr + 4; ++v, ++e) {
-                const int r = e % R;
-                if (!mbar_wait(&empty[r], ((uint32_t)(e / R) & 1) ^ 1)) {
-                    ok = false;
-                    break;
-                }
-                const int q = v - 2;
-                {
-                    const bool valid = q >= 0 && q < nr && tid < kv;
-                    const bf16* src = valid ? a.dz + (((long)i * n1 + js + q) * n2 + k0 + tid) * COUT : a.dz;
-                    const uint32_t d = base + r * F::DZROW + tid * 16;
-#pragma unroll
-                    for (int h = 0; h < COUT / 8; ++h) {
-                        cp16(d + h * kWgDzChunk, src + (valid ? h * 8 : 0), valid);
-                        if (r < 2) cp16(d + R * F::DZROW + h * kWgDzChunk, src + (valid ? h * 8 : 0), valid);
-                    }
-                }
-                if (v >= 2) {
-                    const int jj = js - 1 + q;
-                    for (int kk = tid; kk < kv + 2; kk += kProducers) {
-                        const int k = k0 - 1 + kk;
-                        const bool valid = jj >= 0 && jj < n1 && k >= 0 && k < n2;
-                        const uint32_t d = base + F::DZ + r * F::INROW + kk * 16;
-#pragma unroll
-                        for (int h = 0; h < NG / 8; ++h)
-                            cp16(d + h * kWgInChunk, valid ? in_ptr(a.in, n1, n2, ii, jj, k, cb + h * 8) : a.dz, valid);
-                    }
-                }
-                cp_arrive(&full[r]);
+            int i, k0, js, kv;
+            if (!unit(un, i, k0, js, kv)) continue;
+            const int ii = i + di - 1, r = e % S;
+            if (!mbar_wait(&empty[r], ((uint32_t)(e / S) & 1) ^ 1)) {
+                ok = false;
+                break;
             }
+            ++e;
+            const uint32_t st = base + r * F::STAGE;
+            // 2^lg voxels by 128 / 2^lg rows at once
+            const int lg = kv > 64 ? 7 : kv > 32 ? 6 : kv > 16 ? 5 : 4;
+            const int v = tid & ((1 << lg) - 1), w0 = tid >> lg, ws = kProducers >> lg;
+            if (v < kv) {
+                const bf16* dp = a.dz + (((long)i * n1 + js) * n2 + k0 + v) * COUT;
+                const uint32_t d0 = st + v * 16, i0 = st + F::DZ + (v + 1) * 16;
+                const bf16* p[2];
+                for (int h = 0; h < 2; ++h)
+                    p[h] = src[h] + ((long)(ii >> up[h]) * (n1 >> up[h]) * (n2 >> up[h]) + ((k0 + v) >> up[h])) * cs[h];
+#pragma unroll 2
+                for (int w = w0; w < W; w += ws) {
+                    const bool valid = js + w < n1;
+#pragma unroll
+                    for (int h = 0; h < COUT / 8; ++h)
+                        cp16(d0 + (w * (COUT / 8) + h) * kWgDzChunk, valid ? dp + (long)w * n2 * COUT + h * 8 : a.dz, valid);
+                }
+#pragma unroll 2
+                for (int w = w0; w < W + 2; w += ws) {
+                    const int jj = js - 1 + w;
+                    const bool valid = jj >= 0 && jj < n1;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        cp16(i0 + (w * 2 + h) * kWgInChunk,
+                             valid ? p[h] + (long)((jj >> up[h]) * (n2 >> up[h])) * cs[h] : a.dz, valid);
+                }
+            }
+            // the voxels before and behind the rows
+            if (tid < 2 * (W + 2)) {
+                const int w = tid >> 1, jj = js - 1 + w, k = tid & 1 ? k0 + kv : k0 - 1;
+                const bool valid = jj >= 0 && jj < n1 && k >= 0 && k < n2;
+                const uint32_t d = st + F::DZ + w * 2 * kWgInChunk + (tid & 1 ? kv + 1 : 0) * 16;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    cp16(d + h * kWgInChunk, valid ? in_ptr(a.in, n1, n2, ii, jj, k, cb + h * 8) : a.dz, valid);
+            }
+            cp_arrive(&full[r]);
         }
     } else if (tid == kProducers) {
-        // ---- MMA issue: per step and dk, kv / 16 MMAs of 128 x NG x 16
-        constexpr uint32_t idesc = idesc_bf16(128, NG, true, true);
+        // ---- MMA issue: per block and dk, kv / 16 MMAs of 128 x N x 16
+        constexpr uint32_t idesc = idesc_bf16(128, N, true, true);
         int e = 0;
         for (int un = split; ok && un < units; un += a.nsplit) {
-            int i, k0, js, nr, kv;
-            if (!unit(un, i, k0, js, nr, kv)) continue;
-            for (int u = 0; ok && u < nr + 2; ++u) {
-                for (int v = u == 0 ? 0 : u + 2; v <= u + 2; ++v)
-                    if (!mbar_wait(&full[(e + v) % R], (uint32_t)((e + v) / R) & 1)) ok = false;
-                if (!ok) break;
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                tc_after();
-                const uint32_t as = base + (uint32_t)((e + u) % R) * F::DZROW;
-                const uint32_t bs = base + F::DZ + (uint32_t)((e + u + 2) % R) * F::INROW;
-#pragma unroll 1
-                for (int dk = 0; dk < 3; ++dk)
-#pragma unroll 1
-                    for (int q = 0; q < kv / 16; ++q)
-                        umma(tmem + dk * NG, sdesc(as + q * 256, 128, kWgDzChunk),
-                             sdesc(bs + dk * 16 + q * 256, 128, kWgInChunk), idesc, any || q != 0);
-                any = true;
-                umma_commit(&empty[(e + u) % R]);  // entry u of the unit is not needed again
+            int i, k0, js, kv;
+            if (!unit(un, i, k0, js, kv)) continue;
+            if (!mbar_wait(&full[e % S], (uint32_t)(e / S) & 1)) {
+                ok = false;
+                break;
             }
-            // nor are the last two
-            if (ok) {
-                umma_commit(&empty[(e + nr + 2) % R]);
-                umma_commit(&empty[(e + nr + 3) % R]);
-            }
-            e += nr + 4;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            tc_after();
+            const uint32_t as = base + (uint32_t)(e % S) * F::STAGE, bs = as + F::DZ;
+#pragma unroll 1
+            for (int dk = 0; dk < 3; ++dk)
+#pragma unroll 1
+                for (int q = 0; q < kv / 16; ++q)
+                    umma(tmem + dk * N, sdesc(as + q * 256, 128, kWgDzChunk),
+                         sdesc(bs + dk * 16 + q * 256, 128, kWgInChunk), idesc, any || q != 0);
+            any = true;
+            umma_commit(&empty[e % S]);
+            ++e;
         }
         umma_commit(accb);
     }
 
     if (warp < 4) {
         for (int un = split; !any && un < units; un += a.nsplit) {
-            int i, k0, js, nr, kv;
-            any = unit(un, i, k0, js, nr, kv);
+            int i, k0, js, kv;
+            any = unit(un, i, k0, js, kv);
         }
         bool done = mbar_wait(accb, 0);
         done = __all_sync(0xffffffffu, done);
         tc_after();
         if (!done) ok = false;
-        if (done) {
-            // lane = (ring row r, output channel n): row r met input row jj
-            // with dj = 2 - r
-            const int r = tid / COUT, n = tid % COUT;
-            const int C = a.in.c0 + a.in.c1;
+        // lane = (row r, output channel n) met input row r + dj: every stage has
+        // been read, the diagonals go where they were
+        float* red = reinterpret_cast<float*>(smem);
+        const int r = tid / COUT, n = tid % COUT, r0 = warp * 32 / COUT;
+        constexpr int T = COUT < 32 ? 4 : 3;  // input rows that meet a row of the warp
+        if (done && any) {
 #pragma unroll 1
-            for (int c0 = 0; c0 < 3 * NG; c0 += 16) {
-                float acc[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
-                if (r >= 3) continue;
-                const int dk = c0 / NG, c = cb + c0 % NG;
-                const int row = (di * 9 + (2 - r) * 3 + dk) * C + c;
-                float* dst = a.part + ((long)split * a.rows_pad + row) * COUT + n;
+            for (int dk = 0; dk < 3; ++dk)
+#pragma unroll 1
+                for (int t = 0; t < T; ++t) {
+                    float acc[16];
+                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dk * N + (r0 + t) * 16), acc);
+                    const int dj = r0 + t - r;
+                    if (dj >= 0 && dj < 3) {
+                        float* dst = red + ((r * 9 + dj * 3 + dk) * 16) * COUT + n;
 #pragma unroll
-                for (int q = 0; q < 16; ++q) dst[q * COUT] = any ? acc[q] : 0.f;
+                        for (int q = 0; q < 16; ++q) dst[q * COUT] = acc[q];
+                    }
+                    __syncwarp();
+                }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const int C = a.in.c0 + a.in.c1;
+        if (done) {
+            for (int x = tid; x < 9 * 16 * COUT; x += kProducers) {
+                float sum = 0.f;
+                if (any) {
+#pragma unroll
+                    for (int w = 0; w < W; ++w) sum += red[w * 9 * 16 * COUT + x];
+                }
+                const int c = x / COUT % 16, tap = x / (16 * COUT);
+                a.part[((long)split * a.rows_pad + (di * 9 + tap) * C + cb + c) * COUT + x % COUT] = sum;
             }
         }
     }
@@ -953,32 +986,13 @@ cudaError_t wgrad_inst(const WgradArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int NG, int COUT>
-cudaError_t wgrad_rows_inst(const WgradArgs& a, cudaStream_t s) {
-    constexpr int smem = WgRowShape<NG, COUT>::smem;
-    static_assert(smem <= 113 * 1024, "two CTAs an SM");
-    cudaError_t e = cudaFuncSetAttribute(k_wgrad_rows<NG, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    k_wgrad_rows<NG, COUT><<<dim3((unsigned)a.nsplit, 3, (unsigned)((a.in.c0 + a.in.c1) / NG)), kThreads, smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-// input channels of a group: all of them up to 48 (three taps' columns then
-// leave room for two CTAs' accumulators an SM), else halves; 0: not covered
-int wgrad_group(int cin) {
-    switch (cin) {
-        case 16: case 32: case 48: return cin;
-        case 64: return 32;
-        case 96: return 48;
-        default: return 0;
-    }
-}
-
 template <int COUT>
-cudaError_t wgrad_rows(const WgradArgs& a, int ng, cudaStream_t s) {
-    return ng == 16 ? wgrad_rows_inst<16, COUT>(a, s)
-           : ng == 32 ? wgrad_rows_inst<32, COUT>(a, s)
-                      : wgrad_rows_inst<48, COUT>(a, s);
+cudaError_t wgrad_rows(const WgradArgs& a, cudaStream_t s) {
+    constexpr int smem = WgRowShape<COUT>::smem;
+    cudaError_t e = cudaFuncSetAttribute(k_wgrad_rows<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_wgrad_rows<COUT><<<dim3((unsigned)a.nsplit, 3, (unsigned)((a.in.c0 + a.in.c1) / 16)), kThreads, smem, s>>>(a);
+    return cudaGetLastError();
 }
 
 template <int CG, int NOUT, int JS>
@@ -1074,10 +1088,14 @@ cudaError_t conv_launch(const ConvArgs& a, int kc, int nout, cudaStream_t s) {
 #undef BUN_CONV_CASE
 
 cudaError_t wgrad_launch(const WgradArgs& a, int cout, cudaStream_t s) {
-    // rows of whole 16-voxel groups and channels in whole chunks of 16
-    const int ng = wgrad_group(a.in.c0 + a.in.c1);
-    if (ng && a.n2 % 16 == 0 && a.in.c0 % 8 == 0 && (cout == 16 || cout == 32))
-        return cout == 16 ? wgrad_rows<16>(a, ng, s) : wgrad_rows<32>(a, ng, s);
+    // rows in whole steps of 16 voxels (an MMA's K) and channels in whole blocks
+    // of 16; a row's 8 channels must come from one source
+    const int cin = a.in.c0 + a.in.c1;
+    if (a.n2 % 16 == 0 && cin % 16 == 0 && a.in.c0 % 8 == 0) {
+        if (cout == 16) return wgrad_rows<16>(a, s);
+        if (cout == 32) return wgrad_rows<32>(a, s);
+        if (cout == 64) return wgrad_rows<64>(a, s);
+    }
     if (cout == 16) return wgrad_inst<16>(a, s);
     if (cout == 32) return wgrad_inst<32>(a, s);
     if (cout == 64) return wgrad_inst<64>(a, s);

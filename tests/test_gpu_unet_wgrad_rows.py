@@ -1,10 +1,11 @@
-"""The row-marching weight gradient (k_wgrad_rows) at the edges of its ranges,
-against the FP64 reference: rows of 16 voxels, of a partial and of two
-128-voxel segments, columns of one row, of a whole and of a broken 32-row
-segment, one plane (two of the three plane offsets fall outside), every channel
-group, upsampled and concatenated inputs, one split and more splits than
-segments.  BF16 inputs are exact in the reference, so the error is that of the
-FP32 accumulation: 1e-4, as in test_gpu_unet."""
+"""The weight gradient by blocks of rows (k_wgrad_rows) at the edges of its
+ranges, against the FP64 reference: rows of 16 voxels, of a partial and of two
+128-voxel segments, columns of one row, of whole and of broken blocks (8, 4 and
+2 rows for 16, 32 and 64 output channels), one plane (two of the three plane
+offsets fall outside), one to eight blocks of 16 input channels, upsampled and
+concatenated inputs, one split and more splits than blocks.  BF16 inputs are
+exact in the reference, so the error is that of the FP32 accumulation: 1e-4, as
+in test_gpu_unet."""
 import ctypes
 
 import numpy as np
@@ -25,8 +26,13 @@ CASES = [
     ((2, 3, 144), 48, 0, 0, 16, 2),
     ((2, 2, 256), 16, 0, 0, 16, 9),
     ((4, 6, 32), 32, 1, 16, 16, 3),    # decoder: upsampled + skip, 48 channels
-    ((4, 70, 64), 64, 1, 32, 32, 5),   # 96 channels in two groups
+    ((4, 70, 64), 64, 1, 32, 32, 5),   # 96 channels
     ((2, 5, 16), 64, 0, 0, 32, 4),
+    ((2, 9, 16), 16, 0, 0, 16, 3),
+    ((1, 1, 16), 16, 0, 0, 64, 1),
+    ((2, 5, 32), 48, 0, 0, 64, 2),
+    ((4, 6, 32), 64, 1, 64, 64, 3),
+    ((3, 7, 144), 80, 0, 0, 32, 2),
 ]
 
 
