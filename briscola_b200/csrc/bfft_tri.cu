@@ -10,9 +10,10 @@
 // is cut into chunks of C rows, one thread each, held in registers: the chunk
 // from a zero start and its product, a scan over the line's chunks for the
 // value entering each (in shared memory, log2 steps), and the chunk again from
-// that value.  The serial chain is 2 C rows and the scan instead of n, the field is read and written once, and a thread has all its
-// 2 C loads in flight: 115 us there (139 with chunks of 16 rows, which also
-// kept every row's product), 93 -> 12 us for 128 x 96 x 64 cells.
+// that value.  The serial chain is 2 C rows and the scan instead of n, the field
+// is read and written once, and a thread has all its 2 C loads in flight: 115 us
+// there (139 with chunks of 16 rows, which also kept every row's product),
+// 93 -> 12 us for 128 x 96 x 64 cells.
 //
 // Bound: memory (16 B a cell of the field and 8 B of each factor).
 

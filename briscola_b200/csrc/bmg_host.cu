@@ -141,7 +141,7 @@ struct bmg_ctx {
     std::vector<HostLevel> lv;
     std::vector<std::vector<BrickTransfer>> tr;  // [level][brick]
     int lc = 0;  // coarse solve level
-    int tail = -1;  // first level of the single-CTA coarse cycle, -1: none
+    int tail = -1;  // first level of the cycle's end in the cluster, -1: none
     double* ainv = nullptr;
     int* cidx = nullptr;
     int ncoarse = 0;
@@ -1099,7 +1099,7 @@ void build(bmg_ctx* c, HostLevel&& L0) {
         layout(L);
         if (L.cells >= (1L << 31)) throw BadArg{BMG_UNSUPPORTED, "a level above 2^31 cells"};
         // parity-split rows on the single-brick levels the per-pass kernels
-        // run (above the single-CTA coarse end's size) whose rows are whole
+        // run (above the coarse end's size) whose rows are whole
         // 16-cell blocks
         L.ks = c->opt.row_layout == BMG_ROWS_SPLIT && !c->multi && L.br[0].n[2] % 16 == 0 &&
                L.ncell > kSplitMinCells;

@@ -285,7 +285,7 @@ void launch_prolong_correct(const Bricks<T>& F, const Bricks<T>& C, const Transf
 // dense solve on the coarse level; cidx lists the slab index of each unknown
 template <typename T>
 void launch_coarse_solve(const Bricks<T>& C, const double* ainv, const int* cidx, int n, cudaStream_t s);
-// the coarse end of a cycle in one CTA (bmg_tail.cu)
+// the coarse end of a cycle in one cluster (bmg_tail.cu)
 template <typename T, bool VAR>
 void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s);
 // the whole FP64 loop of a solve whose level 0 is the first level there

@@ -184,9 +184,9 @@ __device__ __forceinline__ void stq<double>(double* p, int kh, const double v[4]
 // The rows j-1, j, j+1, the i neighbours, b and the k couplings are read as
 // whole vectors, and the quad is written back as one vector (the other
 // colour's values are unchanged during the pass, so writing them back is
-// safe; a quad is never a ghost).  colour_quad_item is shared with the
-// single-CTA coarse cycle (k_tail_cycle).  The arithmetic is gs_value's, so results are
-// bit-identical to k_colour_pass and the fused smoother.  Needs every
+// safe; a quad is never a ghost).  The arithmetic is gs_value's, so results are
+// bit-identical to k_colour_pass, the cluster's passes (k_tail_cycle) and the
+// fused smoother.  Needs every
 // brick's n2 % 4 == 0 and natural rows (parity-split levels take
 // k_colour_split).
 // ---------------------------------------------------------------------------

@@ -19,7 +19,8 @@
 //
 // Measured (solves, one B200; before: one 512-thread CTA passing over levels
 // of at most 4096 cells in L2, V cycles only): 16^3 cavity FP64 724 -> 404 us,
-// 64^3 cavity FP64 1430 -> 956 us, 96 x 192 x 24 F cycles FP64 5300 -> 2787 us.
+// 64^3 cavity FP64 1430 -> 900 us, 96 x 192 x 24 F cycles FP64 5300 -> 2670 us
+// (with the whole loop in the kernel, where level 0 fits: 16^3 313 us).
 // A pass of an 8^3 level takes about 700 cycles on CTA 0, one of 32^3 over
 // 16 CTAs 2000, half of it the barrier and the halo stores it waits for; a
 // launch per pass costs 5000.

@@ -145,9 +145,9 @@ typedef struct bmg_options {
     int criterion;      /* criterion (initial): BMG_CRITERION_*                */
     int fused_chunk;    /* fusedChunk (64): planes along i per CTA of the
                            fused smoother when autotune is off (1..128)        */
-    int fuse_coarse;    /* fuseCoarse (1): run the levels of at most 4096
-                           cells and the coarse solve of a single-brick V
-                           cycle in one kernel                                 */
+    int fuse_coarse;    /* fuseCoarse (1): run the levels that fit the shared
+                           memory of a thread-block cluster and the coarse
+                           solve of a single-brick V or F cycle in one kernel  */
     int coarse_mode;    /* coarseMode (direct): BMG_COARSE_* (MG.C:110-126)     */
     int restrict_scheme;/* restrict (linear): BMG_RESTRICT_*                   */
     int prolong_scheme; /* prolong (linear): BMG_PROLONG_*                     */
