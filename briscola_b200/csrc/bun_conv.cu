@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 // level's size, us before / now; two thirds of the time is the rows' supply and
 // the hand-over between the warps, not the MMAs):
 //   256^3  16 -> 16   663 /  592     48 -> 16   3359 / 1336
-//   128^3  96 -> 32  2869 /  442     (16 -> 32: 145, 32 -> 32: 196)
+//   128^3  96 -> 32  2869 /  442     32 -> 32   360 /  196    (16 -> 32: 145)
 //    64^3  32 -> 64   119 /   47     64 -> 64    319 /   78   128 -> 64  589 / 139
 //    32^3  64 -> 64    50 /   21;  16^3 64 -> 64   30 /   17
 constexpr int kRowThreads = 288;
@@ -720,7 +720,10 @@ struct RowPlan {
     int nvox;    // positions of the run: 2 P + 130
     int nr;      // rows of the ring
     int rows;    // rows j a CTA, at most JS
+    int lk;      // log2 of the 8-channel chunks of a packed weight block
+    int ntot;    // output channels, NOUT of them a CTA (blockIdx.y)
     int stream;  // rows one behind another
+    int tiles;   // of 128 positions; CTA = segment * tiles + tile
 };
 
 template <int CG, int NOUT, int JS>
@@ -733,17 +736,18 @@ struct RowShape {
     static_assert(JS * NOUT <= 512 && 3 * NOUT <= 256, "tensor memory");
 };
 
-// the plane and voxel of a position of the run (q = 0: one row and one voxel
-// before the CTA's first position); false outside the grid
-__device__ __forceinline__ bool row_voxel(const ConvArgs& a, const RowPlan& R, int q, int& i, int& k) {
+// the plane and voxel of a position of tile's run (q = 0: one row and one voxel
+// before its first position); false outside the grid
+__device__ __forceinline__ bool row_voxel(const ConvArgs& a, const RowPlan& R, int tile, int q, int& i, int& k) {
     if (R.stream) {
-        const int g = (int)blockIdx.x * kTile - 1 + q;  // counted from the plane before the first
-        i = g < 0 ? -1 : g / R.P - 1;
-        k = g - (i + 1) * R.P;
+        // counted from the voxel before the plane before the first
+        const unsigned g = (unsigned)tile * kTile + (unsigned)q, r = g ? (g - 1) / (unsigned)R.P : 0;
+        i = g ? (int)r - 1 : -1;
+        k = (int)(g - 1 - r * (unsigned)R.P);
     } else {
         const int nk = a.n2 / kTile, di = q / R.P;
-        i = (int)blockIdx.x / nk + di - 1;
-        k = ((int)blockIdx.x % nk) * kTile - 1 + (q - di * R.P);
+        i = tile / nk + di - 1;
+        k = (tile % nk) * kTile - 1 + (q - di * R.P);
     }
     return i >= 0 && i < a.n0 && k >= 0 && k < a.n2;
 }
@@ -751,7 +755,8 @@ __device__ __forceinline__ bool row_voxel(const ConvArgs& a, const RowPlan& R, i
 // a row's accumulator (NOUT columns from col, this warp's lanes) to voxel v, if
 // the position is one
 template <int NOUT>
-__device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int warp, long v, bool live) {
+__device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int warp, long v, bool live, int ntot,
+                                          int n0) {
 #pragma unroll 1
     for (int c0 = 0; c0 < NOUT; c0 += 16) {
         float accv[16];
@@ -759,14 +764,14 @@ __device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int w
         if (!live) continue;
         if (a.bias) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) accv[q] += a.bias[c0 + q];
+            for (int q = 0; q < 16; ++q) accv[q] += a.bias[n0 + c0 + q];
         }
         if (a.relu) {
 #pragma unroll
             for (int q = 0; q < 16; ++q) accv[q] = fmaxf(accv[q], 0.f);
         }
         if (a.mask) {
-            const uint4* mp = reinterpret_cast<const uint4*>(a.mask + v * NOUT + c0);
+            const uint4* mp = reinterpret_cast<const uint4*>(a.mask + v * ntot + n0 + c0);
             uint4 mv[2] = {mp[0], mp[1]};
             const bf16* m = reinterpret_cast<const bf16*>(mv);
 #pragma unroll
@@ -777,7 +782,7 @@ __device__ __forceinline__ void store_row(const ConvArgs& a, uint32_t col, int w
         __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(ov);
 #pragma unroll
         for (int q = 0; q < 8; ++q) o[q] = __floats2bfloat162_rn(accv[2 * q], accv[2 * q + 1]);
-        uint4* op = reinterpret_cast<uint4*>(a.out + v * NOUT + c0);
+        uint4* op = reinterpret_cast<uint4*>(a.out + v * ntot + n0 + c0);
         op[0] = ov[0];
         op[1] = ov[1];
     }
@@ -791,8 +796,10 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
         : "memory");
 }
 
+// (two CTAs of nine warps put five on one scheduler: at most 96 registers, the
+// bound for ten warps each; at 108 the second CTA stayed out, 840 -> 1445 us)
 template <int CG, int NOUT, int JS>
-__global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a, RowPlan R) {
+__global__ void __launch_bounds__(kRowThreads + 32, NOUT == 16 ? 2 : 1) k_conv_rows(ConvArgs a, RowPlan R) {
     using F = RowShape<CG, NOUT, JS>;
     constexpr int NQ = CG / 16;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -808,7 +815,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a, RowPla
 
     const int tid = threadIdx.x, warp = tid >> 5;
     const int n1 = a.n1, n2 = a.n2;
-    const int js = blockIdx.y * R.rows, je = min(js + R.rows, n1);
+    const int seg = (int)blockIdx.x / R.tiles, tile = (int)blockIdx.x - seg * R.tiles;
+    const int js = seg * R.rows, je = min(js + R.rows, n1);
     // input rows inside the grid (those outside are zero)
     const int jlo = max(js - 1, 0), jhi = min(je, n1 - 1);
     const int nqt = (a.in.c0 + a.in.c1) / 16, groups = nqt / NQ;
@@ -853,7 +861,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a, RowPla
 #pragma unroll
         for (int m = 0; m < M; ++m) {
             int i, k;
-            const bool valid = row_voxel(a, R, q0 + m * QS, i, k);
+            const bool valid = row_voxel(a, R, tile, q0 + m * QS, i, k);
             v0[m] = valid ? (i >> up) * (n1 >> up) * (n2 >> up) + (k >> up) : -1;
             v1[m] = valid ? i * n1 * n2 + k : -1;
         }
@@ -863,13 +871,18 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a, RowPla
                 ok = false;
                 break;
             }
-            // packed blocks (tap, 16 channels) to ((di, dk), u, dj = 2, 1, 0)
-            constexpr int WCH = NOUT * 32 / 16;  // 16-byte pieces of a block
+            // packed blocks (tap, kc channels), of their 16-byte pieces (8
+            // outputs, 8 channels, output) those of 16 channels, to
+            // ((di, dk), u, dj = 2, 1, 0)
+            constexpr int WCH = NOUT * 32 / 16;  // pieces of 16 channels
+            const int lk = R.lk, nb = (nqt * 2) >> lk;
             for (int c = lt; c < 27 * NQ * WCH; c += kProducers) {
                 const int blk = c / WCH, t = blk / NQ, u = blk - t * NQ;
                 const int di = t / 9, dj = (t / 3) % 3, dk = t % 3;
+                const int w = (int)blockIdx.y * WCH + (c - blk * WCH), ch8 = (g * NQ + u) * 2 + ((w >> 3) & 1);
+                const int at = ((((w >> 4) << lk) + (ch8 & ((1 << lk) - 1))) << 3) + (w & 7);
                 cp16(wb + (g & 1) * F::WBYTES + ((((di * 3 + dk) * NQ + u) * 3 + 2 - dj) * WCH + (c - blk * WCH)) * 16,
-                     a.wpack + ((long)(t * nqt + g * NQ + u) * WCH + (c - blk * WCH)) * 8, true);
+                     a.wpack + (((long)(t * nb + (ch8 >> lk)) * R.ntot << lk) + at) * 8, true);
             }
             cp_arrive(&wfull[g & 1]);
             const int ch = g * CG + h * 8;
@@ -936,7 +949,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a, RowPla
         // ---- epilogue: position tid of the tile, one row and one voxel into
         // the run
         int i, k;
-        const bool live = row_voxel(a, R, R.P + 1 + tid, i, k);
+        const bool live = row_voxel(a, R, tile, R.P + 1 + tid, i, k);
         for (int j = js; j < je; ++j) {
             bool done = mbar_wait(&tfull[j - js], 0);
             done = __all_sync(0xffffffffu, done);
@@ -945,7 +958,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(ConvArgs a, RowPla
                 break;
             }
             tc_after();
-            store_row<NOUT>(a, tmem + (uint32_t)((j - js) * NOUT), warp, ((long)i * n1 + j) * n2 + k, live);
+            store_row<NOUT>(a, tmem + (uint32_t)((j - js) * NOUT), warp, ((long)i * n1 + j) * n2 + k, live, R.ntot,
+                            (int)blockIdx.y * NOUT);
         }
     }
 
@@ -996,9 +1010,11 @@ cudaError_t wgrad_rows(const WgradArgs& a, cudaStream_t s) {
 }
 
 template <int CG, int NOUT, int JS>
-cudaError_t rows_inst(const ConvArgs& a, cudaStream_t s) {
+cudaError_t rows_inst(const ConvArgs& a, int kc, int parts, cudaStream_t s) {
     using F = RowShape<CG, NOUT, JS>;
     RowPlan R;
+    R.lk = kc == 64 ? 3 : kc == 32 ? 2 : 1;
+    R.ntot = NOUT * parts;
     R.stream = a.n2 % kTile != 0;
     R.P = R.stream ? a.n2 + 1 : kTile + 2;
     R.nvox = 2 * R.P + kTile + 2;
@@ -1012,43 +1028,47 @@ cudaError_t rows_inst(const ConvArgs& a, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(k_conv_rows<CG, NOUT, JS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const long tiles = R.stream ? ((long)a.n0 * R.P + kTile - 1) / kTile : (long)a.n0 * (a.n2 / kTile);
+    R.tiles = (int)tiles;
     // rows a CTA: input rows walked (two more than it owns) times the CTAs an
     // SM gets, at its least; the most rows where that is equal
     long best = 0;
     for (int t = std::min(JS, a.n1); t >= 1; --t) {
-        const long ctas = tiles * ((a.n1 + t - 1) / t), cost = (ctas + kSms - 1) / kSms * (t + 2);
+        const long ctas = tiles * parts * ((a.n1 + t - 1) / t), cost = (ctas + kSms - 1) / kSms * (t + 2);
         if (!best || cost < best) {
             best = cost;
             R.rows = t;
         }
     }
     k_conv_rows<CG, NOUT, JS>
-        <<<dim3((unsigned)tiles, (unsigned)((a.n1 + R.rows - 1) / R.rows)), kRowThreads, smem, s>>>(a, R);
+        <<<dim3((unsigned)(tiles * ((a.n1 + R.rows - 1) / R.rows)), (unsigned)parts), kRowThreads, smem, s>>>(a, R);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-// The row-marching kernel covers 16 to 64 output channels from inputs in whole
-// blocks of 16: it was the faster one at every level of the network (figures at
-// the kernel).  Rows are whole 128-voxel segments or have at most 256 voxels:
+// The row-marching kernel covers 16 to 64 output channels, or 96 and 128 in
+// halves (32 -> 96 at 64^3: 146 -> 89 us, 64 -> 128 at 32^3: 53 -> 28), from
+// inputs in whole blocks of 16: it was the faster one at every level of the
+// network (figures at the kernel).  Rows are whole 128-voxel segments or have at most 256 voxels:
 // a longer run would not leave room for the weights, nor the loader's registers;
 // those, and more than 256 input channels, use k_conv.
 bool rows_supported(int cin, int nout, int n2) {
-    return cin % 16 == 0 && cin <= 256 && (nout == 16 || nout == 32 || nout == 48 || nout == 64) &&
-           (n2 % kTile == 0 || n2 <= 256);
+    const bool out = nout == 16 || nout == 32 || nout == 48 || nout == 64 || nout == 96 || nout == 128;
+    return out && cin % 16 == 0 && cin <= 256 && (n2 % kTile == 0 || n2 <= 256);
 }
 
 // Rows a CTA: 16 of 16 output channels (256 columns of tensor memory, two CTAs
 // an SM), 16 of 32, 10 of 48 and 8 of 64 (all of it).  Groups of 32 input
 // channels where both weight buffers leave room for a ring.
-cudaError_t rows_launch(const ConvArgs& a, int nout, cudaStream_t s) {
+cudaError_t rows_launch(const ConvArgs& a, int kc, int nout, cudaStream_t s) {
     const int cin = a.in.c0 + a.in.c1;
-    if (nout == 16) return rows_inst<16, 16, 16>(a, s);
-    if (nout == 32) return cin % 32 || (a.n2 % kTile && a.n2 > kTile) ? rows_inst<16, 32, 16>(a, s)
-                                                                     : rows_inst<32, 32, 16>(a, s);
-    if (nout == 48) return rows_inst<16, 48, 10>(a, s);
-    if (nout == 64) return rows_inst<16, 64, 8>(a, s);
+    if (nout == 16) return rows_inst<16, 16, 16>(a, kc, 1, s);
+    if (nout == 32) return cin % 32 || (a.n2 % kTile && a.n2 > kTile) ? rows_inst<16, 32, 16>(a, kc, 1, s)
+                                                                     : rows_inst<32, 32, 16>(a, kc, 1, s);
+    if (nout == 48) return rows_inst<16, 48, 10>(a, kc, 1, s);
+    if (nout == 64) return rows_inst<16, 64, 8>(a, kc, 1, s);
+    if (nout == 96) return rows_inst<16, 48, 10>(a, kc, 2, s);
+    if (nout == 128) return rows_inst<16, 64, 8>(a, kc, 2, s);
     return cudaErrorInvalidValue;
 }
 
@@ -1067,11 +1087,10 @@ bool wgrad_supported(int cout) { return cout == 16 || cout == 32 || cout == 64; 
     if (kc == KC && nout == N) return conv_inst<KC, N>(a, s);
 
 cudaError_t conv_launch(const ConvArgs& a, int kc, int nout, cudaStream_t s) {
-    // 16-channel weight blocks: the row-marching kernel
-    // (it counts voxels in 32 bits and column segments in 16)
-    if (kc == 16 && a.in.c0 % 16 == 0 && a.in.c1 % 16 == 0 && rows_supported(a.in.c0 + a.in.c1, nout, a.n2) &&
-        (a.n0 + 1L) * a.n1 * (a.n2 + 1L) < 1L << 31 && a.n1 <= 65535)
-        return rows_launch(a, nout, s);
+    // 16-channel weight blocks, and the widest outputs: the row-marching kernel
+    if ((kc == 16 || nout >= 96) && a.in.c0 % 16 == 0 && a.in.c1 % 16 == 0 &&
+        rows_supported(a.in.c0 + a.in.c1, nout, a.n2))
+        return rows_launch(a, kc, nout, s);
     BUN_CONV_CASE(16, 16)
     BUN_CONV_CASE(16, 32)
     BUN_CONV_CASE(16, 48)

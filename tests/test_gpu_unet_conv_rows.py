@@ -36,6 +36,8 @@ CASES = [
     ((2, 3, 255), 16, 0, 0, 64),
     ((1, 2, 300), 16, 0, 0, 16),   # too long a row: the tiled kernel
     ((2, 2, 24), 256, 0, 0, 16),
+    ((2, 11, 64), 32, 0, 0, 96),   # two halves of the output channels
+    ((1, 9, 128), 64, 0, 0, 128),
 ]
 
 
@@ -46,6 +48,7 @@ def test_convolution_rows(dims, c0, up0, c1, cout):
     L = unet.load()
     rng = np.random.default_rng(c0 + 3 * cout + dims[2])
     cin = c0 + c1
+    kc = {96: 32, 128: 64}.get(cout, 16)
     half = tuple(d // 2 for d in dims) if up0 else dims
     s0 = R.bf16(rng.standard_normal(half + (c0,)))
     s1 = R.bf16(rng.standard_normal(dims + (c1,))) if c1 else None
@@ -61,11 +64,11 @@ def test_convolution_rows(dims, c0, up0, c1, cout):
     t0, t1, wd, bd = dev(s0), dev(s1) if c1 else None, dev(W, torch.float32), dev(bias, torch.float32)
     wp = torch.zeros(W.size, dtype=torch.bfloat16, device="cuda")
     s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    assert L.bun_pack_weights(wd.data_ptr(), cin, cout, 16, 0, wp.data_ptr(), s) == 0
+    assert L.bun_pack_weights(wd.data_ptr(), cin, cout, kc, 0, wp.data_ptr(), s) == 0
     n = int(np.prod(dims)) * cout
     buf = torch.full((n + 64,), 7.0, dtype=torch.bfloat16, device="cuda")  # 64 values of guard behind the output
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
-    rc = L.bun_conv3(*dims, t0.data_ptr(), c0, up0, t1.data_ptr() if c1 else None, c1, wp.data_ptr(), 16, cout,
+    rc = L.bun_conv3(*dims, t0.data_ptr(), c0, up0, t1.data_ptr() if c1 else None, c1, wp.data_ptr(), kc, cout,
                      bd.data_ptr(), 1, None, buf.data_ptr(), err.data_ptr(), s)
     assert rc == 0
     torch.cuda.synchronize()
