@@ -1049,9 +1049,9 @@ cudaError_t rows_inst(const ConvArgs& a, int kc, int parts, cudaStream_t s) {
 // The row-marching kernel covers 16 to 64 output channels, or 96 and 128 in
 // halves (32 -> 96 at 64^3: 146 -> 89 us, 64 -> 128 at 32^3: 53 -> 28), from
 // inputs in whole blocks of 16: it was the faster one at every level of the
-// network (figures at the kernel).  Rows are whole 128-voxel segments or have at most 256 voxels:
-// a longer run would not leave room for the weights, nor the loader's registers;
-// those, and more than 256 input channels, use k_conv.
+// network (figures at the kernel).  Rows are whole 128-voxel segments or have at
+// most 256 voxels: a longer run would not leave room for the weights, nor the
+// loader's registers; those, and more than 256 input channels, use k_conv.
 bool rows_supported(int cin, int nout, int n2) {
     const bool out = nout == 16 || nout == 32 || nout == 48 || nout == 64 || nout == 96 || nout == 128;
     return out && cin % 16 == 0 && cin <= 256 && (n2 % kTile == 0 || n2 <= 256);
