@@ -18,7 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_lib", "libbmg.so")
 SOURCES = ["bmg_host.cu", "bmg_kernels.cu", "bmg_smooth_fused.cu", "bmg_krylov.cu", "bmg_noalloc.cu",
            "bmg_project.cu", "bmg_tail.cu"]
-HEADERS = ["bmg_internal.h", "bmg_stencil.cuh", "bmg_grid.cuh"]
+HEADERS = ["bmg_internal.h", "bmg_plan.h", "bmg_stencil.cuh", "bmg_grid.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FFT_OUT = os.path.join(HERE, "_lib", "libbfft.so")
 FFT_SOURCES = ["bfft.cu", "bfft_pair.cu", "bfft_tri.cu"]

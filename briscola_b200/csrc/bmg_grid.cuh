@@ -81,11 +81,16 @@ __device__ __forceinline__ void solve_decision(SolveState* st, double l2, int mo
 }
 
 inline dim3 block_for(int n2) {
-    // k extent on lanes; small rows give the spare lanes to j
-    if (n2 >= 64) return dim3(64, 4, 1);
-    if (n2 >= 32) return dim3(32, 8, 1);
-    if (n2 >= 16) return dim3(16, 16, 1);
-    return dim3(8, 32, 1);
+    const Tile t = cell_tile(n2);
+    return dim3(t.x, t.y, 1);
+}
+
+// what bmg_plan.h counts with
+template <typename T>
+inline Level0 level0(const Bricks<T>& B) {
+    bool quads = true;
+    for (int b = 0; b < B.nb; ++b) quads = quads && B.v[b].n2 % 4 == 0;
+    return {B.nb, B.max1, B.max2, B.z0[B.nb], quads};
 }
 
 template <typename T>

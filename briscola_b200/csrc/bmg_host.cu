@@ -1145,7 +1145,7 @@ void build(bmg_ctx* c, HostLevel&& L0) {
     c->variable = c->multi && !c->conforming;
     if (c->multi) uploadLambda(c);
     buildTransfers(c);
-    c->partials = dalloc<double>(3 * reduce_blocks(bricks<double>(c, 0)));
+    c->partials = dalloc<double>(reduce_doubles(bricks<double>(c, 0)));
     c->st = dalloc<SolveState>(1);
     BMG_CUDA(cudaMallocHost(&c->st_host, sizeof(SolveState)));
     c->stage_b = dalloc<double>(c->lv[0].ncell);

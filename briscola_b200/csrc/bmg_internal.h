@@ -31,6 +31,8 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "bmg_plan.h"
+
 namespace bmg {
 
 constexpr int kMaxBricks = 8;
@@ -310,8 +312,10 @@ void launch_finalize(const Bricks<double>& B, const double* partials, SolveState
 void launch_mean(const Bricks<double>& B, double* partials, SolveState* st, cudaStream_t s);
 // st->ybar = plain mean of the interior x (gAverage, solver.C:24)
 void launch_plain_mean(const Bricks<double>& B, double* partials, SolveState* st, cudaStream_t s);
-// number of per-block partial sums the level-0 reductions write
+// number of per-block partial sums the level-0 reductions write, and the
+// doubles of the buffer that holds those of every reduction
 long reduce_blocks(const Bricks<double>& B);
+long reduce_doubles(const Bricks<double>& B);
 // sets the dynamic shared memory limits of the fused smoother instances
 void configure_fused_kernels();
 

@@ -1302,10 +1302,10 @@ __global__ void __launch_bounds__(256) k_add_correction(Bricks<double> B, Bricks
 // ---- launchers --------------------------------------------------------------
 
 long reduce_blocks(const Bricks<double>& B) {
-    const dim3 blk = block_for(B.max2);
-    const dim3 g = grid_for(B, B.max2, blk);
-    return (long)g.x * g.y * g.z;
+    return cell_partials(level0(B));
 }
+
+long reduce_doubles(const Bricks<double>& B) { return partials_capacity(level0(B)); }
 
 template <typename T, bool VAR>
 void launch_colour_pass(const Bricks<T>& B, int colour, cudaStream_t s, bool zero) {

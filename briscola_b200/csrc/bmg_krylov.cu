@@ -207,8 +207,6 @@ __global__ void __launch_bounds__(kFinalThreads) k_fcg_true_norm(const double* p
 // per-block partials for the one-block kernels to add.  Same per-cell
 // arithmetic as the kernels above; used when every brick's n2 % 4 == 0.
 
-constexpr int kQuadPlanes = 64;  // grid z: plane groups
-
 // The logical k-quad k0 .. k0+3 at slab index p (its first cell): one
 // vector in a natural row (kh = 0); in a parity-split row the even pair
 // (k0, k0+2) at p and the odd pair (k0+1, k0+3) at p + kh.
@@ -696,26 +694,16 @@ __global__ void __launch_bounds__(kFinalThreads) k_fcg_coeffs(const double* part
 
 #undef BMG_QUAD_LOOP
 
-bool fcg_quads(const Bricks<double>& B) {
-    for (int b = 0; b < B.nb; ++b)
-        if (B.v[b].n2 % 4) return false;
-    return true;
-}
+bool fcg_quads(const Bricks<double>& B) { return level0(B).quads; }
 
-// several bricks: more plane groups, since many blocks of a plane lie outside
-// their brick
 dim3 quad_grid(const Bricks<double>& B) {
-    return dim3((unsigned)((B.max2 / 4 + 15) / 16), (unsigned)((B.max1 + 15) / 16),
-                (unsigned)std::min(B.z0[B.nb], B.nb > 1 ? 4 * kQuadPlanes : kQuadPlanes));
+    const Level0 L = level0(B);
+    return dim3(blocks_of(L.max2 / 4, kQuadTile), blocks_of(L.max1, kQuadTile), quad_planes(L));
 }
 
 }  // namespace
 
-long fcg_partials(const Bricks<double>& B) {
-    if (!fcg_quads(B)) return reduce_blocks(B);
-    const dim3 g = quad_grid(B);
-    return (long)g.x * g.y * g.z;
-}
+long fcg_partials(const Bricks<double>& B) { return step_partials(level0(B)); }
 
 template <bool VAR>
 long launch_residual_split(const Bricks<double>& B, const Walls& W, int mode, double* r, float* pre32,
