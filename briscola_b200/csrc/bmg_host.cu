@@ -1616,10 +1616,8 @@ void tailCycle(bmg_ctx* c, int first) {
     P.nops = (int)ops.size();
     std::copy(ops.begin(), ops.end(), P.ops);
     c->launches += 1;
-    if (c->variable)
-        launch_tail_cycle<T, true>(P, c->stream);
-    else
-        launch_tail_cycle<T, false>(P, c->stream);
+    const cudaError_t e = c->variable ? launch_tail_cycle<T, true>(P, c->stream) : launch_tail_cycle<T, false>(P, c->stream);
+    BMG_CUDA(e);
 }
 
 // A graphed solve runs its whole loop in the cluster where all its levels
@@ -1637,10 +1635,8 @@ void tailSolve(bmg_ctx* c) {
     std::copy(ops.begin(), ops.end(), P.ops);
     P.st = c->st;
     c->launches += 1;
-    if (c->variable)
-        launch_tail_solve<true>(P, c->stream);
-    else
-        launch_tail_solve<false>(P, c->stream);
+    const cudaError_t e = c->variable ? launch_tail_solve<true>(P, c->stream) : launch_tail_solve<false>(P, c->stream);
+    BMG_CUDA(e);
 }
 
 // The level solver's turn (bmg_set_level_solver): the level's right-hand
@@ -1926,6 +1922,7 @@ void captureGraph(bmg_ctx* c, bool zero) {
         BMG_CUDA(cudaStreamEndCapture(s, &g));
         c->launchesInitPost = c->launches - l0;
         c->launchesBody = 0;
+        checkLaunch();
         BMG_CUDA(cudaGraphInstantiate(&c->gexec, c->graph, 0));
         c->graphZero = zero;
         return;
@@ -1962,6 +1959,8 @@ void captureGraph(bmg_ctx* c, bool zero) {
     BMG_CUDA(cudaStreamEndCapture(s, &body));
     c->launchesInitPost = l1 - l0;
     c->launchesBody = c->launches - l1;
+    // (a launch that the capture refused would be missing from the graph)
+    checkLaunch();
     BMG_CUDA(cudaGraphInstantiate(&c->gexec, c->graph, 0));
     c->graphZero = zero;
 }
@@ -2293,6 +2292,7 @@ int bmg_set_coefficients(bmg_ctx* c, const double* lx, const double* ly, const d
         c->variable = c->userLambda || (c->multi && !c->conforming);
         if (c->variable) uploadLambda(c);
         refreshCoarseInverse(c);
+        c->tail = tailFirst(c);  // face coefficients take shared memory there
         destroyGraph(c);  // kernels differ between constant and variable coefficients
         return BMG_OK;
     });

@@ -289,10 +289,10 @@ template <typename T>
 void launch_coarse_solve(const Bricks<T>& C, const double* ainv, const int* cidx, int n, cudaStream_t s);
 // the coarse end of a cycle in one cluster (bmg_tail.cu)
 template <typename T, bool VAR>
-void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s);
+cudaError_t launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s);
 // the whole FP64 loop of a solve whose level 0 is the first level there
 template <bool VAR>
-void launch_tail_solve(const TailPlan<double>& P, cudaStream_t s);
+cudaError_t launch_tail_solve(const TailPlan<double>& P, cudaStream_t s);
 cudaError_t configure_tail_kernels();
 template <typename T, bool VAR>
 void launch_residual_out(const Bricks<T>& B, double* r_unscaled_compact, cudaStream_t s);

@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail_cycle(const __grid_con
 }  // namespace
 
 template <typename T, bool VAR, bool SOLVE>
-static void launch_tail(const TailPlan<T>& P, cudaStream_t s) {
+static cudaError_t launch_tail(const TailPlan<T>& P, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P.ranks);
     cfg.blockDim = dim3(kTailThreads);
@@ -587,17 +587,17 @@ static void launch_tail(const TailPlan<T>& P, cudaStream_t s) {
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = kProgrammaticLaunch ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, k_tail_cycle<T, VAR, SOLVE>, P);
+    return cudaLaunchKernelEx(&cfg, k_tail_cycle<T, VAR, SOLVE>, P);
 }
 
 template <typename T, bool VAR>
-void launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s) {
-    launch_tail<T, VAR, false>(P, s);
+cudaError_t launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s) {
+    return launch_tail<T, VAR, false>(P, s);
 }
 
 template <bool VAR>
-void launch_tail_solve(const TailPlan<double>& P, cudaStream_t s) {
-    launch_tail<double, VAR, true>(P, s);
+cudaError_t launch_tail_solve(const TailPlan<double>& P, cudaStream_t s) {
+    return launch_tail<double, VAR, true>(P, s);
 }
 
 template <typename T, bool VAR, bool SOLVE = false>
@@ -615,11 +615,11 @@ cudaError_t configure_tail_kernels() {
     return cudaSuccess;
 }
 
-template void launch_tail_cycle<double, false>(const TailPlan<double>&, cudaStream_t);
-template void launch_tail_cycle<double, true>(const TailPlan<double>&, cudaStream_t);
-template void launch_tail_cycle<float, false>(const TailPlan<float>&, cudaStream_t);
-template void launch_tail_cycle<float, true>(const TailPlan<float>&, cudaStream_t);
-template void launch_tail_solve<false>(const TailPlan<double>&, cudaStream_t);
-template void launch_tail_solve<true>(const TailPlan<double>&, cudaStream_t);
+template cudaError_t launch_tail_cycle<double, false>(const TailPlan<double>&, cudaStream_t);
+template cudaError_t launch_tail_cycle<double, true>(const TailPlan<double>&, cudaStream_t);
+template cudaError_t launch_tail_cycle<float, false>(const TailPlan<float>&, cudaStream_t);
+template cudaError_t launch_tail_cycle<float, true>(const TailPlan<float>&, cudaStream_t);
+template cudaError_t launch_tail_solve<false>(const TailPlan<double>&, cudaStream_t);
+template cudaError_t launch_tail_solve<true>(const TailPlan<double>&, cudaStream_t);
 
 }  // namespace bmg

@@ -58,3 +58,31 @@ def test_cluster_tail_matches_per_pass(native, n, bc, coarse, cycle):
             assert out[0][1] < out[1][1]  # the cluster ran
             # the same operations cell by cell
             assert np.array_equal(out[0][0], out[1][0]), (precision, coef is not None)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [(512, 8, 8), (8, 128, 256), (128, 8, 256), (2, 2, 512), (2, 2, 1024)])
+def test_coefficients_given_to_a_context_that_fits_without_them(native, n, precision):
+    """face coefficients take shared memory in the cluster: a context planned
+    without them plans again when they come and when they go"""
+    mesh = _mesh(n, (N, N, N))
+    rng = np.random.default_rng(6)
+    V = mesh.bricks[0].cell_volumes()
+    b = np.ascontiguousarray((-V * workloads.zero_mean(rng.standard_normal(n), V)).ravel())
+    lam = [rng.uniform(0.5, 1.5, s) for s in ((n[0] + 1, n[1], n[2]), (n[0], n[1] + 1, n[2]), (n[0], n[1], n[2] + 1))]
+    out = {}
+    for fuse in ("on", "off"):
+        c = bb.Context(mesh, bb.make_options({
+            "relTol": 0.0, "tolerance": 0, "minIter": 2, "maxIter": 2, "nSweepsPre": 2, "nSweepsPost": 2,
+            "cycleType": "V", "coarseLevel": 0, "precision": precision, "fuseCoarse": fuse, "autotune": "off"}))
+        out[fuse] = []
+        for coef in (None, lam, None):
+            c.set_coefficients(coef)
+            for _ in range(2):  # the second one replays the graph
+                x = np.zeros_like(b)
+                rep = c.solve(b, x, zero_guess=True)
+                out[fuse].append((x, rep.cycles, rep.final_l2))
+        c.close()
+    for on, off in zip(out["on"], out["off"]):
+        assert on[1] == off[1] == 2 and np.isfinite(on[2])
+        assert np.array_equal(on[0], off[0])
