@@ -1507,7 +1507,7 @@ TailPlan<T> tailPlan(const bmg_ctx* c, int first) {
         L.P = L.n0;
         if (L.dist) {
             const int g = c->lv[l + 1].br[0].R[0];
-            L.P = g * ((L.n0 + g * kTailRanks - 1) / (g * kTailRanks));
+            L.P = tail_planes(L.n0, g, kTailRanks);
             used = std::max(used, (L.n0 + L.P - 1) / L.P);
         }
         L.sj = V.n2 + 2;

@@ -1,9 +1,15 @@
 // bmg_plan.h -- counts and extents that a launch and the buffer it writes
-// have to agree on, as plain integer arithmetic (no CUDA types: the CPU tests
-// compile this header by itself).
+// have to agree on, and index ranges of kernels, as plain integer arithmetic
+// (no CUDA types: the CPU tests compile this header by itself).
 #pragma once
 
 #include <algorithm>
+
+#ifdef __CUDACC__
+#define BMG_HD __host__ __device__
+#else
+#define BMG_HD
+#endif
 
 namespace bmg {
 
@@ -55,5 +61,26 @@ inline long step_partials(const Level0& L) { return L.quads ? quad_partials(L) :
 // (rows of 4 or 8 cells have half as many rows of blocks in cell_partials as in
 // quad_partials)
 inline long partials_capacity(const Level0& L) { return 3 * std::max(cell_partials(L), step_partials(L)); }
+
+// ---- a level spread over a cluster's CTAs (bmg_tail.cu) ----------------------
+// i-planes of a CTA, in whole groups of g (the planes that one coarse plane
+// covers): rank r owns planes r P .. r P + P - 1 as far as there are any
+inline int tail_planes(int n0, int g, int ranks) { return g * ((n0 + g * ranks - 1) / (g * ranks)); }
+
+struct Planes {
+    int first, count;
+};
+BMG_HD inline Planes tail_own(int n0, int P, int rank) {
+    const int first = rank * P, left = n0 - first;
+    return {first, left < 0 ? 0 : left < P ? left : P};
+}
+
+// planes of x that a CTA with `own` reads from memory: its own and the
+// neighbours' on either side (-1 and n0 are the level's ghost planes).  The
+// cluster is a power of two, so CTAs behind the last plane own none and read
+// none.
+BMG_HD inline Planes tail_read(Planes own) {
+    return {own.first - 1, own.count ? own.count + 2 : 0};
+}
 
 }  // namespace bmg

@@ -57,8 +57,8 @@ struct Own {
 };
 template <typename T>
 __device__ __forceinline__ Own own_planes(const TailLevel<T>& L, int rank) {
-    const int p0 = rank * L.P;
-    return {p0, max(0, min(L.P, L.n0 - p0))};
+    const Planes p = tail_own(L.n0, L.P, rank);
+    return {p.first, p.count};
 }
 
 // stores x of cell (i, j, k) at word c (local plane li of cnt), its periodic
@@ -492,13 +492,14 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail_cycle(const __grid_con
             sm[L.b + ij * L.n2 + spos(L, k)] =
                 P.gb[L.gbase + (o.p0 + li) * L.gsi + j * L.gsj + (L.gkh ? kpos_split(k, L.gkh) : k)];
         }
+        const Planes in = tail_read({o.p0, o.cnt});
         for (int e = threadIdx.x; e < L.xcells; e += kTailThreads) {
             T v = T(0);
             if (!P.zeroStart) {
                 const int s = e / L.si, j = (e - s * L.si) / L.sj, p = e - s * L.si - j * L.sj - 1;
                 const int k = p < 0 || p >= L.n2 ? p : p < L.ne ? 2 * p : 2 * (p - L.ne) + 1;
-                if (s < o.cnt + 2)
-                    v = P.gx[L.gbase + (o.p0 + s - 1) * L.gsi + (j - 1) * L.gsj + (L.gkh ? kpos_split(k, L.gkh) : k)];
+                if (s < in.count)
+                    v = P.gx[L.gbase + (in.first + s) * L.gsi + (j - 1) * L.gsj + (L.gkh ? kpos_split(k, L.gkh) : k)];
             }
             sm[L.x + e] = v;
         }

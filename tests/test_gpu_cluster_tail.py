@@ -86,3 +86,26 @@ def test_coefficients_given_to_a_context_that_fits_without_them(native, n, preci
     for on, off in zip(out["on"], out["off"]):
         assert on[1] == off[1] == 2 and np.isfinite(on[2])
         assert np.array_equal(on[0], off[0])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,bc", [((24, 16, 16), (N, N, N)), ((48, 8, 16), (D, N, P)), ((24, 24, 8), (N, D, N))])
+def test_level_0_in_the_cluster_from_a_guess(native, n, bc, precision):
+    """level 0 read into the cluster with its ghosts, where the last of its
+    CTAs own no plane"""
+    mesh = _mesh(n, bc)
+    rng = np.random.default_rng(7)
+    V = mesh.bricks[0].cell_volumes()
+    b = np.ascontiguousarray((-V * workloads.zero_mean(rng.standard_normal(n), V)).ravel())
+    guess = rng.standard_normal(b.size)
+    out = []
+    for fuse in ("on", "off"):
+        c = bb.Context(mesh, bb.make_options({
+            "relTol": 0.0, "tolerance": 0, "minIter": 2, "maxIter": 2, "nSweepsPre": 2, "nSweepsPost": 2,
+            "cycleType": "V", "coarseLevel": 0, "precision": precision, "fuseCoarse": fuse, "autotune": "off"}))
+        x = guess.copy()
+        rep = c.solve(b, x)
+        out.append((x, rep.kernel_launches))
+        c.close()
+    assert out[0][1] < out[1][1]
+    assert np.array_equal(out[0][0], out[1][0])

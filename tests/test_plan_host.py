@@ -46,3 +46,37 @@ def test_partial_sums_fit_their_buffer(tmp_path):
         else:
             assert step == cell
         assert 3 * max(cell, step) <= room, row
+
+
+def test_planes_of_a_level_over_the_cluster(tmp_path):
+    """every plane has one owner, in whole groups, and what a CTA reads of x
+    lies inside the level and its ghost planes -- also a CTA that owns nothing
+    because the cluster is the next power of two"""
+    rows = run_plan(tmp_path, r"""
+        for (int ranks : {1, 2, 4, 8, 16})
+            for (int g : {1, 2})
+                for (int n0 = g; n0 <= 600; n0 += g) {
+                    const int P = tail_planes(n0, g, ranks), used = (n0 + P - 1) / P;
+                    int launched = 1;
+                    while (launched < used) launched *= 2;
+                    for (int r = 0; r < launched; ++r) {
+                        const Planes o = tail_own(n0, P, r), x = tail_read(o);
+                        std::printf("%d %d %d %d %d %d %d %d %d %d\n", ranks, g, n0, P, launched, r, o.first, o.count,
+                                    x.first, x.count);
+                    }
+                }
+    """)
+    owned, idle = {}, 0
+    for row in rows:
+        ranks, g, n0, P, launched, r, first, count, x0, nx = map(int, row.split())
+        assert launched <= ranks and P % g == 0
+        assert count % g == 0 and 0 <= count <= P
+        owned.setdefault((ranks, g, n0), []).extend(range(first, first + count))
+        idle += count == 0
+        if nx:
+            assert -1 <= x0 and x0 + nx <= n0 + 1, row
+        if count:
+            assert x0 <= first - 1 and x0 + nx >= first + count + 1, row
+    assert idle > 0
+    for (ranks, g, n0), planes in owned.items():
+        assert planes == list(range(n0)), (ranks, g, n0)
