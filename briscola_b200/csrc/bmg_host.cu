@@ -142,6 +142,7 @@ struct bmg_ctx {
     std::vector<std::vector<BrickTransfer>> tr;  // [level][brick]
     int lc = 0;  // coarse solve level
     int tail = -1;  // first level of the cycle's end in the cluster, -1: none
+    int tailRanks = 0;  // CTAs of the largest cluster the device runs it in, 0: none
     double* ainv = nullptr;
     int* cidx = nullptr;
     int ncoarse = 0;
@@ -1507,7 +1508,7 @@ TailPlan<T> tailPlan(const bmg_ctx* c, int first) {
         L.P = L.n0;
         if (L.dist) {
             const int g = c->lv[l + 1].br[0].R[0];
-            L.P = tail_planes(L.n0, g, kTailRanks);
+            L.P = tail_planes(L.n0, g, c->tailRanks);
             used = std::max(used, (L.n0 + L.P - 1) / L.P);
         }
         L.sj = V.n2 + 2;
@@ -1578,7 +1579,7 @@ TailPlan<T> tailPlan(const bmg_ctx* c, int first) {
 }
 
 int tailFirst(bmg_ctx* c) {
-    if (!c->opt.fuse_coarse || c->multi ||
+    if (!c->opt.fuse_coarse || c->multi || !c->tailRanks ||
         (c->opt.cycle_type != BMG_CYCLE_V && c->opt.cycle_type != BMG_CYCLE_F) ||
         c->opt.smoother != BMG_SMOOTHER_RBGS || c->opt.coarse_mode != BMG_COARSE_DIRECT)
         return -1;
@@ -2184,7 +2185,7 @@ int bmg_create(bmg_ctx** out, const bmg_mesh_desc* mesh, const bmg_options* opts
         c->own_stream = true;
         BMG_CUDA(cudaStreamCreateWithFlags(&c->capStream, cudaStreamNonBlocking));
         configure_fused_kernels();
-        BMG_CUDA(configure_tail_kernels());
+        c->tailRanks = configure_tail_kernels();
         build(c, std::move(L0));
         configureCoarse(c);
         c->tail = tailFirst(c);

@@ -220,7 +220,7 @@ constexpr int kMaxTailOps = 384;
 constexpr int kTailThreads = 1024;
 // A level runs in the cluster where every CTA has at most one pair of cells a
 // thread (32^3 on 16 CTAs), so that a pass is one update's latency.
-constexpr int kTailRanks = 16;         // CTAs of the cluster
+constexpr int kTailRanks = 16;         // most CTAs of the cluster
 constexpr long kTailGather = 1024;     // levels this small run on CTA 0 alone
 
 constexpr int kTailCoarse = 512;       // largest dense coarse solve there
@@ -293,7 +293,10 @@ cudaError_t launch_tail_cycle(const TailPlan<T>& P, cudaStream_t s);
 // the whole FP64 loop of a solve whose level 0 is the first level there
 template <bool VAR>
 cudaError_t launch_tail_solve(const TailPlan<double>& P, cudaStream_t s);
-cudaError_t configure_tail_kernels();
+// allows the kernels their shared memory and cluster size on the current device;
+// CTAs of the largest cluster that it can hold, 0 where it holds none (the
+// levels then keep a launch per pass)
+int configure_tail_kernels();
 template <typename T, bool VAR>
 void launch_residual_out(const Bricks<T>& B, double* r_unscaled_compact, cudaStream_t s);
 // x[dst[q]] = x[src[q]]: ghost refresh between bricks

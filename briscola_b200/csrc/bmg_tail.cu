@@ -602,18 +602,35 @@ cudaError_t launch_tail_solve(const TailPlan<double>& P, cudaStream_t s) {
 }
 
 template <typename T, bool VAR, bool SOLVE = false>
-static cudaError_t allow_tail() {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_tail_cycle<T, VAR, SOLVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_tail_cycle<T, VAR, SOLVE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+static int allow_tail() {
+    const auto kernel = k_tail_cycle<T, VAR, SOLVE>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem) != cudaSuccess) return 0;
+    // a cluster lies in one GPC: a part of a device may hold a small one only,
+    // or none
+    const bool most = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (int r = most ? kTailRanks : 8; r >= 1; r /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(r);
+        cfg.blockDim = dim3(kTailThreads);
+        cfg.dynamicSmemBytes = kTailSmem;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = r;
+        at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n >= 1) return r;
+    }
+    return 0;
 }
 
-cudaError_t configure_tail_kernels() {
-    for (cudaError_t e : {allow_tail<float, false>(), allow_tail<float, true>(), allow_tail<double, false>(),
-                          allow_tail<double, true>(), allow_tail<double, false, true>(), allow_tail<double, true, true>()})
-        if (e != cudaSuccess) return e;
-    return cudaSuccess;
+int configure_tail_kernels() {
+    const int r = std::min({allow_tail<float, false>(), allow_tail<float, true>(), allow_tail<double, false>(),
+                            allow_tail<double, true>(), allow_tail<double, false, true>(), allow_tail<double, true, true>()});
+    if (r < kTailRanks) cudaGetLastError();  // a refused query is an answer
+    return r;
 }
 
 template cudaError_t launch_tail_cycle<double, false>(const TailPlan<double>&, cudaStream_t);
