@@ -1585,11 +1585,16 @@ int tailFirst(bmg_ctx* c) {
         return -1;
     const int lc = c->lc;
     if (c->ncoarse > kTailCoarse) return -1;
+    // a level solver takes its turn between launches: the cluster's levels lie
+    // below its level
+    const int hooked = c->hook ? c->hookLevel : -1;
+    if (hooked >= lc) return -1;
     const bool f32 = c->opt.precision == BMG_PRECISION_MIXED;
     int first = lc;
     for (; first > 0; --first) {
         const HostLevel& H = c->lv[first - 1];
         if (lc - first + 2 > kMaxTail) break;
+        if (first - 1 == hooked) break;
         const TailPlan<double> S = tailPlan<double>(c, first - 1);
         if ((long)S.v[0].P * S.v[0].n1 * S.v[0].ne > kTailThreads) break;
         // (a periodic axis of one cell has two images of it)
@@ -1603,10 +1608,7 @@ int tailFirst(bmg_ctx* c) {
         if ((int)ops.size() > kMaxTailOps) break;
     }
     std::fill(c->visits.begin(), c->visits.end(), 0);
-    if (first == lc) return -1;
-    // a level solver inside the tail's levels would be skipped by it
-    if (c->hook && c->hookLevel >= first) return -1;
-    return first;
+    return first == lc ? -1 : first;
 }
 
 template <typename T>

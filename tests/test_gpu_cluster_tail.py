@@ -109,3 +109,42 @@ def test_level_0_in_the_cluster_from_a_guess(native, n, bc, precision):
         c.close()
     assert out[0][1] < out[1][1]
     assert np.array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("mode", ["guess", "replace"])
+@pytest.mark.parametrize("level", [1, 2, 3, 4])
+def test_levels_below_a_level_solver(native, level, mode):
+    """a level solver at a level that would fit the cluster: the levels below
+    it run there, and the solver is called as often as with a launch per pass"""
+    import torch
+
+    from briscola_b200 import learned
+
+    mesh = learned.cube_mesh(64)
+    b = np.random.default_rng(8).standard_normal(64**3)
+    b -= b.mean()
+    out = []
+    for fuse in ("on", "off"):
+        c = bb.Context(mesh, bb.make_options({
+            "relTol": 0.0, "tolerance": 0, "minIter": 3, "maxIter": 3, "nSweepsPre": 2, "nSweepsPost": 2,
+            "cycleType": "V", "coarseLevel": 1, "precision": "mixed", "krylov": "fcg", "fuseCoarse": fuse,
+            "graph": "off", "autotune": "off"}))
+        calls = []
+
+        def smooth_guess(stream, rhs, x, shape):
+            torch.cuda.synchronize()
+            r = torch.empty(int(np.prod(shape)), dtype=torch.float32, device="cuda")
+            learned._copy_from_ptr(r, rhs)
+            calls.append(shape)
+            learned._copy_to_ptr(x, (r * (-0.1 / 64**2 * 4**level)).contiguous())
+            torch.cuda.synchronize()
+
+        c.set_level_solver(level, smooth_guess, mode)
+        x = np.zeros_like(b)
+        rep = c.solve(b, x, zero_guess=True)
+        out.append((x, len(calls), rep.kernel_launches))
+        c.close()
+    assert out[0][1] == out[1][1] == 3
+    assert np.array_equal(out[0][0], out[1][0])
+    if mode == "guess" and level < 3:  # (the coarse solve's level is 4)
+        assert out[0][2] < out[1][2]
