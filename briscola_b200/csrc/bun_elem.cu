@@ -179,18 +179,32 @@ __global__ void __launch_bounds__(kBlock, 2) k_conv_in(int n0, int n1, int n2, c
 // channels each and march along k over runs of kInRun voxels with the nine rows'
 // three columns in registers, so dz is read once, and x nine values a step: bound
 // by the 56 sums a step.  A CTA for every tap, then three taps, read dz 28 and
-// ten times: 346 and 206 us at 128^3, now 150.
+// ten times: 346 and 206 us at 128^3, now 146.
+// A run's sums go to totals in shared memory (two channels a word, a column a
+// thread): a chain of FP32 additions is a run's voxels or the thread's runs
+// long, not their product, which at 256^3 had 2048 terms and lost to the
+// thread-per-voxel kernel's 256 (relative error against 64 bits 8.5e-7, now 3.4e-7;
+// that kernel 3.7e-7); the totals cost no time that shows (1134 -> 1123 us).
 constexpr int kInRun = 32;
+constexpr int kInTotals = 28 * kBlock * (int)sizeof(float2);
 __global__ void __launch_bounds__(kBlock, 2) k_conv_in_wgrad(int n0, int n1, int n2, const float* __restrict__ x,
                                                              const bf16* __restrict__ dz, float* __restrict__ part) {
     constexpr int WARPS = kBlock / 32;
     __shared__ float sh[WARPS][28 * 16];
+    extern __shared__ float2 total[];  // [28][kBlock]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c2 = lane & 7;
     const int nr = (n2 + kInRun - 1) / kInRun;
     const long runs = (long)n0 * n1 * nr, groups = (long)gridDim.x * (kBlock / 8);
+    // (zeros the compiler does not see: it would peel the first steps of a run and spill)
+    auto zero = [](float& v) { asm volatile("mov.b32 %0, 0;" : "=f"(v)); };
     float acc[28][2];
 #pragma unroll
-    for (int t = 0; t < 28; ++t) acc[t][0] = acc[t][1] = 0.f;
+    for (int t = 0; t < 28; ++t) {
+        zero(acc[t][0]);
+        zero(acc[t][1]);
+        total[t * kBlock + threadIdx.x] = make_float2(0.f, 0.f);
+    }
+#pragma unroll 1
     for (long g = ((long)blockIdx.x * kBlock + threadIdx.x) >> 3; g < runs; g += groups) {
         int i, j, q;
         decode(g, n1, nr, i, j, q);
@@ -232,17 +246,28 @@ __global__ void __launch_bounds__(kBlock, 2) k_conv_in_wgrad(int n0, int n1, int
             acc[27][0] += d.x;
             acc[27][1] += d.y;
         }
+#pragma unroll
+        for (int t = 0; t < 28; ++t) {
+            float2& s = total[t * kBlock + threadIdx.x];
+            s = make_float2(s.x + acc[t][0], s.y + acc[t][1]);
+            zero(acc[t][0]);
+            zero(acc[t][1]);
+        }
     }
     // the warp's four groups, then the warps
 #pragma unroll
-    for (int t = 0; t < 28; ++t)
+    for (int t = 0; t < 28; ++t) {
+        float2 v = total[t * kBlock + threadIdx.x];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            float v = acc[t][e];
-            v += __shfl_xor_sync(0xffffffffu, v, 8);
-            v += __shfl_xor_sync(0xffffffffu, v, 16);
-            if (lane < 8) sh[warp][t * 16 + 2 * c2 + e] = v;
+        for (int o = 8; o <= 16; o *= 2) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
         }
+        if (lane < 8) {
+            sh[warp][t * 16 + 2 * c2] = v.x;
+            sh[warp][t * 16 + 2 * c2 + 1] = v.y;
+        }
+    }
     __syncthreads();
     for (int q = threadIdx.x; q < 28 * 16; q += kBlock) {
         float v = 0.f;
@@ -594,7 +619,10 @@ cudaError_t conv_in_launch(int n0, int n1, int n2, const float* x, const float* 
 
 cudaError_t conv_in_wgrad_launch(int n0, int n1, int n2, const float* x, const bf16* dz, float* part, int nblocks,
                                  float* dw, cudaStream_t s) {
-    k_conv_in_wgrad<<<(unsigned)nblocks, kBlock, 0, s>>>(n0, n1, n2, x, dz, part);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_conv_in_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kInTotals);
+    if (e != cudaSuccess) return e;
+    k_conv_in_wgrad<<<(unsigned)nblocks, kBlock, kInTotals, s>>>(n0, n1, n2, x, dz, part);
     k_sum_parts<<<blocks_for(28 * 16), kBlock, 0, s>>>(part, nblocks, 28 * 16, 28 * 16, 1.f, dw);
     return cudaGetLastError();
 }

@@ -76,3 +76,35 @@ def test_input_convolution_and_its_gradient(dims):
     ref = np.concatenate([R.conv3_wgrad(x64, dz).reshape(27, 16), dz.sum(axis=(0, 1, 2))[None]])
     got = dw.cpu().numpy().astype(np.float64).reshape(28, 16)
     assert np.linalg.norm(got - ref) <= 1e-4 * np.linalg.norm(ref)  # FP32 sums
+
+
+@pytest.mark.parametrize("sign", ["constant", "random"])
+def test_input_gradient_over_many_voxels(sign):
+    """the FP32 sums of a large grid against 64 bits: a thread adds the voxels of
+    a run of 32, its runs, then the groups and blocks -- one rounding each, and
+    terms of one sign are the worst case"""
+    from briscola_b200 import unet
+
+    L = unet.load()
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    n, nblocks = 128, 4
+    V = n**3
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.full((V,), 0.1, device="cuda")
+    dz = torch.full((V, 16), 0.3, device="cuda")
+    if sign == "random":
+        x, dz = torch.randn(V, generator=g, device="cuda"), torch.randn((V, 16), generator=g, device="cuda")
+    dz = dz.bfloat16()
+    part, dw = torch.zeros(nblocks * 448, device="cuda"), torch.zeros(448, device="cuda")
+    assert L.bun_conv_in_wgrad(n, n, n, x.data_ptr(), dz.data_ptr(), nblocks, part.data_ptr(), dw.data_ptr(), s) == 0
+    xp = torch.nn.functional.pad(x.double().view(n, n, n), (1,) * 6)
+    sums, sizes = [], []
+    for t in range(28):
+        a = xp[t // 9:t // 9 + n, t // 3 % 3:t // 3 % 3 + n, t % 3:t % 3 + n].reshape(1, -1) if t < 27 else \
+            torch.ones((1, V), dtype=torch.float64, device="cuda")
+        sums.append(a @ dz.double())
+        sizes.append(a.abs() @ dz.double().abs())
+    # the product is not rounded (a fused multiply-add); 32 + runs of a group + 4 groups, 8 warps, the blocks
+    chain = 32 + V // 32 // (nblocks * 32) + 2 + 8 + nblocks
+    err = (dw.double() - torch.cat(sums).reshape(-1)).abs()
+    assert bool((err <= chain * 2.0**-24 * torch.cat(sizes).reshape(-1)).all())
