@@ -713,7 +713,6 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 //    32^3  64 -> 64    50 /   21;  16^3 64 -> 64   30 /   17
 constexpr int kRowThreads = 288;
 constexpr int kRowRing = 8;  // most rows of the ring
-constexpr int kSms = 148;
 
 struct RowPlan {
     int P;       // distance of the planes' rows in the run

@@ -74,22 +74,22 @@ __device__ __forceinline__ float block_sum(float x, float* sh) {
 // each tap's weights four channels at a time, so one shared-memory load
 // feeds sixteen FMAs.
 constexpr int kInK = 64, kInJ = 16;  // kInK * kInJ == 4 * kBlock
-constexpr int kInI = 8;              // planes a CTA
-// A CTA walks kInI planes of its tile with the input planes in a ring of four,
-// the next one's copies under this one's arithmetic, so a plane is fetched once
-// and not three times with every load waited for: 256^3 545 -> 381 us. Bound by
-// the multiply-adds (432 a voxel, two channels an instruction: 200 us of issue)
+constexpr int kInI = 8;              // most planes a CTA
+// A CTA walks up to kInI planes of its tile with the input planes in a ring of
+// four, the next one's copies under this one's arithmetic, so a plane is fetched
+// once and not three times with every load waited for: 256^3 543 -> 365 us. Bound
+// by the multiply-adds (432 a voxel, two channels an instruction: 200 us of issue)
 // and the weights' shared loads between them.
-__global__ void __launch_bounds__(kBlock, 2) k_conv_in(int n0, int n1, int n2, const float* __restrict__ x,
-                                                       const float* __restrict__ w, const float* __restrict__ b,
-                                                       bf16* __restrict__ out) {
+__global__ void __launch_bounds__(kBlock, 2) k_conv_in(int n0, int n1, int n2, int planes,
+                                                       const float* __restrict__ x, const float* __restrict__ w,
+                                                       const float* __restrict__ b, bf16* __restrict__ out) {
     constexpr int SK = kInK + 2, PL = (kInJ + 2) * SK, NL = (PL + kBlock - 1) / kBlock;
     __shared__ __align__(16) float sw[27 * 16 + 16];
     __shared__ float sx[4][PL];
     for (int q = threadIdx.x; q < 27 * 16; q += blockDim.x) sw[q] = w[q];
     if (threadIdx.x < 16) sw[27 * 16 + threadIdx.x] = b[threadIdx.x];
     const int k0 = blockIdx.x * kInK, j0 = blockIdx.y * kInJ;
-    const int is = blockIdx.z * kInI, ie = min(is + kInI, n0);
+    const int is = blockIdx.z * planes, ie = min(is + planes, n0);
     const long plane = (long)n1 * n2;
     // this thread's values of a plane: offset in the plane, -1 outside the grid
     long off[NL];
@@ -611,9 +611,23 @@ inline unsigned blocks_for(long n) { return (unsigned)((n + kBlock - 1) / kBlock
 
 cudaError_t conv_in_launch(int n0, int n1, int n2, const float* x, const float* w, const float* b, bf16* out,
                            cudaStream_t s) {
+    const long tiles = (long)((n2 + kInK - 1) / kInK) * ((n1 + kInJ - 1) / kInJ);
+    // planes a CTA: those it walks, and about two more of start-up, times the
+    // rounds of two CTAs an SM, at its least.  Eight on large grids; on small ones
+    // a march of eight leaves SMs idle (16^3 31.0 -> 7.5 us, 64^3 33.7 -> 11.2,
+    // 96^3 34.5 -> 31.0; a tile and plane a CTA without the ring took 10.5, 14.6, 43.3)
+    int planes = kInI;
+    long best = 0;
+    for (int p = kInI; p >= 1; --p) {
+        const long cost = (tiles * ((n0 + p - 1) / p) + 2 * kSms - 1) / (2 * kSms) * (p + 2);
+        if (!best || cost < best) {
+            best = cost;
+            planes = p;
+        }
+    }
     const dim3 grid((unsigned)((n2 + kInK - 1) / kInK), (unsigned)((n1 + kInJ - 1) / kInJ),
-                    (unsigned)((n0 + kInI - 1) / kInI));
-    k_conv_in<<<grid, kBlock, 0, s>>>(n0, n1, n2, x, w, b, out);
+                    (unsigned)((n0 + planes - 1) / planes));
+    k_conv_in<<<grid, kBlock, 0, s>>>(n0, n1, n2, planes, x, w, b, out);
     return cudaGetLastError();
 }
 

@@ -54,6 +54,9 @@ struct WgradArgs {
     int* err;
 };
 
+// SMs, for the rules that choose how much work a CTA takes
+constexpr int kSms = 148;
+
 // error code written to *err by a kernel that gave up waiting
 constexpr int kErrTimeout = 1;
 

@@ -108,3 +108,24 @@ def test_input_gradient_over_many_voxels(sign):
     chain = 32 + V // 32 // (nblocks * 32) + 2 + 8 + nblocks
     err = (dw.double() - torch.cat(sums).reshape(-1)).abs()
     assert bool((err <= chain * 2.0**-24 * torch.cat(sizes).reshape(-1)).all())
+
+
+@pytest.mark.parametrize("dims", [(13, 96, 320), (50, 130, 200), (130, 260, 250)])
+def test_input_convolution_over_several_planes(dims):
+    """2, 7 and 8 planes a thread block with a remainder: the march over planes,
+    which smaller grids do not take"""
+    from briscola_b200 import unet
+
+    L = unet.load()
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, w, b = (torch.randn(k, generator=g, device="cuda") for k in (dims, (27, 16), (16,)))
+    out = torch.zeros((*dims, 16), dtype=torch.bfloat16, device="cuda")
+    assert L.bun_conv_in(*dims, x.data_ptr(), w.data_ptr(), b.data_ptr(), out.data_ptr(), s) == 0
+    xp = torch.nn.functional.pad(x.double(), (1,) * 6)
+    for c in range(0, 16, 5):
+        ref = b[c].double() + sum(w[t, c].double() * xp[t // 9:t // 9 + dims[0], t // 3 % 3:t // 3 % 3 + dims[1],
+                                                        t % 3:t % 3 + dims[2]] for t in range(27))
+        ref = ref.clamp(min=0)
+        err = (out[..., c].double() - ref).norm(dim=(1, 2))  # plane by plane
+        assert bool((err <= 4e-3 * ref.norm(dim=(1, 2))).all())
