@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 // level's size, us before / now; two thirds of the time is the rows' supply and
 // the hand-over between the warps, not the MMAs):
 //   256^3  16 -> 16   663 /  592     48 -> 16   3359 / 1336
-//   128^3  96 -> 32  2869 /  442     32 -> 32   360 /  196    (16 -> 32: 145)
+//   128^3  96 -> 32  2869 /  442     32 -> 32   360 /  196     16 -> 32  132 / 121
 //    64^3  32 -> 64   119 /   47     64 -> 64    319 /   78   128 -> 64  589 / 139
 //    32^3  64 -> 64    50 /   21;  16^3 64 -> 64   30 /   17
 constexpr int kRowThreads = 288;
@@ -718,6 +718,7 @@ struct RowPlan {
     int P;       // distance of the planes' rows in the run
     int nvox;    // positions of the run: 2 P + 130
     int nr;      // rows of the ring
+    int nw;      // weight buffers: two, one where there is one group of channels
     int rows;    // rows j a CTA, at most JS
     int lk;      // log2 of the 8-channel chunks of a packed weight block
     int ntot;    // output channels, NOUT of them a CTA (blockIdx.y)
@@ -798,13 +799,13 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
 // (two CTAs of nine warps put five on one scheduler: at most 96 registers, the
 // bound for ten warps each; at 108 the second CTA stayed out, 840 -> 1445 us)
 template <int CG, int NOUT, int JS>
-__global__ void __launch_bounds__(kRowThreads + 32, NOUT == 16 ? 2 : 1) k_conv_rows(ConvArgs a, RowPlan R) {
+__global__ void __launch_bounds__(kRowThreads + 32, JS * NOUT <= 256 ? 2 : 1) k_conv_rows(ConvArgs a, RowPlan R) {
     using F = RowShape<CG, NOUT, JS>;
     constexpr int NQ = CG / 16;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int NR = R.nr;
     const uint32_t chunk = (uint32_t)R.nvox * 16, set_bytes = (CG / 8) * chunk;
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + NR * set_bytes + 2 * F::WBYTES);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + NR * set_bytes + R.nw * F::WBYTES);
     uint64_t* empty = full + kRowRing;
     uint64_t* wfull = empty + kRowRing;   // [2]
     uint64_t* wempty = wfull + 2;   // [2]
@@ -1008,22 +1009,29 @@ cudaError_t wgrad_rows(const WgradArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// the plan's extents of a run, and rows of a ring in `bytes` of shared memory
+template <int CG, int NOUT, int JS>
+int rows_ring(const ConvArgs& a, RowPlan& R, int bytes) {
+    R.stream = a.n2 % kTile != 0;
+    R.P = R.stream ? a.n2 + 1 : kTile + 2;
+    R.nvox = 2 * R.P + kTile + 2;
+    R.nw = std::min(2, (a.in.c0 + a.in.c1) / CG);
+    const int fixed = R.nw * RowShape<CG, NOUT, JS>::WBYTES + RowShape<CG, NOUT, JS>::BARS;
+    return std::min(kRowRing, (bytes - fixed) / ((CG / 8) * R.nvox * 16));
+}
+constexpr int kRowsTwo = 113 * 1024, kRowsOne = 227 * 1024;  // shared memory of a CTA, two and one an SM
+
 template <int CG, int NOUT, int JS>
 cudaError_t rows_inst(const ConvArgs& a, int kc, int parts, cudaStream_t s) {
     using F = RowShape<CG, NOUT, JS>;
     RowPlan R;
     R.lk = kc == 64 ? 3 : kc == 32 ? 2 : 1;
     R.ntot = NOUT * parts;
-    R.stream = a.n2 % kTile != 0;
-    R.P = R.stream ? a.n2 + 1 : kTile + 2;
-    R.nvox = 2 * R.P + kTile + 2;
-    const int set = (CG / 8) * R.nvox * 16, fixed = 2 * F::WBYTES + F::BARS;
     // as deep a ring as fits: two CTAs an SM where their accumulators do
-    const int room = (F::NCOLS == 256 ? 113 : 227) * 1024 - fixed;
-    R.nr = std::min(kRowRing, room / set);
-    if (R.nr < 2) R.nr = std::min(kRowRing, (227 * 1024 - fixed) / set);
+    R.nr = rows_ring<CG, NOUT, JS>(a, R, F::NCOLS == 256 ? kRowsTwo : kRowsOne);
+    if (R.nr < 2) R.nr = rows_ring<CG, NOUT, JS>(a, R, kRowsOne);
     if (R.nr < 1) return cudaErrorInvalidValue;
-    const int smem = R.nr * set + fixed;
+    const int smem = R.nr * (CG / 8) * R.nvox * 16 + R.nw * F::WBYTES + F::BARS;
     cudaError_t e = cudaFuncSetAttribute(k_conv_rows<CG, NOUT, JS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const long tiles = R.stream ? ((long)a.n0 * R.P + kTile - 1) / kTile : (long)a.n0 * (a.n2 / kTile);
@@ -1056,17 +1064,29 @@ bool rows_supported(int cin, int nout, int n2) {
     return out && cin % 16 == 0 && cin <= 256 && (n2 % kTile == 0 || n2 <= 256);
 }
 
-// Rows a CTA: 16 of 16 output channels (256 columns of tensor memory, two CTAs
-// an SM), 16 of 32, 10 of 48 and 8 of 64 (all of it).  Groups of 32 input
-// channels where both weight buffers leave room for a ring.
+// 48 output channels, parts of them: 5 rows a CTA where two CTAs fit an SM, else 10
+cudaError_t rows48(const ConvArgs& a, int kc, int parts, cudaStream_t s) {
+    RowPlan R;
+    return rows_ring<16, 48, 5>(a, R, kRowsTwo) >= 2 ? rows_inst<16, 48, 5>(a, kc, parts, s)
+                                                     : rows_inst<16, 48, 10>(a, kc, parts, s);
+}
+
+// Rows a CTA: 16 of 16 output channels, 8 of 32 and 5 of 48 (256 columns of
+// tensor memory each: two CTAs an SM, one's start and end under the other's
+// rows), 8 of 64, and of 32 from groups of 32 input channels 16 (all of it).  With
+// one CTA an SM, 16 rows of 32 and 10 of 48, 16 -> 32 at 128^3 took 144 us
+// (now 121; a tap an MMA 132) and 16 -> 48 197 (155; 133); 32 -> 96 at 64^3 86 (64).
+// 10 rows of 48 stay where the weights leave two CTAs no ring: 32 -> 48 on
+// 40 x 24 x 200 40 us against 47.  Groups of 32 input channels where both weight
+// buffers leave room for a ring.
 cudaError_t rows_launch(const ConvArgs& a, int kc, int nout, cudaStream_t s) {
     const int cin = a.in.c0 + a.in.c1;
     if (nout == 16) return rows_inst<16, 16, 16>(a, kc, 1, s);
-    if (nout == 32) return cin % 32 || (a.n2 % kTile && a.n2 > kTile) ? rows_inst<16, 32, 16>(a, kc, 1, s)
+    if (nout == 32) return cin % 32 || (a.n2 % kTile && a.n2 > kTile) ? rows_inst<16, 32, 8>(a, kc, 1, s)
                                                                      : rows_inst<32, 32, 16>(a, kc, 1, s);
-    if (nout == 48) return rows_inst<16, 48, 10>(a, kc, 1, s);
+    if (nout == 48) return rows48(a, kc, 1, s);
     if (nout == 64) return rows_inst<16, 64, 8>(a, kc, 1, s);
-    if (nout == 96) return rows_inst<16, 48, 10>(a, kc, 2, s);
+    if (nout == 96) return rows48(a, kc, 2, s);
     if (nout == 128) return rows_inst<16, 64, 8>(a, kc, 2, s);
     return cudaErrorInvalidValue;
 }

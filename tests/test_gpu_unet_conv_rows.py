@@ -38,6 +38,11 @@ CASES = [
     ((2, 2, 24), 256, 0, 0, 16),
     ((2, 11, 64), 32, 0, 0, 96),   # two halves of the output channels
     ((1, 9, 128), 64, 0, 0, 128),
+    ((1, 6, 128), 16, 0, 0, 48),   # 48 channels: one weight buffer, a CTA of 5 rows and one of 1
+    ((2, 10, 188), 32, 0, 0, 48),  # the longest rows that leave two CTAs an SM their rings
+    ((1, 10, 189), 32, 0, 0, 48),  # and longer ones: 10 rows a CTA
+    ((2, 6, 250), 32, 0, 0, 96),
+    ((2, 9, 256), 48, 0, 0, 32),   # 8 rows of 32 channels a CTA and one more
 ]
 
 
