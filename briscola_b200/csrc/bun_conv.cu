@@ -1129,7 +1129,13 @@ cudaError_t wgrad_launch(const WgradArgs& a, int cout, cudaStream_t s) {
     // rows in whole steps of 16 voxels (an MMA's K) and channels in whole blocks
     // of 16; a row's 8 channels must come from one source
     const int cin = a.in.c0 + a.in.c1;
-    if (a.n2 % 16 == 0 && cin % 16 == 0 && a.in.c0 % 8 == 0) {
+    // and blocks of rows that are filled: a block's MMAs are those of W =
+    // 128 / cout rows, whatever it holds.  Below 24 whole voxel columns of it the
+    // gather was faster or equal (64 x 1 x 128, 16 -> 16: 14.7 against 20.8 us;
+    // 128 x 2 x 32 14.6 against 20.8), above it the rows (128 x 4 x 128, 39.2
+    // against 31.0), unless the grid has W rows (128 x 16 x 16, 29.0 against 27.0)
+    const bool filled = a.n1 * cout >= 128 || (long)a.n1 * std::min(a.n2, kWgVox) * cout >= 24 * 128;
+    if (filled && a.n2 % 16 == 0 && cin % 16 == 0 && a.in.c0 % 8 == 0) {
         if (cout == 16) return wgrad_rows<16>(a, s);
         if (cout == 32) return wgrad_rows<32>(a, s);
         if (cout == 64) return wgrad_rows<64>(a, s);

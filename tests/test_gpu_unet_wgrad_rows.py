@@ -33,6 +33,10 @@ CASES = [
     ((2, 5, 32), 48, 0, 0, 64, 2),
     ((4, 6, 32), 64, 1, 64, 64, 3),
     ((3, 7, 144), 80, 0, 0, 32, 2),
+    ((2, 2, 80), 16, 0, 0, 16, 2),     # too few rows for a block: the gather
+    ((2, 2, 96), 16, 0, 0, 16, 2),     # rows long enough for a part of one
+    ((3, 1, 80), 32, 0, 0, 32, 1),
+    ((3, 1, 96), 32, 0, 0, 32, 1),
 ]
 
 
