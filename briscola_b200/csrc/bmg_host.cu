@@ -358,7 +358,7 @@ Bricks<T> bricks(const bmg_ctx* c, int l) {
         v.cpar = K.cpar;
         v.kh = H.ks ? K.n[2] / 2 : 0;
         v.mask = c->multi && !c->userLambda;
-        v.gmap = H.gmap;
+        v.gmap = v.mask ? H.gmap : nullptr;
         // a smoothed coarse level of a singular system keeps global cell 0
         // (brick 0's first cell) at zero
         v.pin = l == c->lc && b == 0 && c->singular && c->opt.coarse_mode == BMG_COARSE_SMOOTH;
@@ -1302,8 +1302,9 @@ void smooth(bmg_ctx* c, int l, int sweeps) {
         }
         return;
     }
-    // (several bricks: the passes read their neighbours through gmap)
     for (int col : seq) {
+        // (without the user's coefficients the passes read other bricks through gmap)
+        if (!B.v[0].gmap) exchange<T>(c, l);
         c->launches += 1;
         if (c->variable)
             launch_colour_pass<T, true>(B, col, s, zeroFirst);

@@ -105,11 +105,11 @@ struct LevelView {
     int pin;           // smoothers keep cell (0,0,0) at zero: the singularity pin
                        // of an iteratively smoothed coarse level (solver.C:201-231)
     int mask;          // the face arrays are 1 but on the brick's outer faces (the
-                       // contact mask of a constant coefficient): only cells there
-                       // read them
-    const int* gmap;   // multi-brick levels: for a ghost cell's slab index, the cell
-                       // that it copies (itself beyond a Dirichlet face); the colour
-                       // passes read through it, so they need no ghost refresh
+                       // contact mask of a constant coefficient)
+    const int* gmap;   // several bricks without the user's coefficients: for a ghost
+                       // cell's slab index, the cell that it copies (itself beyond a
+                       // Dirichlet face); the colour passes read through it, so they
+                       // need no ghost refresh
     int kh;            // parity-split rows: offset n2/2 of the odd-k half (see
                        // above); 0: natural k order
 };
@@ -143,6 +143,12 @@ struct Bricks {
     int nb;
     int max1, max2;          // largest n1 and n2 (grid extents)
 };
+
+// The coefficient a kernel is compiled for: constant, face arrays, or face
+// arrays that are a mask.  (One instance for the last two, deciding at run time,
+// held more registers and waited for one coefficient after the other: W cycles
+// of one brick with face coefficients took up to 1.37 times as long.)
+enum { C_CONST = 0, C_FACES = 1, C_MASK = 2 };
 
 // Transfer tables between level l (fine) and l+1 (coarse), fine-indexed.
 struct TransferTabs {

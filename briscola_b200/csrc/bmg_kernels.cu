@@ -36,8 +36,10 @@ struct Pair<double> {
 // Neighbour rows and planes are read as whole pairs (8/16-byte loads), so a
 // warp's loads fill every L1 wavefront; the k neighbour outside the pair is
 // one scalar load.
+// ACROSS: the neighbours in other bricks are read through gmap; otherwise the
+// ghosts hold them (refreshed before the pass where there are other bricks).
 // ---------------------------------------------------------------------------
-template <typename T, bool VAR>
+template <typename T, int COEF, bool ACROSS>
 __global__ void __launch_bounds__(256) k_colour_pass(Bricks<T> B, int colour) {
     grid_dep_sync();
     using V2 = typename Pair<T>::type;
@@ -61,10 +63,10 @@ __global__ void __launch_bounds__(256) k_colour_pass(Bricks<T> B, int colour) {
     const long c = r + k;
     if (L.pin && (i | j | k) == 0) return;  // the pinned cell stays zero
     T w[6];
-    couplings<T, VAR>(L, i, j, k, c, c + 1, w);  // natural rows only (n2 % 4 != 0)
+    couplings<T, COEF>(L, i, j, k, c, c + 1, w);  // natural rows only (n2 % 4 != 0)
     T xn[6] = {e ? xm.y : xm.x, e ? xp.y : xp.x, e ? ym.y : ym.x, e ? yp.y : yp.x,
                e ? own.x : x[c0 - 1], e ? x[c0 + 2] : own.y};
-    if (L.gmap) {  // neighbours in other bricks
+    if (ACROSS) {
         if (i == 0) xn[0] = x[ldg(L.gmap + c - L.si)];
         if (i == L.n0 - 1) xn[1] = x[ldg(L.gmap + c + L.si)];
         if (j == 0) xn[2] = x[ldg(L.gmap + c - L.sj)];
@@ -190,7 +192,7 @@ __device__ __forceinline__ void stq<double>(double* p, int kh, const double v[4]
 // brick's n2 % 4 == 0 and natural rows (parity-split levels take
 // k_colour_split).
 // ---------------------------------------------------------------------------
-template <typename T, bool VAR>
+template <typename T, int COEF, bool ACROSS>
 __device__ __forceinline__ void colour_quad_item(const LevelView<T>& L, int i, int j, int p, int colour) {
     const int k0 = 4 * p;
     const int c = cell32(L, i, j, k0), si = (int)L.si, sj = (int)L.sj;
@@ -212,7 +214,7 @@ __device__ __forceinline__ void colour_quad_item(const LevelView<T>& L, int i, i
     // below is a compile-time constant picked by a select
     const bool odd = ((colour ^ (i + j + k0 + L.cpar)) & 1) != 0;
 #define BMG_SEL(a, e) (odd ? a[(e) + 1] : a[e])
-    if (L.gmap) {  // neighbours in other bricks, of the two cells of the colour
+    if (ACROSS) {  // of the two cells of the colour
         auto across = [&](T v[4], int at) {
             const T a = x[ldg(L.gmap + at + (odd ? 1 : 0))], b = x[ldg(L.gmap + at + (odd ? 3 : 2))];
             v[0] = v[1] = a;
@@ -227,8 +229,7 @@ __device__ __forceinline__ void colour_quad_item(const LevelView<T>& L, int i, i
     }
     T w0[6] = {wil, wih, wjl, wjh, BMG_SEL(wkl, 0), BMG_SEL(wkh, 0)};
     T w2[6] = {wil, wih, wjl, wjh, BMG_SEL(wkl, 2), BMG_SEL(wkh, 2)};
-    if (VAR && L.mask) {
-        // 1 but on the brick's outer faces
+    if (COEF == C_MASK) {
         const int o = odd ? 1 : 0;
         if (i == 0) {
             w0[0] *= ldg(L.lam0 + c + o);
@@ -248,7 +249,8 @@ __device__ __forceinline__ void colour_quad_item(const LevelView<T>& L, int i, i
         }
         if (k0 == 0 && !odd) w0[4] *= ldg(L.lam2 + c);
         if (k0 + 4 == L.n2 && odd) w2[5] *= ldg(L.lam2 + c + 4);
-    } else if (VAR) {
+    }
+    if (COEF == C_FACES) {
         T l0[4], l0p[4], l1[4], l1p[4], l2[4];
         Row4<T>::ldg4(L.lam0 + c, l0);
         Row4<T>::ldg4(L.lam0 + c + si, l0p);
@@ -287,7 +289,7 @@ __device__ __forceinline__ void colour_quad_item(const LevelView<T>& L, int i, i
     }
 }
 
-template <typename T, bool VAR>
+template <typename T, int COEF, bool ACROSS>
 __global__ void __launch_bounds__(256) k_colour_quad(Bricks<T> B, int colour) {
     grid_dep_sync();
     int i;
@@ -295,7 +297,7 @@ __global__ void __launch_bounds__(256) k_colour_quad(Bricks<T> B, int colour) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (j >= L.n1 || 4 * p >= L.n2) return;
-    colour_quad_item<T, VAR>(L, i, j, p, colour);
+    colour_quad_item<T, COEF, ACROSS>(L, i, j, p, colour);
 }
 
 // ---------------------------------------------------------------------------
@@ -643,7 +645,7 @@ __global__ void __launch_bounds__(256) k_prolong_quad(Bricks<T> FB, Bricks<T> CB
     prolong_quad_item<T>(FB.v[b], CB.v[b], ts.t[b], i, j, p);
 }
 
-template <typename T, bool VAR>
+template <typename T, int COEF>
 __device__ __forceinline__ void restrict_quad_item(const LevelView<T>& F, const LevelView<T>& C,
                                                    const TransferTabs& t, int I, int J, int P) {
     const int K0 = 2 * P;  // the thread's coarse k-pair
@@ -681,22 +683,29 @@ __device__ __forceinline__ void restrict_quad_item(const LevelView<T>& F, const 
             const int cl = row + kpos(F, k0 - 1), cr = row + kpos(F, k0 + 4);
             const T left = F.x[cl], right = F.x[cr];
             T l0[4], l0p[4], l1[4], l1p[4], l2[4], l2r = T(1);
-            if (VAR) {
-                const bool all = !F.mask;  // else 1 but on the brick's outer faces
+            if (COEF == C_FACES) {
+                ldgq(F.lam0 + c, kh, l0);
+                ldgq(F.lam0 + c + si, kh, l0p);
+                ldgq(F.lam1 + c, kh, l1);
+                ldgq(F.lam1 + c + sj, kh, l1p);
+                ldgq(F.lam2 + c, kh, l2);
+                l2r = ldg(F.lam2 + cr);
+            }
+            if (COEF == C_MASK) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) l0[q] = l0p[q] = l1[q] = l1p[q] = l2[q] = T(1);
-                if (all || i == 0) ldgq(F.lam0 + c, kh, l0);
-                if (all || i == F.n0 - 1) ldgq(F.lam0 + c + si, kh, l0p);
-                if (all || j == 0) ldgq(F.lam1 + c, kh, l1);
-                if (all || j == F.n1 - 1) ldgq(F.lam1 + c + sj, kh, l1p);
-                if (all || k0 == 0) ldgq(F.lam2 + c, kh, l2);
-                if (all || k0 + 4 == F.n2) l2r = ldg(F.lam2 + cr);
+                if (i == 0) ldgq(F.lam0 + c, kh, l0);
+                if (i == F.n0 - 1) ldgq(F.lam0 + c + si, kh, l0p);
+                if (j == 0) ldgq(F.lam1 + c, kh, l1);
+                if (j == F.n1 - 1) ldgq(F.lam1 + c + sj, kh, l1p);
+                if (k0 == 0) ldgq(F.lam2 + c, kh, l2);
+                if (k0 + 4 == F.n2) l2r = ldg(F.lam2 + cr);
             }
             T r[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 T w[6] = {wil, wih, wjl, wjh, wkl[q], wkh[q]};
-                if (VAR) {
+                if (COEF != C_CONST) {
                     w[0] *= l0[q];
                     w[1] *= l0p[q];
                     w[2] *= l1[q];
@@ -717,7 +726,7 @@ __device__ __forceinline__ void restrict_quad_item(const LevelView<T>& F, const 
     C.b[cell32(C, I, J, K0 + 1)] = acc1;
 }
 
-template <typename T, bool VAR>
+template <typename T, int COEF>
 __global__ void __launch_bounds__(256) k_restrict_quad(Bricks<T> FB, Bricks<T> CB, TransferSet ts) {
     grid_dep_sync();
     int I;
@@ -725,7 +734,7 @@ __global__ void __launch_bounds__(256) k_restrict_quad(Bricks<T> FB, Bricks<T> C
     const int P = blockIdx.x * blockDim.x + threadIdx.x;
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
     if (J >= CB.v[b].n1 || 2 * P >= CB.v[b].n2) return;
-    restrict_quad_item<T, VAR>(FB.v[b], CB.v[b], ts.t[b], I, J, P);
+    restrict_quad_item<T, COEF>(FB.v[b], CB.v[b], ts.t[b], I, J, P);
 }
 
 // ---------------------------------------------------------------------------
@@ -1063,7 +1072,7 @@ __global__ void __launch_bounds__(256) k_residual_out(Bricks<T> B, double* out) 
 // the level-0 operator vanish (every coupling is paired with the centre)
 // except in the rows of Dirichlet faces.
 // ---------------------------------------------------------------------------
-template <bool VAR>
+template <int COEF>
 __global__ void __launch_bounds__(kReduceThreads) k_residual_norm(Bricks<double> B, Walls W, int mode,
                                                                   double* partials, long nblocks, float* b32) {
     grid_dep_sync();
@@ -1078,7 +1087,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_residual_norm(Bricks<double>
         const long row = row_at(L, i, j), c = row + kpos(L, k);
         double w[6];
         const long ckm = row + kpos(L, k - 1), ckp = row + kpos(L, k + 1);
-        couplings<double, VAR>(L, i, j, k, c, ckp, w);
+        couplings<double, COEF>(L, i, j, k, c, ckp, w);
         const double xn[6] = {L.x[c - L.si], L.x[c + L.si], L.x[c - L.sj], L.x[c + L.sj], L.x[ckm], L.x[ckp]};
         const double r = res_value(w, xn, L.x[c], L.b[c]);
         const double V = L.tab64[L.to.h[0] + i] * L.tab64[L.to.h[1] + j] * L.tab64[L.to.h[2] + k];
@@ -1322,21 +1331,34 @@ void launch_colour_pass(const Bricks<T>& B, int colour, cudaStream_t s, bool zer
             launch_k(k_colour_split<T, VAR, false>, grid, blk, 0, s, L, colour);
         return;
     }
+    // face arrays without the user's coefficients are a mask
+    constexpr int MASK = VAR ? C_MASK : C_CONST;
+    const bool across = B.v[0].gmap != nullptr;
     bool quads = true;
     for (int b = 0; b < B.nb; ++b) quads = quads && B.v[b].n2 % 4 == 0;
     if (quads) {
         // one row per thread: two rows per thread (R = 2) measured no faster
         // on the 256^3 level and costs registers in FP64
         // several bricks: runs of 8 quads (128 bytes of FP32), which bricks of
-        // different row lengths all fill
+        // different row lengths all fill (the seven-brick mesh, four cycles:
+        // mixed 2590 us, 2890 with 32 quads; FP64 3119, 3480)
         const int nq = B.max2 / 4;
-        const dim3 blk = nq >= 32 && B.nb == 1 ? dim3(32, 8, 1) : nq >= 8 ? dim3(8, 32, 1) : dim3(2, 128, 1);
-        launch_k(k_colour_quad<T, VAR>, grid_for(B, nq, blk), blk, 0, s, B, colour);
+        // rows of fewer than 8 quads on one brick: whole rows, in small blocks that
+        // spread over the SMs (192 x 192 x 24, four V cycles without the fused
+        // smoother: FP64 1064 us with blocks of 2 x 128, 979 with 256 threads of
+        // whole rows, 915 with 64; 48 x 96 x 12 417, 412, 393)
+        const dim3 blk = nq >= 32 && B.nb == 1 ? dim3(32, 8, 1)
+                         : nq >= 8             ? dim3(8, 32, 1)
+                         : B.nb == 1           ? dim3(nq, 64 / nq, 1)
+                                               : dim3(2, 128, 1);
+        launch_k(across ? k_colour_quad<T, MASK, true> : k_colour_quad<T, VAR, false>, grid_for(B, nq, blk), blk, 0, s, B,
+                 colour);
         return;
     }
     const int pairs = (B.max2 + 1) / 2;
     const dim3 blk = pairs >= 32 ? dim3(32, 8, 1) : pairs >= 8 ? dim3(8, 32, 1) : dim3(2, 128, 1);
-    launch_k(k_colour_pass<T, VAR>, grid_for(B, pairs, blk), blk, 0, s, B, colour);
+    launch_k(across ? k_colour_pass<T, MASK, true> : k_colour_pass<T, VAR, false>, grid_for(B, pairs, blk), blk, 0, s, B,
+             colour);
 }
 
 template <typename T, bool VAR>
@@ -1380,7 +1402,8 @@ void launch_residual_restrict(const Bricks<T>& F, const Bricks<T>& C, const Tran
     if (quad_transfers(F, t)) {
         const int np = C.max2 / 2;
         const dim3 blk = np >= 32 ? dim3(32, 8, 1) : np >= 8 ? dim3(8, 32, 1) : dim3(2, 128, 1);
-        launch_k(k_restrict_quad<T, VAR>, grid_for(C, np, blk), blk, 0, s, F, C, t);
+        launch_k(F.v[0].mask ? k_restrict_quad<T, VAR ? C_MASK : C_CONST> : k_restrict_quad<T, VAR>, grid_for(C, np, blk), blk,
+                 0, s, F, C, t);
         return;
     }
     const dim3 blk = block_for(C.max2);
@@ -1429,7 +1452,8 @@ long launch_residual_norm(const Bricks<double>& B, const Walls& W, int mode, dou
                           cudaStream_t s) {
     if (B.v[0].kh) return launch_residual_split<VAR>(B, W, mode, nullptr, b32, nullptr, partials, s);
     const dim3 blk = block_for(B.max2);
-    launch_k(k_residual_norm<VAR>, grid_for(B, B.max2, blk), blk, 0, s, B, W, mode, partials, reduce_blocks(B), b32);
+    launch_k(B.v[0].mask ? k_residual_norm<VAR ? C_MASK : C_CONST> : k_residual_norm<VAR>, grid_for(B, B.max2, blk), blk, 0,
+             s, B, W, mode, partials, reduce_blocks(B), b32);
     return reduce_blocks(B);
 }
 

@@ -35,7 +35,7 @@ __device__ __forceinline__ double cell_volume(const LevelView<double>& L, int i,
 
 // r = b - A'x (FP64), written to r and to the cycle's right-hand side;
 // partials: ||V r||^2 and, for mode 0, the normFactor sum (as k_residual_norm)
-template <bool VAR>
+template <int COEF>
 __global__ void __launch_bounds__(kReduceThreads) k_fcg_residual(Bricks<double> B, Walls W, int mode, double* r_out,
                                                                  float* pre32, double* pre64, double* partials,
                                                                  long nblocks) {
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_residual(Bricks<double> 
         const long row = row_at(L, i, j), c = row + kpos(L, k);
         double w[6];
         const long ckm = row + kpos(L, k - 1), ckp = row + kpos(L, k + 1);
-        couplings<double, VAR>(L, i, j, k, c, ckp, w);
+        couplings<double, COEF>(L, i, j, k, c, ckp, w);
         const double xn[6] = {L.x[c - L.si], L.x[c + L.si], L.x[c - L.sj], L.x[c + L.sj], L.x[ckm], L.x[ckp]};
         const double r = res_value(w, xn, L.x[c], L.b[c]);
         const double V = cell_volume(L, i, j, k);
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kFinalThreads) k_fcg_beta(const double* partia
 }
 
 // p = z + beta p, q = A'z + beta q; partials of (p, V q)
-template <typename T, bool VAR>
+template <typename T, int COEF>
 __global__ void __launch_bounds__(kReduceThreads) k_fcg_direction(Bricks<double> B, const T* z, double* p,
                                                                   double* q, double* partials,
                                                                   const SolveState* st) {
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_direction(Bricks<double>
         const long row = row_at(L, i, j), c = row + kpos(L, k);
         double w[6];
         const long ckm = row + kpos(L, k - 1), ckp = row + kpos(L, k + 1);
-        couplings<double, VAR>(L, i, j, k, c, ckp, w);
+        couplings<double, COEF>(L, i, j, k, c, ckp, w);
         const double zc = (double)z[c];
         const double s = w[0] * (double)z[c - L.si] + w[1] * (double)z[c + L.si] + w[2] * (double)z[c - L.sj] +
                          w[3] * (double)z[c + L.sj] + w[4] * (double)z[ckm] + w[5] * (double)z[ckp];
@@ -302,7 +302,7 @@ struct Quad4<float> {
     double Az[4];                                                                                      \
     for (int e = 0; e < 4; ++e) {                                                                       \
         double w[6];                                                                                    \
-        couplings<double, VAR>(L, i, j, k0 + e, c + quad_off(ks, e), e < 3 ? c + quad_off(ks, e + 1) : cr_, w); \
+        couplings<double, COEF>(L, i, j, k0 + e, c + quad_off(ks, e), e < 3 ? c + quad_off(ks, e + 1) : cr_, w); \
         const double km = e > 0 ? (double)zc[e - 1] : (double)zl_;                                      \
         const double kp = e < 3 ? (double)zc[e + 1] : (double)zr_;                                      \
         const double sv = w[0] * (double)zim_[e] + w[1] * (double)zip_[e] + w[2] * (double)zjm_[e] +     \
@@ -311,7 +311,7 @@ struct Quad4<float> {
         Az[e] = sv - d * (double)zc[e];                                                                 \
     }
 
-template <typename T, bool VAR>
+template <typename T, int COEF>
 __global__ void __launch_bounds__(kReduceThreads) k_fcg_dots3_4(Bricks<double> B, const T* z, const double* r,
                                                                 const double* q, double* partials, long nblocks) {
     grid_dep_sync();
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_dots3_4(Bricks<double> B
     }
 }
 
-template <typename T, bool VAR>
+template <typename T, int COEF>
 __global__ void __launch_bounds__(kReduceThreads) k_fcg_step4(Bricks<double> B, const T* z, double* p, double* q,
                                                               double* r, float* pre32, double* pre64,
                                                               double* partials, const SolveState* st) {
@@ -718,7 +718,7 @@ long launch_fcg_residual(const Bricks<double>& B, const Walls& W, int mode, doub
                          double* partials, cudaStream_t s) {
     if (B.v[0].kh) return launch_residual_split<VAR>(B, W, mode, r, pre32, pre64, partials, s);
     const dim3 blk = block_for(B.max2);
-    launch_k(k_fcg_residual<VAR>, grid_for(B, B.max2, blk), blk, 0, s, B, W, mode, r, pre32, pre64, partials,
+    launch_k(B.v[0].mask ? k_fcg_residual<VAR ? C_MASK : C_CONST> : k_fcg_residual<VAR>, grid_for(B, B.max2, blk), blk, 0, s, B, W, mode, r, pre32, pre64, partials,
                                                                    reduce_blocks(B));
     return reduce_blocks(B);
 }
@@ -726,6 +726,7 @@ long launch_fcg_residual(const Bricks<double>& B, const Walls& W, int mode, doub
 template <typename T, bool VAR>
 void launch_fcg_step(const Bricks<double>& B, const T* z, double* p, double* q, double* r, float* pre32,
                      double* pre64, double* partials, SolveState* st, cudaStream_t s) {
+    constexpr int MASK = VAR ? C_MASK : C_CONST;
     const long nb = fcg_partials(B);
     if (fcg_quads(B)) {
         // two passes and one reduction (k_fcg_coeffs)
@@ -733,12 +734,12 @@ void launch_fcg_step(const Bricks<double>& B, const T* z, double* p, double* q, 
         if (B.v[0].kh)
             launch_k(k_fcg_dots3_split<T, VAR>, g, blk, 0, s, B, z, r, q, partials, nb);
         else
-            launch_k(k_fcg_dots3_4<T, VAR>, g, blk, 0, s, B, z, r, q, partials, nb);
+            launch_k(B.v[0].mask ? k_fcg_dots3_4<T, MASK> : k_fcg_dots3_4<T, VAR>, g, blk, 0, s, B, z, r, q, partials, nb);
         launch_k(k_fcg_coeffs, 1, kFinalThreads, 0, s, partials, nb, st);
         if (B.v[0].kh)
             launch_k(k_fcg_step_split<T, VAR>, g, blk, 0, s, B, z, p, q, r, pre32, pre64, partials, st);
         else
-            launch_k(k_fcg_step4<T, VAR>, g, blk, 0, s, B, z, p, q, r, pre32, pre64, partials, st);
+            launch_k(B.v[0].mask ? k_fcg_step4<T, MASK> : k_fcg_step4<T, VAR>, g, blk, 0, s, B, z, p, q, r, pre32, pre64, partials, st);
         return;
     }
     // rows of n2 % 4 != 0: one cell per thread, three passes
@@ -746,7 +747,7 @@ void launch_fcg_step(const Bricks<double>& B, const T* z, double* p, double* q, 
     const dim3 g = grid_for(B, B.max2, blk);
     launch_k(k_fcg_dots<T>, g, blk, 0, s, B, z, r, q, partials, nb);
     launch_k(k_fcg_beta, 1, kFinalThreads, 0, s, partials, nb, st);
-    launch_k(k_fcg_direction<T, VAR>, g, blk, 0, s, B, z, p, q, partials, st);
+    launch_k(B.v[0].mask ? k_fcg_direction<T, MASK> : k_fcg_direction<T, VAR>, g, blk, 0, s, B, z, p, q, partials, st);
     launch_k(k_fcg_alpha, 1, kFinalThreads, 0, s, partials, nb, st);
     launch_k(k_fcg_update, g, blk, 0, s, B, p, r, q, pre32, pre64, partials, st);
 }

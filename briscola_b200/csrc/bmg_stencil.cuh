@@ -29,7 +29,10 @@ __device__ __forceinline__ int kpos(const LevelView<T>& L, int k) {
 // :96-102), i.e. axis 0 lower/upper, axis 1 lower/upper, axis 2 lower/upper.
 // c is the cell's slab index, ckp the slab index of cell (i,j,k+1), whose
 // lower face is the cell's upper k face.
-template <typename T, bool VAR>
+// COEF: the coefficient, constant (C_CONST), the face arrays (C_FACES), or face
+// arrays that are 1 but on the brick's outer faces (C_MASK, LevelView::mask: only
+// cells there read them).
+template <typename T, int COEF>
 __device__ __forceinline__ void couplings(const LevelView<T>& L, int i, int j, int k, long c, long ckp,
                                           T w[6]) {
     w[0] = ldg(L.tab + L.to.wl[0] + i);
@@ -38,14 +41,21 @@ __device__ __forceinline__ void couplings(const LevelView<T>& L, int i, int j, i
     w[3] = ldg(L.tab + L.to.wh[1] + j);
     w[4] = ldg(L.tab + L.to.wl[2] + k);
     w[5] = ldg(L.tab + L.to.wh[2] + k);
-    if (VAR) {
-        const bool all = !L.mask;  // else only the brick's outer faces differ from 1
-        if (all || i == 0) w[0] *= ldg(L.lam0 + c);
-        if (all || i == L.n0 - 1) w[1] *= ldg(L.lam0 + c + L.si);
-        if (all || j == 0) w[2] *= ldg(L.lam1 + c);
-        if (all || j == L.n1 - 1) w[3] *= ldg(L.lam1 + c + L.sj);
-        if (all || k == 0) w[4] *= ldg(L.lam2 + c);
-        if (all || k == L.n2 - 1) w[5] *= ldg(L.lam2 + ckp);
+    if (COEF == C_FACES) {
+        w[0] *= ldg(L.lam0 + c);
+        w[1] *= ldg(L.lam0 + c + L.si);
+        w[2] *= ldg(L.lam1 + c);
+        w[3] *= ldg(L.lam1 + c + L.sj);
+        w[4] *= ldg(L.lam2 + c);
+        w[5] *= ldg(L.lam2 + ckp);
+    }
+    if (COEF == C_MASK) {
+        if (i == 0) w[0] *= ldg(L.lam0 + c);
+        if (i == L.n0 - 1) w[1] *= ldg(L.lam0 + c + L.si);
+        if (j == 0) w[2] *= ldg(L.lam1 + c);
+        if (j == L.n1 - 1) w[3] *= ldg(L.lam1 + c + L.sj);
+        if (k == 0) w[4] *= ldg(L.lam2 + c);
+        if (k == L.n2 - 1) w[5] *= ldg(L.lam2 + ckp);
     }
 }
 
