@@ -9,7 +9,7 @@
 // F cycle) comes from the host as a list.
 //
 // What bounds it: the number of dependent passes times the latency of one
-// (shared loads, seven multiply-adds, a division, the barrier), and on the
+// (shared loads, a chain of multiply-adds, the barrier), and on the
 // larger levels the shared-memory bandwidth of one SM (13 loads an update).
 // So levels above kTailGather cells are spread over the CTAs of the cluster,
 // whole i-planes each, one cell update per thread and pass; a CTA pushes the
@@ -29,7 +29,10 @@
 // whatever n2 is), so a colour pass reads and writes consecutive words.  Per
 // cell the arithmetic and its order are those of the per-pass kernels
 // (gs_value, restrict_quad_item / k_residual_restrict, prolong_quad_item /
-// k_prolong_correct, coarse_solve_block), so the results are bit-identical.
+// k_prolong_correct, coarse_solve_block).  gs_value is shared and rounds
+// explicitly; the transfers are written out here again, and that the compiler
+// contracts both copies alike is a tested property: whole solves are
+// bit-identical (tests/test_gpu_tail.py, tests/test_gpu_cluster_tail.py).
 
 #include <cooperative_groups.h>
 

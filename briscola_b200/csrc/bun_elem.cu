@@ -2,9 +2,9 @@
 // convolution and the 1x1x1 output head (too narrow for a tensor-core tile),
 // pooling and its gradients, the loss, weight packing for the tensor-core
 // convolutions, Adam, and the scalings between the solver's FP64 fields and
-// the network's FP32 input/output.  All of them are bandwidth-trivial next
-// to the 3x3x3 convolutions; reductions write one partial per block and are
-// added in a fixed order.
+// the network's FP32 input/output.  Most are a pass over memory; the input layer
+// is bound by its multiply-adds (8 % of a forward pass at 256^3).  Reductions
+// write one partial per block and are added in a fixed order.
 
 #include "bun_api_internal.h"
 

@@ -2,7 +2,8 @@
 oracle's restatement: the paired transforms (bfft_pair.cu) at every length
 they take, with line counts that leave a last tile nearly empty and rows whose
 lines are not adjacent pairs, and the tridiagonal solves (bfft_tri.cu) around
-the chunk sizes, for a line per thread block and beyond the longest."""
+the chunk sizes, for a line per thread block and beyond the longest of them
+(2048 rows; longer lines are marched by a thread each, bfft.cu)."""
 import numpy as np
 import pytest
 
@@ -45,7 +46,7 @@ def test_paired_transforms(m, kind):
     _check((32, m, 7), (P, kind, N), 2)  # odd rows: no adjacent pairs, solve along z
 
 
-@pytest.mark.parametrize("ns", [2, 3, 4, 5, 63, 64, 65, 255, 256, 257, 512, 513, 1030])
+@pytest.mark.parametrize("ns", [2, 3, 4, 5, 63, 64, 65, 255, 256, 257, 512, 513, 1030, 2048, 2049, 3000])
 def test_tridiagonal_chunks(ns):
     _check((8, ns, 4), (P, N, P), 1)
     _check((ns, 4, 8), (D, P, N), 0)

@@ -1,9 +1,9 @@
-"""The coarse end of the V-cycle in one CTA (k_tail_cycle, option
-fuseCoarse) against the per-pass launches it replaces: the kernel runs the
-same per-item functions (colour_quad_item, restrict_quad_item,
-prolong_quad_item, coarse_solve_block), so whole solves are bit-identical in
-FP64 and mixed precision, with constant and variable coefficients, with and
-without the flexible-CG outer loop, and they launch fewer kernels."""
+"""The coarse end of the V-cycle in one thread-block cluster (k_tail_cycle,
+option fuseCoarse) against the per-pass launches it replaces: the kernel has the
+arithmetic of the per-pass kernels in the same order, so whole solves are
+bit-identical in FP64 and mixed precision, with constant and variable
+coefficients, with and without the flexible-CG outer loop, and they launch
+fewer kernels."""
 import numpy as np
 import pytest
 

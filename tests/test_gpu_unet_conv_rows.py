@@ -35,6 +35,8 @@ CASES = [
     ((2, 3, 130), 32, 0, 0, 32),   # a long run: groups of 16
     ((2, 3, 255), 16, 0, 0, 64),
     ((1, 2, 300), 16, 0, 0, 16),   # too long a row: the tiled kernel
+    ((2, 2, 264), 32, 0, 0, 96),   # and its widest outputs
+    ((1, 3, 260), 64, 0, 0, 128),
     ((2, 2, 24), 256, 0, 0, 16),
     ((2, 11, 64), 32, 0, 0, 96),   # two halves of the output channels
     ((1, 9, 128), 64, 0, 0, 128),
