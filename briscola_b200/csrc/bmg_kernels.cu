@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(256) k_restrict_quad(Bricks<T> FB, Bricks<T> C
 // both halves of a row -- the 2 NS consecutive cells from k = 2 NS P, half of
 // them even and half odd -- so every fine array moves as one 16-byte vector
 // a thread, whole lines a warp (FP64 threads of four slots moved half lines,
-// and the L1 was their bound: 256^3 restriction 96 us, prolongation 103 us).
+// and the L1 was their bound: 256^3 restriction 96 us, now 85, prolongation 103 us, now 78).
 // The restriction writes the coarse cells K = NS P .. (the parents of those
 // cells); on small levels the four fine rows over them go to four lanes, so a
 // thread waits for one row's loads and there are threads enough.  The
@@ -1386,11 +1386,15 @@ inline dim3 split_block(int groups) {
 template <typename T, bool VAR>
 void launch_residual_restrict(const Bricks<T>& F, const Bricks<T>& C, const TransferSet& t, cudaStream_t s) {
     if (F.v[0].kh && quad_transfers(F, t)) {
-        // four lanes a group where the groups alone are at most 256 CTAs (64^3
-        // fine: 11 -> 6 us); above that one thread reads its rows' shared
-        // planes and rows once (256^3 FP64: 124 us with four lanes)
+        // four lanes a group where the groups alone leave the SMs waiting; above
+        // that one thread reads its rows' shared planes and rows once.  Measured,
+        // us with four lanes / one: FP64 64^3 5.2 / 10.0, 96^3 9.8 / 10.1, 128 x 96 x
+        // 96 12.9 / 11.4, 256^3 129 / 85; FP64 with face coefficients 64 x 96 x 96
+        // 10.4 / 10.5, 96^3 14.4 / 11.6; FP32 64 x 96 x 96 6.9 / 8.4, 96^3 9.2 / 8.6,
+        // 128^3 12.4 / 10.1 (with coefficients 15.9 / 12.0)
         const int groups = F.v[0].kh / Vec16<T>::N;
-        const bool spread = (long)groups * C.v[0].n1 * C.v[0].n0 <= 256 * 256;
+        constexpr long limit = (sizeof(T) == 8 && !VAR ? 64 : 24) * 1024;
+        const bool spread = (long)groups * C.v[0].n1 * C.v[0].n0 <= limit;
         const dim3 blk = split_block(spread ? 4 * groups : groups);
         const dim3 grid(((spread ? 4 * groups : groups) + blk.x - 1) / blk.x, (C.v[0].n1 + blk.y - 1) / blk.y, C.v[0].n0);
         if (spread)
