@@ -726,8 +726,10 @@ __device__ __forceinline__ void restrict_quad_item(const LevelView<T>& F, const 
     C.b[cell32(C, I, J, K0 + 1)] = acc1;
 }
 
+// (FP32 with the contact mask: 152 registers left one block an SM, 51 us on level 0
+// of the seven-brick mesh; two blocks at 128 registers 30)
 template <typename T, int COEF>
-__global__ void __launch_bounds__(256) k_restrict_quad(Bricks<T> FB, Bricks<T> CB, TransferSet ts) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 && COEF == C_MASK ? 2 : 0) k_restrict_quad(Bricks<T> FB, Bricks<T> CB, TransferSet ts) {
     grid_dep_sync();
     int I;
     const int b = brick_of(CB, blockIdx.z, I);
