@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(WgradArgs a) {
 // they hold); of the products those of rows j and j-1 .. j+1 are wanted, the
 // diagonal blocks, which is 3 W of W (W + 2).  One input row against the three
 // rows that meet it filled 48 of the 128 rows of M for 16 channels and was bound
-// by the tensor pipe (68 - 90 %): five times as many MMA cycles a row.
+// by the tensor pipe: five times as many MMA cycles a row.
 // Rows outside the grid are zero.  Both operands are MN-major: chunks of 8
 // channels x voxels of 16 bytes.
 // D: lane = (row, output channel), column = (dk, input row, input channel),
@@ -470,7 +470,9 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(WgradArgs a) {
 // channels 1936 / 663 / 292, 16 -> 16 735 / 250 / 119; at 64^3 96 -> 32
 // 802 / 210 / 162, 32 -> 32 286 / 78 / 61, 16 -> 32 160 / 72 / 40; k_wgrad / now:
 // at 32^3 128 -> 64 150 / 74, 64 -> 64 90 / 42; at 16^3 64 -> 64 27 / 17.  Bound
-// by the blocks' supply from L2 at the larger sizes (74 KB against 24 MMAs).
+// by the blocks' supply (74 KB against 24 MMAs): 48 -> 16 at 128^3 has the tensor
+// pipe active 39 %, L1 51 %, and its warps wait for the loads; 64 -> 64 there, two
+// stages, has L1 at 95 %.
 constexpr int kWgVox = 128;                      // voxels of a block's rows
 constexpr int kWgInChunk = (kWgVox + 2) * 16;    // bytes of 8 input channels of a row (k0-1 .. k0+128)
 constexpr int kWgDzChunk = kWgVox * 16;          // bytes of 8 output channels of a row
@@ -691,8 +693,8 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 // starting at chunk 2u, position P di + dk, with the chunks' distance as
 // leading and 128 bytes (8 positions) as stride byte offset: a tap is a change
 // of start address.
-// With 16 to 48 output channels an MMA costs what its A operand's 4 KB cost
-// (54 cycles for N up to 48), whatever N is, so the three dj of (di, dk) are one
+// With 16 to 48 output channels an MMA costs what its A operand's 4 KB cost,
+// whatever N is, so the three dj of (di, dk) are one
 // MMA: the input row's products for output rows jj-1, jj and jj+1, whose
 // accumulators are neighbours in tensor memory (all JS rows' are there, zeroed
 // at the start), with the weights of dj = 2, 1, 0 side by side as B.
@@ -705,11 +707,11 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 // thread issues the MMAs.
 // Measured against a tap an MMA on the n2 % 128 == 0 rows, the only ones that
 // marched, and against k_conv elsewhere (256^3 network, cin -> nout at the
-// level's size, us before / now; two thirds of the time is the rows' supply and
-// the hand-over between the warps, not the MMAs):
-//   256^3  16 -> 16   663 /  592     48 -> 16   3359 / 1336
-//   128^3  96 -> 32  2869 /  442     32 -> 32   360 /  196     16 -> 32  132 / 121
-//    64^3  32 -> 64   119 /   47     64 -> 64    319 /   78   128 -> 64  589 / 139
+// level's size, us before / now; the tensor pipe is active 18 to 37 % of the time,
+// L1 46 to 52 %: the rows' supply and the hand-over between the warps bound it):
+//   256^3  16 -> 16   663 /  569     48 -> 16   3359 / 1282
+//   128^3  96 -> 32  2869 /  418     32 -> 32   360 /  191     16 -> 32  132 / 121
+//    64^3  32 -> 64   119 /   47     64 -> 64    319 /   76   128 -> 64  589 / 134
 //    32^3  64 -> 64    50 /   21;  16^3 64 -> 64   30 /   17
 constexpr int kRowThreads = 288;
 constexpr int kRowRing = 8;  // most rows of the ring
