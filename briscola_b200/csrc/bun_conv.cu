@@ -696,12 +696,15 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 // With 16 to 48 output channels an MMA costs what its A operand's 4 KB cost,
 // whatever N is, so the three dj of (di, dk) are one
 // MMA: the input row's products for output rows jj-1, jj and jj+1, whose
-// accumulators are neighbours in tensor memory (all JS rows' are there, zeroed
+// accumulators are neighbours in tensor memory (JS rows' are there, zeroed
 // at the start), with the weights of dj = 2, 1, 0 side by side as B.
-// Input channels go in groups of CG: the CTA walks its rows once per group
-// with that group's weights (two buffers, the next group's load under this
+// Input channels go in groups of CG: the CTA walks its rows, JS at most, once per
+// group with that group's weights (two buffers, the next group's load under this
 // one's MMAs); the sums stay in FP32 in tensor memory from the first group to
-// the last.
+// the last.  With one group a row is complete after its three input rows, and the
+// CTA may walk more (RING): the epilogue zeroes a row's accumulator for the JS-th
+// row after it, and where the three rows' accumulators begin again they take two
+// MMAs.
 // Warps 0-3: epilogue (thread = position = TMEM lane), a row as soon as the
 // last group completes it; warps 4-7: loader; warp 8: TMEM allocation, one
 // thread issues the MMAs.
@@ -715,13 +718,14 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 //    32^3  64 -> 64    50 /   21;  16^3 64 -> 64   30 /   17
 constexpr int kRowThreads = 288;
 constexpr int kRowRing = 8;  // most rows of the ring
+constexpr int kRowsMost = 32;  // most rows j a CTA
 
 struct RowPlan {
     int P;       // distance of the planes' rows in the run
     int nvox;    // positions of the run: 2 P + 130
     int nr;      // rows of the ring
     int nw;      // weight buffers: two, one where there is one group of channels
-    int rows;    // rows j a CTA, at most JS
+    int rows;    // rows j a CTA; at most JS but with RING
     int lk;      // log2 of the 8-channel chunks of a packed weight block
     int ntot;    // output channels, NOUT of them a CTA (blockIdx.y)
     int stream;  // rows one behind another
@@ -732,7 +736,7 @@ template <int CG, int NOUT, int JS>
 struct RowShape {
     static constexpr int WBYTES = 27 * CG * NOUT * 2;
     static constexpr uint32_t NCOLS = JS * NOUT <= 256 ? 256 : 512;
-    static constexpr int BARS = (2 * kRowRing + 4 + JS + 1) * 8 + 16;
+    static constexpr int BARS = (2 * kRowRing + 4 + 2 * JS + 1) * 8 + 16;
     // longest run: P of 256 (or 130; groups of 32 have rows below 128 only)
     static constexpr int MAXVOX = CG == 16 ? 2 * 256 + kTile + 2 : 2 * 130 + kTile + 2;
     static_assert(JS * NOUT <= 512 && 3 * NOUT <= 256, "tensor memory");
@@ -800,7 +804,7 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
 
 // (two CTAs of nine warps put five on one scheduler: at most 96 registers, the
 // bound for ten warps each; at 108 the second CTA stayed out, 840 -> 1445 us)
-template <int CG, int NOUT, int JS>
+template <int CG, int NOUT, int JS, bool RING>
 __global__ void __launch_bounds__(kRowThreads + 32, JS * NOUT <= 256 ? 2 : 1) k_conv_rows(ConvArgs a, RowPlan R) {
     using F = RowShape<CG, NOUT, JS>;
     constexpr int NQ = CG / 16;
@@ -812,7 +816,8 @@ __global__ void __launch_bounds__(kRowThreads + 32, JS * NOUT <= 256 ? 2 : 1) k_
     uint64_t* wfull = empty + kRowRing;   // [2]
     uint64_t* wempty = wfull + 2;   // [2]
     uint64_t* tfull = wempty + 2;   // [JS]
-    uint64_t* fin = tfull + JS;     // every MMA of the CTA has completed
+    uint64_t* tempty = tfull + JS;  // [JS]
+    uint64_t* fin = tempty + JS;    // every MMA of the CTA has completed
     uint32_t* slot = reinterpret_cast<uint32_t*>(fin + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -832,7 +837,10 @@ __global__ void __launch_bounds__(kRowThreads + 32, JS * NOUT <= 256 ? 2 : 1) k_
             mbar_init(&wfull[q], kProducers);
             mbar_init(&wempty[q], 1);
         }
-        for (int q = 0; q < JS; ++q) mbar_init(&tfull[q], 1);
+        for (int q = 0; q < JS; ++q) {
+            mbar_init(&tfull[q], 1);
+            mbar_init(&tempty[q], kProducers);
+        }
         mbar_init(fin, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -922,24 +930,45 @@ __global__ void __launch_bounds__(kRowThreads + 32, JS * NOUT <= 256 ? 2 : 1) k_
                 tc_after();
                 // output rows lo .. hi of jj-1 .. jj+1 lie in the segment
                 const int lo = max(js, jj - 1), hi = min(je - 1, jj + 1);
-                const uint32_t idesc = idesc_bf16(kTile, (hi - lo + 1) * NOUT, false, false);
-                const uint32_t d = tmem + (uint32_t)((lo - js) * NOUT);
-                const uint32_t set = base + (e % NR) * set_bytes, wj = wg + (uint32_t)((lo - (jj - 1)) * NOUT * 32);
-#pragma unroll
-                for (int di = 0; di < 3; ++di) {
-#pragma unroll
-                    for (int dk = 0; dk < 3; ++dk) {
-#pragma unroll
-                        for (int u = 0; u < NQ; ++u)
-                            umma(d, sdesc(set + 2 * u * chunk + (di * R.P + dk) * 16, chunk, 128),
-                                 sdesc(wj + (uint32_t)(((di * 3 + dk) * NQ + u) * 3 * NOUT * 32), 128, 256), idesc, 1u);
+                // RING: a row beyond the JS-th takes the accumulator of the JS-th before it
+                if (RING && hi == jj + 1 && hi - js >= JS) {
+                    if (!mbar_wait(&tempty[(hi - js) % JS], (uint32_t)((hi - js) / JS - 1) & 1)) {
+                        ok = false;
+                        break;
                     }
+                    tc_after();
+                }
+                const uint32_t set = base + (e % NR) * set_bytes;
+                auto issue = [&](int row, int at, int n) {
+                    const uint32_t idesc = idesc_bf16(kTile, n * NOUT, false, false);
+                    const uint32_t d = tmem + (uint32_t)(at * NOUT), wj = wg + (uint32_t)((row - (jj - 1)) * NOUT * 32);
+#pragma unroll
+                    for (int di = 0; di < 3; ++di) {
+#pragma unroll
+                        for (int dk = 0; dk < 3; ++dk) {
+#pragma unroll
+                            for (int u = 0; u < NQ; ++u)
+                                umma(d, sdesc(set + 2 * u * chunk + (di * R.P + dk) * 16, chunk, 128),
+                                     sdesc(wj + (uint32_t)(((di * 3 + dk) * NQ + u) * 3 * NOUT * 32), 128, 256), idesc, 1u);
+                        }
+                    }
+                };
+                if constexpr (RING) {
+                    // one MMA, or two where the accumulators begin again
+#pragma unroll 1
+                    for (int row = lo, n; row <= hi; row += n) {
+                        const int at = (row - js) % JS;
+                        n = min(hi - row + 1, JS - at);
+                        issue(row, at, n);
+                    }
+                } else {
+                    issue(lo, lo - js, hi - lo + 1);
                 }
                 umma_commit(&empty[e % NR]);
                 if (g == groups - 1) {
                     // complete: the row before, and at the end the last one
-                    if (jj - 1 >= js) umma_commit(&tfull[jj - 1 - js]);
-                    if (jj == jhi && jj < je) umma_commit(&tfull[jj - js]);
+                    if (jj - 1 >= js) umma_commit(&tfull[RING ? (jj - 1 - js) % JS : jj - 1 - js]);
+                    if (jj == jhi && jj < je) umma_commit(&tfull[RING ? (jj - js) % JS : jj - js]);
                 }
             }
             if (ok) umma_commit(&wempty[g & 1]);
@@ -953,15 +982,24 @@ __global__ void __launch_bounds__(kRowThreads + 32, JS * NOUT <= 256 ? 2 : 1) k_
         int i, k;
         const bool live = row_voxel(a, R, tile, R.P + 1 + tid, i, k);
         for (int j = js; j < je; ++j) {
-            bool done = mbar_wait(&tfull[j - js], 0);
+            const int at = RING ? (j - js) % JS : j - js;
+            bool done = mbar_wait(&tfull[at], RING ? (uint32_t)((j - js) / JS) & 1 : 0u);
             done = __all_sync(0xffffffffu, done);
             if (!done) {
                 ok = false;
                 break;
             }
             tc_after();
-            store_row<NOUT>(a, tmem + (uint32_t)((j - js) * NOUT), warp, ((long)i * n1 + j) * n2 + k, live, R.ntot,
+            store_row<NOUT>(a, tmem + (uint32_t)(at * NOUT), warp, ((long)i * n1 + j) * n2 + k, live, R.ntot,
                             (int)blockIdx.y * NOUT);
+            if (RING && j + JS < je) {  // the accumulator's next row
+#pragma unroll 1
+                for (int c = 0; c < NOUT; c += 16)
+                    tmem_zero16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(at * NOUT + c));
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_before();
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[at])) : "memory");
+            }
         }
     }
 
@@ -1023,6 +1061,18 @@ int rows_ring(const ConvArgs& a, RowPlan& R, int bytes) {
 }
 constexpr int kRowsTwo = 113 * 1024, kRowsOne = 227 * 1024;  // shared memory of a CTA, two and one an SM
 
+template <int CG, int NOUT, int JS, bool RING>
+cudaError_t rows_go(const ConvArgs& a, const RowPlan& R, int parts, cudaStream_t s) {
+    using F = RowShape<CG, NOUT, JS>;
+    const int smem = R.nr * (CG / 8) * R.nvox * 16 + R.nw * F::WBYTES + F::BARS;
+    const auto kernel = k_conv_rows<CG, NOUT, JS, RING>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const unsigned segs = (unsigned)((a.n1 + R.rows - 1) / R.rows);
+    kernel<<<dim3((unsigned)R.tiles * segs, (unsigned)parts), kRowThreads, smem, s>>>(a, R);
+    return cudaGetLastError();
+}
+
 template <int CG, int NOUT, int JS>
 cudaError_t rows_inst(const ConvArgs& a, int kc, int parts, cudaStream_t s) {
     using F = RowShape<CG, NOUT, JS>;
@@ -1031,26 +1081,35 @@ cudaError_t rows_inst(const ConvArgs& a, int kc, int parts, cudaStream_t s) {
     R.ntot = NOUT * parts;
     // as deep a ring as fits: two CTAs an SM where their accumulators do
     R.nr = rows_ring<CG, NOUT, JS>(a, R, F::NCOLS == 256 ? kRowsTwo : kRowsOne);
+    const bool two = F::NCOLS == 256 && R.nr >= 2;
     if (R.nr < 2) R.nr = rows_ring<CG, NOUT, JS>(a, R, kRowsOne);
     if (R.nr < 1) return cudaErrorInvalidValue;
-    const int smem = R.nr * (CG / 8) * R.nvox * 16 + R.nw * F::WBYTES + F::BARS;
-    cudaError_t e = cudaFuncSetAttribute(k_conv_rows<CG, NOUT, JS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     const long tiles = R.stream ? ((long)a.n0 * R.P + kTile - 1) / kTile : (long)a.n0 * (a.n2 / kTile);
     R.tiles = (int)tiles;
-    // rows a CTA: input rows walked (two more than it owns) times the CTAs an
-    // SM gets, at its least; the most rows where that is equal
+    // Rows a CTA, at the least cost, the most rows where that is equal: input rows
+    // walked (two more than it owns) times the CTAs an SM gets.  With one group of
+    // channels a row is complete after its three input rows and its accumulator can
+    // go to the JS-th row after it, so a CTA may take more rows; its start and end
+    // take about as long as 5 rows, and two CTAs on an SM slow each other to 1.4
+    // times a row's time (64^3, 16 -> 32: 18.7 us with 8 rows a CTA, 23.0 with 16).
+    // 16 -> 48 at 128^3 takes 113 us with up to 32 rows, 155 with 5.  With one CTA an
+    // SM that was slower (32 -> 32 at 128^3 202 us against 189).
+    const bool march = two && R.nw == 1;
     long best = 0;
-    for (int t = std::min(JS, a.n1); t >= 1; --t) {
-        const long ctas = tiles * parts * ((a.n1 + t - 1) / t), cost = (ctas + kSms - 1) / kSms * (t + 2);
+    for (int t = std::min(march ? kRowsMost : JS, a.n1); t >= 1; --t) {
+        const long ctas = tiles * parts * ((a.n1 + t - 1) / t);
+        const long cost = !march         ? (ctas + kSms - 1) / kSms * (t + 2)
+                          : ctas <= kSms ? 5 * (t + 2 + 5)
+                                         : (ctas + 2 * kSms - 1) / (2 * kSms) * (7 * (t + 2) + 25);
         if (!best || cost < best) {
             best = cost;
             R.rows = t;
         }
     }
-    k_conv_rows<CG, NOUT, JS>
-        <<<dim3((unsigned)(tiles * ((a.n1 + R.rows - 1) / R.rows)), (unsigned)parts), kRowThreads, smem, s>>>(a, R);
-    return cudaGetLastError();
+    if constexpr (F::NCOLS == 256) {
+        if (R.rows > JS) return rows_go<CG, NOUT, JS, true>(a, R, parts, s);
+    }
+    return rows_go<CG, NOUT, JS, false>(a, R, parts, s);
 }
 
 }  // namespace
@@ -1078,8 +1137,9 @@ cudaError_t rows48(const ConvArgs& a, int kc, int parts, cudaStream_t s) {
 // Rows a CTA: 16 of 16 output channels, 8 of 32 and 5 of 48 (256 columns of
 // tensor memory each: two CTAs an SM, one's start and end under the other's
 // rows), 8 of 64, and of 32 from groups of 32 input channels 16 (all of it).  With
-// one CTA an SM, 16 rows of 32 and 10 of 48, 16 -> 32 at 128^3 took 144 us
-// (now 121; a tap an MMA 132) and 16 -> 48 197 (155; 133); 32 -> 96 at 64^3 86 (64).
+// one CTA an SM, 16 rows of 32 and 10 of 48, 48 -> 32 at 128^3 took 316 us (now 272)
+// and 32 -> 48 306 (246), 32 -> 96 at 64^3 86 (64); a tap an MMA 16 -> 32 132 (103)
+// and 16 -> 48 133 (113).
 // 10 rows of 48 stay where the weights leave two CTAs no ring: 32 -> 48 on
 // 40 x 24 x 200 40 us against 47.  Groups of 32 input channels where both weight
 // buffers leave room for a ring.

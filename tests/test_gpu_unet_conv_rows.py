@@ -45,6 +45,10 @@ CASES = [
     ((1, 10, 189), 32, 0, 0, 48),  # and longer ones: 10 rows a CTA
     ((2, 6, 250), 32, 0, 0, 96),
     ((2, 9, 256), 48, 0, 0, 32),   # 8 rows of 32 channels a CTA and one more
+    ((64, 37, 128), 16, 0, 0, 48),  # one group: 10 rows a CTA on 5 accumulators, and 7
+    ((60, 37, 100), 16, 0, 0, 48),  # 7 rows, planes one behind another
+    ((64, 45, 128), 16, 0, 0, 32),  # 12 rows on 8
+    ((100, 40, 128), 16, 0, 0, 16),  # 20 rows on 16
 ]
 
 
