@@ -710,10 +710,10 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_rows(WgradArgs a) {
 // thread issues the MMAs.
 // Measured against a tap an MMA on the n2 % 128 == 0 rows, the only ones that
 // marched, and against k_conv elsewhere (256^3 network, cin -> nout at the
-// level's size, us before / now; the tensor pipe is active 18 to 37 % of the time,
-// L1 46 to 52 %: the rows' supply and the hand-over between the warps bound it):
-//   256^3  16 -> 16   663 /  569     48 -> 16   3359 / 1282
-//   128^3  96 -> 32  2869 /  418     32 -> 32   360 /  191     16 -> 32  132 / 121
+// level's size, us before / now; the tensor pipe is active 18 to 40 % of the time,
+// L1 47 to 57 %: the rows' supply and the hand-over between the warps bound it):
+//   256^3  16 -> 16   663 /  547     48 -> 16   3359 / 1282
+//   128^3  96 -> 32  2869 /  418     32 -> 32   360 /  191     16 -> 32  132 / 103
 //    64^3  32 -> 64   119 /   47     64 -> 64    319 /   76   128 -> 64  589 / 134
 //    32^3  64 -> 64    50 /   21;  16^3 64 -> 64   30 /   17
 constexpr int kRowThreads = 288;
